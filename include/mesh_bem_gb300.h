@@ -126,6 +126,16 @@ int mb_mom_zmat_rwg_edges_c64(const float* verts, int64_t n_verts, const int32_t
                               const float* gp_x, const float* gw_x, int n_x, const float* gp_y,
                               const float* gw_y, int n_y, double wavenumber, int64_t m_begin, int64_t m_end,
                               float* z, void* stream);
+/* The same matrix with each face pair's quadrature sized by its separation (csrc/mom_tiers.cu: the
+ * reference's points on close pairs, rules of the same exactness with fewer points on the
+ * others, entries equal within FP32 rounding); accumulated into z.  float32 meshes, gaussQR 3
+ * to 5; any number of faces per edge.  workspace: mb_mom_tiers_workspace_bytes(n_faces), 16-byte aligned. */
+int64_t mb_mom_tiers_workspace_bytes(int64_t n_faces);
+int mb_mom_zmat_rwg_tiers_c64(const float* verts, int64_t n_verts, const int32_t* faces, int64_t n_faces,
+                              const float* face_areas, const float* face_normals, const int32_t* face_edge_indices,
+                              int64_t n_edges, const float* gp_x, const float* gw_x, int n_x, const float* gp_y,
+                              const float* gw_y, int n_y, double wavenumber, void* workspace,
+                              int64_t workspace_bytes, float* z, void* stream);
 /* The same matrix in gather form: thread (m, n) sums the (up to 2 x 2) face-edge entries of
  * Z[m, n] and writes the entry once (no atomics): rows [m_begin, m_end) of z are OVERWRITTEN
  * (no zeroing needed; half the DRAM traffic of the edge order, ~3 % slower at 20480 faces).
@@ -420,6 +430,17 @@ int mb_mom_ref_zmat_batched_persistent_c64(const float* verts, const int32_t* fa
                                            const int64_t* block_offsets, int64_t total_blocks, const double* ks,
                                            int n_mesh, const float* gpx, const float* gwx, int nx, const float* gpy,
                                            const float* gwy, int ny, float* z, void* stream);
+/* The same matrices as mb_mom_zmat_rwg_tiers_c64 builds them; gaussQR 3 to 5.  far_offsets / close_offsets
+ * [n_mesh + 1]: first block of each mesh with ceil(F_i / rows) x ceil(F_i / 128) blocks (rows <= 32) and with
+ * ceil(F_i / tp) x ceil(F_i / tq) blocks (tp <= 256, tq a power of two <= 128, tp tq <= 1024).  workspace: as above for the
+ * faces of all meshes. */
+int mb_mom_ref_zmat_batched_tiers_c64(const float* verts, const int32_t* faces, int64_t total_faces,
+                                      const float* face_areas, const float* face_normals, const int32_t* fei,
+                                      const int64_t* desc, const int64_t* far_offsets, int64_t far_blocks,
+                                      const int64_t* close_offsets, int64_t close_blocks, int rows, int tp, int tq,
+                                      const double* ks, int n_mesh, const float* gpx, const float* gwx, int nx,
+                                      const float* gpy, const float* gwy, int ny, void* workspace,
+                                      int64_t workspace_bytes, float* z, void* stream);
 int mb_mom_ref_rhs_batched_c64(const float* verts, const int32_t* faces, const float* face_areas,
                                const float* face_normals, const int32_t* fei, const int64_t* desc,
                                int n_mesh, int64_t total_faces, const float* gp, const float* gw, int n,

@@ -42,6 +42,11 @@ _SIGS = {
     "mb_gmres_multi_column_steps": [_P, _I64, _I64, _I, _P, _P],
     "mb_mom_zmat_rwg_edges_c64": [_P, _I64, _P, _I64, _P, _P, _P, _P, _I64, _P, _P, _I, _P, _P, _I, _D,
                                   _I64, _I64, _P, _P],
+    "mb_mom_tiers_workspace_bytes": [_I64],
+    "mb_mom_zmat_rwg_tiers_c64": [_P, _I64, _P, _I64, _P, _P, _P, _I64, _P, _P, _I, _P, _P, _I, _D, _P, _I64, _P,
+                                  _P],
+    "mb_mom_ref_zmat_batched_tiers_c64": [_P, _P, _I64, _P, _P, _P, _P, _P, _I64, _P, _I64, _I, _I, _I, _P, _I, _P,
+                                          _P, _I, _P, _P, _I, _P, _I64, _P, _P],
     "mb_mom_zmat_rwg_gather_c64": [_P, _I64, _P, _I64, _P, _P, _P, _I64, _P, _P, _I, _P, _P, _I, _D, _I64, _I64,
                                    _P, _P],
     "mb_mom_zmat_rwg_to_host_c64": [_P, _I64, _P, _I64, _P, _P, _P, _I64, _P, _P, _I, _P, _P, _I, _D,
@@ -128,7 +133,7 @@ _SIGS = {
     "mb_pgmres_c128": [_P, _I64, _P, _P, _P, _P, _I, _I, _D, _I, _P, ctypes.c_size_t, _P, _P],
 }
 
-_RESTYPES = {"mb_gmres_workspace_bytes": ctypes.c_size_t, "mb_ray_bvh_bytes": ctypes.c_size_t,
+_RESTYPES = {"mb_mom_tiers_workspace_bytes": ctypes.c_int64, "mb_gmres_workspace_bytes": ctypes.c_size_t, "mb_ray_bvh_bytes": ctypes.c_size_t,
              "mb_gmres_real_workspace_bytes": ctypes.c_size_t, "mb_cgemm_workspace_bytes": ctypes.c_size_t,
              "mb_gmres_multi_workspace_bytes": ctypes.c_size_t,
              "mb_gmres_blockdiag_workspace_bytes": ctypes.c_size_t,

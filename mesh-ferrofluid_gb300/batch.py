@@ -89,6 +89,12 @@ class MeshBatch:
             nfs = desc[:, 1]
             per = 3 * nfs * ((3 * nfs + 127) // 128)
             self.ref_boff = torch.tensor(np.concatenate([[0], np.cumsum(per)]).astype(np.int64), device=dev)
+            if gaussQR in (3, 4, 5):
+                rows, tp, tq = self._tier_tiles = (32, 16, 64)
+                tiles = [((nfs + a - 1) // a) * ((nfs + b - 1) // b) for a, b in ((rows, 128), (tp, tq))]
+                off = np.stack([np.concatenate([[0], np.cumsum(t)]) for t in tiles]).astype(np.int64)
+                self._tier_blocks = (int(off[0, -1]), int(off[1, -1]))
+                self._tier_off = torch.tensor(off, device=dev)
         self.ks = torch.tensor(np.asarray(wavenumbers, np.float64), device=dev)
         if not bool(torch.all(self.ks > 0)):
             raise ValueError("wavenumbers must be > 0")
@@ -142,6 +148,17 @@ class MeshBatch:
             out.zero_()
         if self.formulation == "cfie_ref":
             cfg = getattr(self, "asm_config", None)
+            if self.gq in (3, 4, 5) and cfg in (None, ("grid", None)):
+                ws = torch.empty(int(_lib.load().mb_mom_tiers_workspace_bytes(self.total_faces)), dtype=torch.uint8,
+                                 device=self.device)
+                _lib.call("mb_mom_ref_zmat_batched_tiers_c64", _lib.ptr(self.verts), _lib.ptr(self.faces),
+                          self.total_faces, _lib.ptr(self.areas), _lib.ptr(self.normals), _lib.ptr(self.fei),
+                          _lib.ptr(self.desc), _lib.ptr(self._tier_off[0]), self._tier_blocks[0],
+                          _lib.ptr(self._tier_off[1]), self._tier_blocks[1], *self._tier_tiles, _lib.ptr(self.ks),
+                          self.n_mesh, _lib.ptr(self.gpx), _lib.ptr(self.gwx), self.gq, _lib.ptr(self.gpy),
+                          _lib.ptr(self.gwy), self.gq - 1, _lib.ptr(ws), ws.numel(), _lib.ptr(out),
+                          _lib.stream_of(out))
+                return out
             name = "mb_mom_ref_zmat_batched_persistent_c64" if cfg == ("persistent", None) else \
                 "mb_mom_ref_zmat_batched_c64"
             _lib.call(name, _lib.ptr(self.verts), _lib.ptr(self.faces), _lib.ptr(self.areas),
@@ -181,9 +198,10 @@ class MeshBatch:
     def autotune_assembly(self, out: torch.Tensor | None = None, reps: int = 2):
         """Pick the assembly's tile and block schedule by timing each candidate.  EFIE: the one-
         pair-per-thread kernel, or the rows layout with 8, 16 or 32 test faces per block and the
-        meshes' blocks in packing order or largest mesh first.  Reference CFIE: one block per
-        (mesh, row, 128-column tile) ("grid", None) or a resident grid taking those tiles from a
-        work counter ("persistent", None).  Returns the chosen configuration."""
+        meshes' blocks in packing order or largest mesh first.  Reference CFIE: a grid
+        over the meshes' tiles ("grid", None; each face pair's quadrature sized by its separation
+        for gaussQR 3-5, one block per (mesh, row, 128-column tile) for 2) or a resident grid taking
+        the (mesh, row, 128-column) tiles from a work counter ("persistent", None).  Returns the chosen configuration."""
         if self.desc is None:
             self._set_nc(1)
         if out is None:

@@ -89,6 +89,15 @@ int gnn_relu_bwd(const void* y, const float* dy, int64_t count, float* dz, cudaS
 int gnn_adam(float* w, float* m1, float* m2, const float* g, int64_t count, float lr, float b1, float b2, float eps,
              int step, void* w16, cudaStream_t s);
 int launch_edge_rows(const int32_t* fei, int64_t nf, int64_t n_edges, int32_t* er, cudaStream_t s);
+bool mom_tier_rule(int nx, int ny);
+int launch_mom_tiers(const float* verts, const int32_t* faces, int64_t nf, const float* areas, const float* normals,
+                     const int32_t* fei, int64_t n_edges, const float* gpx, const float* gwx, int nx, const float* gpy,
+                     const float* gwy, int ny, double k, float* rec, float* z, cudaStream_t s);
+int launch_mom_tiers_batched(const float* verts, const int32_t* faces, int64_t total_faces, const float* areas,
+                             const float* normals, const int32_t* fei, const int64_t* desc, const int64_t* far_off,
+                             int64_t far_blocks, const int64_t* close_off, int64_t close_blocks, int rows, int tp, int tq,
+                             const double* ks, int n_mesh, const float* gpx, const float* gwx, int nx, const float* gpy,
+                             const float* gwy, int ny, float* rec, float* z, cudaStream_t s);
 bool launch_fast_zmat_edges(const float* verts, const int32_t* faces, const float* areas, const float* normals,
                             const int32_t* fei, const int32_t* edge_rows, int64_t n_edges, const float* gpx,
                             const float* gwx, int nx, const float* gpy, const float* gwy, int ny, double k,
@@ -278,6 +287,28 @@ int mb_mom_zmat_rwg_edges_c64(const float* verts, int64_t n_verts, const int32_t
                                 as_stream(stream)))
         return set_error(MB_ERR_UNSUPPORTED, "edge-row assembly: no instance for rule sizes (%d, %d)", n_x, n_y);
     return check_launch("mom_ref_zmat_edges");
+}
+
+int64_t mb_mom_tiers_workspace_bytes(int64_t n_faces) { return n_faces > 0 ? 128 * n_faces : 0; }
+
+int mb_mom_zmat_rwg_tiers_c64(const float* verts, int64_t n_verts, const int32_t* faces, int64_t n_faces,
+                              const float* face_areas, const float* face_normals, const int32_t* face_edge_indices,
+                              int64_t n_edges, const float* gp_x, const float* gw_x, int n_x, const float* gp_y,
+                              const float* gw_y, int n_y, double wavenumber, void* workspace,
+                              int64_t workspace_bytes, float* z, void* stream) {
+    (void)n_verts;
+    MB_REQUIRE(n_faces >= 0 && n_edges >= 0, "bad sizes");
+    if (n_faces == 0) return MB_OK;
+    MB_REQUIRE(verts && faces && face_areas && face_normals && face_edge_indices && gp_x && gw_x && gp_y && gw_y &&
+                   workspace && z,
+               "null pointer argument");
+    MB_REQUIRE(wavenumber > 0, "wavenumber must be > 0");
+    MB_REQUIRE(workspace_bytes >= mb_mom_tiers_workspace_bytes(n_faces) && (uintptr_t)workspace % 16 == 0,
+               "workspace too small or not 16-byte aligned");
+    if (!mom_tier_rule(n_x, n_y))
+        return set_error(MB_ERR_UNSUPPORTED, "tiered assembly: no instance for rule sizes (%d, %d)", n_x, n_y);
+    return launch_mom_tiers(verts, faces, n_faces, face_areas, face_normals, face_edge_indices, n_edges, gp_x, gw_x, n_x,
+                            gp_y, gw_y, n_y, wavenumber, static_cast<float*>(workspace), z, as_stream(stream));
 }
 
 int mb_mom_zmat_rwg_gather_c64(const float* verts, int64_t n_verts, const int32_t* faces, int64_t n_faces,
@@ -736,6 +767,29 @@ int mb_mom_ref_zmat_batched_persistent_c64(const float* verts, const int32_t* fa
                "null pointer argument");
     return launch_mom_ref_zmat_batched(verts, faces, face_areas, face_normals, fei, desc, block_offsets,
                                        total_blocks, ks, n_mesh, gpx, gwx, nx, gpy, gwy, ny, z, as_stream(stream), 1);
+}
+
+int mb_mom_ref_zmat_batched_tiers_c64(const float* verts, const int32_t* faces, int64_t total_faces,
+                                      const float* face_areas, const float* face_normals, const int32_t* fei,
+                                      const int64_t* desc, const int64_t* far_offsets, int64_t far_blocks,
+                                      const int64_t* close_offsets, int64_t close_blocks, int rows, int tp, int tq,
+                                      const double* ks, int n_mesh, const float* gpx, const float* gwx, int nx,
+                                      const float* gpy, const float* gwy, int ny, void* workspace,
+                                      int64_t workspace_bytes, float* z, void* stream) {
+    MB_REQUIRE(n_mesh >= 0 && total_faces >= 0 && far_blocks >= 0 && close_blocks >= 0, "bad sizes");
+    if (n_mesh == 0 || total_faces == 0) return MB_OK;
+    MB_REQUIRE(verts && faces && face_areas && face_normals && fei && desc && far_offsets && close_offsets && ks && gpx &&
+                   gwx && gpy && gwy && workspace && z,
+               "null pointer argument");
+    MB_REQUIRE(rows >= 1 && rows <= 32 && tp >= 1 && tp <= 256 && tq >= 1 && tq <= 128 && (tq & (tq - 1)) == 0 &&
+                   tp * tq <= 1024,
+               "tile sizes out of range");
+    MB_REQUIRE(workspace_bytes >= mb_mom_tiers_workspace_bytes(total_faces) && (uintptr_t)workspace % 16 == 0,
+               "workspace too small or not 16-byte aligned");
+    if (!mom_tier_rule(nx, ny)) return set_error(MB_ERR_UNSUPPORTED, "tiered assembly: gaussQR in {3, 4, 5}");
+    return launch_mom_tiers_batched(verts, faces, total_faces, face_areas, face_normals, fei, desc, far_offsets,
+                                    far_blocks, close_offsets, close_blocks, rows, tp, tq, ks, n_mesh, gpx, gwx, nx, gpy,
+                                    gwy, ny, static_cast<float*>(workspace), z, as_stream(stream));
 }
 
 int mb_mom_ref_rhs_batched_c64(const float* verts, const int32_t* faces, const float* face_areas,

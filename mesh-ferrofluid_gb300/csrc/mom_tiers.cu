@@ -1,0 +1,756 @@
+// mom_tiers.cu -- the reference-rule CFIE matrix in FP32 with each face pair's quadrature
+// sized by its separation.
+//
+// The reference anchors its collapsed Gauss rule at every local edge's free vertex, so the
+// nine entries of a face pair use nine point sets: 1296 kernel evaluations at gaussQR 4.
+// What makes those sets differ is only what the rules do not integrate exactly: anchored
+// at any vertex, the n x n collapsed rule is exact for polynomials of total degree 2n - 2.
+// On a pair that is far apart, compared with its triangles, and small, compared with the
+// wavelength, the integrand is such a polynomial up to less than the rounding of its FP32
+// evaluation, and any rule of that degree -- one set of points for all nine entries -- gives
+// the same entry.  With rho the larger distance of a corner from its centroid of the two
+// faces and R the centroid distance, measured on spheres of 0.15 <= kh <= 1.5 in 64 bits
+// (rms over entries, relative to them; FP32 evaluation of the 1296 points is off by
+// 1e-5 .. 6e-5 at kh = 0.38, by 1.4e-6 .. 6e-6 at kh = 1.5, the four face pairs of an entry
+// cancelling to (kh)^2 of their size):
+//   tier 1   6-point degree-4 rule on both faces        36 evaluations
+//            off by 2.7e-4 (k rho)^4 + 3.2e-2 (rho/R)^4, taken up to 2e-6
+//   tier 2   7-point degree-5 rule on the test face, the anchored source rule   189
+//            off by 1.2e-5 (k rho)^6 + 0.4 (rho/R)^6, taken up to 5e-7
+//   tier 3   12-point degree-6 rule on the test face, the anchored source rule  324
+//            off by 1.5e-6 (k rho)^8 + 0.73 (rho/R)^8, taken up to 6e-7 where k rho <= 0.8 (above, the SFU's
+//            error in the phases relative to the centroids' exceeds that of the 1296 points' mean)
+//   tier 4   the reference's points (mom_entry_fast)                           1296
+// (counts at gaussQR 4).  gaussQR 3: its source rule has degree 2, so no tier 1; its test rule
+// degree 4, so tier 2 up to the first bound.  gaussQR 5: all tiers.  A rule that is not
+// Gauss-Legendre, a normal that is not perpendicular to its face and coordinates that are
+// not finite put every pair concerned into tier 4.
+//
+// Measured on GB300 (2070 MHz), whole call: 20480 faces, k 10, unit sphere 499.3 -> 35.1 ms (far pairs 26.2, close
+// pairs 4.0 + 3.6); 5120 faces, k 6, ellipsoid 32.1 -> 4.8 ms; 1280 faces at k 10, all in tier 4, 2.54 -> 2.63 ms.
+// Error of the entries against 64 bits by distance, of the 1296 points' FP32 error: 1.0 .. 1.1 below 4 h, 0.5 .. 0.95
+// beyond (kh 0.15 .. 0.9).  The four adds of an entry are atomic, so its last bit depends on their order.
+//
+// Rules: O. C. Zienkiewicz / D. A. Dunavant, Int. J. Numer. Meth. Eng. 21 (1985), degrees 4 to 6.
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <algorithm>
+
+#include "common.cuh"
+#include "mom_entry.cuh"
+#include "packed.cuh"
+
+namespace mb {
+
+namespace {
+
+// ---------------------------------------------------------------------------------------
+// face records: 32 floats per face
+// ---------------------------------------------------------------------------------------
+constexpr int kRec = 32;
+enum {
+    kC = 0,      // centroid (hi)
+    kRho2 = 3,   // max |corner - centroid|^2; NaN: the face takes part in tier 4 only
+    kCl = 4,     // centroid (lo): hi + lo carries ~48 bits
+    kEdge = 7,   // RWG edge id of local edge e at 7 + 4 e (int bits)
+    kA = 8,      // corner a - centroid at 8 + 4 a
+    kHalf = 19,  // +-l / 2 of local edge e at 19 + 4 e (RWG sign of the reference)
+    kN = 20,     // normal
+    kAA = 24,    // |A_0|^2, |A_1|^2, |A_2|^2
+    kAB = 28     // A_0.A_1, A_1.A_2, A_2.A_0
+};
+
+// degree-4 rule: corners (1 - 2 q, q, q) of two orbits lie at s A_a from the centroid
+constexpr float kS1 = (float)(1.0 - 3.0 * 0.445948490915965), kW1 = 0.223381589678011f;
+constexpr float kS2 = (float)(1.0 - 3.0 * 0.091576213509771), kW2 = 0.109951743655322f;
+
+// test rules of tiers 2 and 3: barycentric coordinates and weights (sum 1)
+__constant__ float c_test[19][4] = {
+    {0.33333333333f, 0.33333333333f, 0.33333333333f, 0.225f},
+    {0.101286507323456f, 0.101286507323456f, 0.797426985353087f, 0.125939180544827f},
+    {0.101286507323456f, 0.797426985353087f, 0.101286507323456f, 0.125939180544827f},
+    {0.797426985353087f, 0.101286507323456f, 0.101286507323456f, 0.125939180544827f},
+    {0.470142064105115f, 0.470142064105115f, 0.059715871789770f, 0.132394152788506f},
+    {0.470142064105115f, 0.059715871789770f, 0.470142064105115f, 0.132394152788506f},
+    {0.059715871789770f, 0.470142064105115f, 0.470142064105115f, 0.132394152788506f},
+    {0.249286745170910f, 0.249286745170910f, 0.501426509658179f, 0.116786275726379f},
+    {0.249286745170910f, 0.501426509658179f, 0.249286745170910f, 0.116786275726379f},
+    {0.501426509658179f, 0.249286745170910f, 0.249286745170910f, 0.116786275726379f},
+    {0.063089014491502f, 0.063089014491502f, 0.873821971016996f, 0.050844906370207f},
+    {0.063089014491502f, 0.873821971016996f, 0.063089014491502f, 0.050844906370207f},
+    {0.873821971016996f, 0.063089014491502f, 0.063089014491502f, 0.050844906370207f},
+    {0.053145049844817f, 0.310352451033784f, 0.636502499121399f, 0.082851075618374f},
+    {0.310352451033784f, 0.053145049844817f, 0.636502499121399f, 0.082851075618374f},
+    {0.053145049844817f, 0.636502499121399f, 0.310352451033784f, 0.082851075618374f},
+    {0.310352451033784f, 0.636502499121399f, 0.053145049844817f, 0.082851075618374f},
+    {0.636502499121399f, 0.053145049844817f, 0.310352451033784f, 0.082851075618374f},
+    {0.636502499121399f, 0.310352451033784f, 0.053145049844817f, 0.082851075618374f},
+};
+
+// Gauss-Legendre nodes and weights on [0, 1], n = 2 .. 5 (the second half mirrors the first)
+__constant__ float c_gl[4][3][2] = {
+    {{0.2113248654f, 0.5f}, {0.f, 0.f}, {0.f, 0.f}},
+    {{0.1127016654f, 0.2777777778f}, {0.5f, 0.4444444444f}, {0.f, 0.f}},
+    {{0.0694318442f, 0.1739274226f}, {0.3300094782f, 0.3260725774f}, {0.f, 0.f}},
+    {{0.0469100770f, 0.1184634425f}, {0.2307653449f, 0.2393143352f}, {0.5f, 0.2844444444f}},
+};
+
+__device__ bool is_gauss(const float* p, const float* w, int n) {
+    for (int i = 0; i < n; ++i) {
+        const int j = i < (n + 1) / 2 ? i : n - 1 - i;
+        const float x = j == i ? c_gl[n - 2][j][0] : 1.f - c_gl[n - 2][j][0];
+        if (!(fabsf(p[i] - x) <= 1e-6f) || !(fabsf(w[i] - c_gl[n - 2][j][1]) <= 1e-6f)) return false;
+    }
+    return true;
+}
+
+__global__ void face_record_kernel(const float* __restrict__ verts, const int32_t* __restrict__ faces,
+                                   const float* __restrict__ normals, const int32_t* __restrict__ fei, int64_t nf,
+                                   const float* __restrict__ gpx, const float* __restrict__ gwx, int nx,
+                                   const float* __restrict__ gpy, const float* __restrict__ gwy, int ny,
+                                   float* __restrict__ rec) {
+    const int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= nf) return;
+    double v[3][3];
+    int32_t id[3];
+    float n[3];
+    for (int a = 0; a < 3; ++a) {
+        id[a] = faces[3 * f + a];
+        n[a] = normals[3 * f + a];
+        for (int d = 0; d < 3; ++d) v[a][d] = (double)verts[3 * (int64_t)id[a] + d];
+    }
+    float r[kRec];
+    float A[3][3];
+    for (int d = 0; d < 3; ++d) {
+        const double c = (v[0][d] + v[1][d] + v[2][d]) * (1.0 / 3.0);
+        r[kC + d] = (float)c;
+        r[kCl + d] = (float)(c - (double)(float)c);
+        for (int a = 0; a < 3; ++a) A[a][d] = (float)(v[a][d] - c);
+        r[kN + d] = n[d];
+    }
+    float rho2 = 0.f;
+    bool ok = is_gauss(gpx, gwx, nx) && is_gauss(gpy, gwy, ny);
+    const float nn = n[0] * n[0] + n[1] * n[1] + n[2] * n[2];
+    for (int a = 0; a < 3; ++a) {
+        const int b = (a + 1) % 3, c = (a + 2) % 3;
+        r[kAA + a] = A[a][0] * A[a][0] + A[a][1] * A[a][1] + A[a][2] * A[a][2];
+        r[kAB + a] = A[a][0] * A[b][0] + A[a][1] * A[b][1] + A[a][2] * A[b][2];
+        rho2 = fmaxf(rho2, r[kAA + a]);
+        const double ex = v[c][0] - v[b][0], ey = v[c][1] - v[b][1], ez = v[c][2] - v[b][2];
+        const float half = (float)(0.5 * sqrt(ex * ex + ey * ey + ez * ez));
+        r[kHalf + 4 * a] = id[b] < id[c] ? half : -half;
+        r[kEdge + 4 * a] = __int_as_float(fei[3 * f + a]);
+        for (int d = 0; d < 3; ++d) r[kA + 4 * a + d] = A[a][d];
+        const float na = n[0] * A[a][0] + n[1] * A[a][1] + n[2] * A[a][2];
+        ok = ok && na * na <= 1e-10f * nn * r[kAA + a];
+    }
+    r[kRho2] = ok ? rho2 : __int_as_float(0x7fc00000);
+    r[31] = 0.f;
+    float4* out = reinterpret_cast<float4*>(rec) + (kRec / 4) * f;
+    for (int q = 0; q < kRec / 4; ++q) out[q] = make_float4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+}
+
+// ---------------------------------------------------------------------------------------
+// the rule of a pair.  Both kernels below evaluate it and take disjoint sets of pairs, so its
+// arithmetic is spelled out with rounding intrinsics (no contraction that differs by context).
+// ---------------------------------------------------------------------------------------
+__device__ __forceinline__ float centre_dist2(float dx, float dy, float dz) {
+    return __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
+}
+
+template <int NX>
+__device__ __forceinline__ int pair_tier(float r2, float rho2p, float rho2q, float k2) {
+    // fmaxf drops a NaN operand; the sum does not
+    const float rho2 = __fadd_rn(fmaxf(rho2p, rho2q), __fmul_rn(0.f, __fadd_rn(rho2p, rho2q)));
+    const float u = __fmul_rn(rho2, __frcp_rn(r2)), q = __fmul_rn(k2, rho2);
+    const float u2 = __fmul_rn(u, u), q2 = __fmul_rn(q, q);
+    const bool t1 = __fmaf_rn(2.7e-4f, q2, __fmul_rn(3.2e-2f, u2)) <= 2e-6f;
+    if (NX == 3) return t1 ? 2 : 4;
+    if (t1) return 1;
+    if (__fmaf_rn(1.2e-5f, __fmul_rn(q2, q), __fmul_rn(0.4f, __fmul_rn(u2, u))) <= 5e-7f) return 2;
+    const bool t3 = __fmaf_rn(1.5e-6f, __fmul_rn(q2, q2), __fmul_rn(0.73f, __fmul_rn(u2, u2))) <= 6e-7f;
+    return t3 && q <= 0.64f ? 3 : 4;
+}
+
+// The centroid distance of a pair in two floats -- the subtraction's error (TwoSum), the centroids'
+// low parts, the squares' errors and the square root's -- and e^{-jkR_c} = c - j s from it, the
+// wavenumber in turns as kth + ktl.  d = fl(c_p - c_q).
+struct Centre {
+    float r2, r, ri, ril, c, s;  // R^2, R, 1/R (ri + ril), cos and sin of k R
+    // -e^{-jkR} j q / R in two floats (hi + lo): the entry's charge term at the centroids, common
+    // to its nine entries and cancelling between an entry's four face pairs to (kh)^2 of itself
+    float br, brl, bi, bil;
+};
+__device__ __forceinline__ Centre pair_centre(const float4& p, const float4& pl, const float4& q, const float4& ql,
+                                              float dx, float dy, float dz, float kth, float ktl, float q4) {
+    Centre o;
+    const float bx = dx - p.x, by = dy - p.y, bz = dz - p.z;
+    const float ex = ((p.x - (dx - bx)) - (q.x + bx)) + (pl.x - ql.x);
+    const float ey = ((p.y - (dy - by)) - (q.y + by)) + (pl.y - ql.y);
+    const float ez = ((p.z - (dz - bz)) - (q.z + bz)) + (pl.z - ql.z);
+    // (rounding intrinsics: a contraction of these sums would void their error terms)
+    const float sx = __fmul_rn(dx, dx), sy = __fmul_rn(dy, dy), sz = __fmul_rn(dz, dz);
+    const float s1 = __fadd_rn(sx, sy), b1 = __fsub_rn(s1, sx);
+    o.r2 = __fadd_rn(s1, sz);
+    const float b2 = __fsub_rn(o.r2, s1);
+    float lo = (fmaf(dx, dx, -sx) + fmaf(dy, dy, -sy)) + fmaf(dz, dz, -sz);
+    lo += ((sx - (s1 - b1)) + (sy - b1)) + ((s1 - (o.r2 - b2)) + (sz - b2));
+    lo = fmaf(2.f, fmaf(dx, ex, fmaf(dy, ey, dz * ez)), lo);
+    o.ri = rsqrtf(o.r2);
+    o.r = __fmul_rn(o.r2, o.ri);
+    const float rl = (fmaf(-o.r, o.r, o.r2) + lo) * (0.5f * o.ri);
+    o.ril = o.ri * fmaf(-o.r, o.ri, 1.f) - o.ri * o.ri * rl;
+    const float t = __fmul_rn(kth, o.r), te = fmaf(kth, rl, fmaf(ktl, o.r, fmaf(kth, o.r, -t)));
+    const float f0 = t - rintf(t), f = __fadd_rn(f0, te);
+    sincospif(2.f * f, &o.s, &o.c);
+    const float fl = 6.2831853f * (te - __fsub_rn(f, f0)), g = __fmul_rn(q4, o.ri), gl = fmaf(q4, o.ri, -g) + q4 * o.ril;
+    const float pr = __fmul_rn(g, o.s), pi = __fmul_rn(g, o.c);
+    o.br = -pr;
+    o.bi = -pi;
+    o.brl = -(fmaf(g, o.s, -pr) + fmaf(gl, o.s, g * o.c * fl));
+    o.bil = -(fmaf(g, o.c, -pi) + fmaf(gl, o.c, -g * o.s * fl));
+    return o;
+}
+
+// A squared centroid distance from which every pair of faces with rho^2 <= rho2 is in tier 1 (for gaussQR 3,
+// in tier 2): pair_tier is monotone in both, and the factor covers its rounding.  Infinite where
+// there is none, NaN for a NaN.
+__device__ __forceinline__ float far_limit(float rho2, float k2) {
+    const float q = k2 * rho2, rest = 2e-6f - 2.7e-4f * q * q;
+    return rest > 2e-8f ? 1.001f * rho2 * sqrtf(3.2e-2f / rest) : rho2 == rho2 ? __int_as_float(0x7f800000) : rho2;
+}
+
+// One mesh of a launch: all meshes of a batch share the arrays, desc as in the batched kernels
+// (n_mesh 0: one mesh, its values as arguments).
+struct TierArgs {
+    const float* verts;
+    const int32_t* faces;
+    const float* areas;
+    const float* normals;
+    const float* rec;
+    const float *gpx, *gwx, *gpy, *gwy;
+    const int64_t* desc;   // batch: [n_mesh, 6]
+    const int64_t* boff;   // batch: first block of each mesh
+    const double* ks;      // batch: wavenumbers
+    int n_mesh;
+    int64_t nf, n_edges;   // single mesh
+    double k;
+    float* z;
+};
+
+struct MeshRef {
+    int64_t f0, nf, pitch, block;
+    double k;
+    float* z;
+};
+
+__device__ __forceinline__ MeshRef find_mesh(const TierArgs& a) {
+    MeshRef m;
+    if (a.n_mesh == 0) {
+        m.f0 = 0;
+        m.nf = a.nf;
+        m.pitch = a.n_edges;
+        m.block = blockIdx.x;
+        m.k = a.k;
+        m.z = a.z;
+        return m;
+    }
+    int lo = 0, hi = a.n_mesh - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (__ldg(a.boff + mid) <= (int64_t)blockIdx.x) lo = mid;
+        else hi = mid - 1;
+    }
+    const int64_t* d = a.desc + 6 * lo;
+    const int64_t ne = __ldg(d + 2);
+    m.f0 = __ldg(d);
+    m.nf = __ldg(d + 1);
+    m.pitch = ne + (ne & 1);
+    m.block = (int64_t)blockIdx.x - __ldg(a.boff + lo);
+    m.k = __ldg(a.ks + lo);
+    m.z = a.z + 2 * __ldg(d + 3);
+    return m;
+}
+
+// ---------------------------------------------------------------------------------------
+// tier 1.  A thread keeps one source face q and meets the block's test faces.  With centroids
+// c_p, c_q, D = c_p - c_q, corners A_a, B_b relative to them, the rule points are s A_a and
+// s' B_b, and everything the entry needs is built from the scalars m_ab = A_a.B_b, D.A_a,
+// D.B_b, A_a.A_a', n.B_b, n.D (n the test normal) and from sums of w w' G and w w' h over the
+// 36 points, h = G (1 + jkR) / R^2, weighted by powers of s, s':
+//   sum G f_m.f_n    = T - sum_b m_mb M0b - sum_a m_an Ma0 + m_mn M00
+//   MFIE part        = R_m - (n.B_n) S_m + (n.B_n - n.D)(U - U_m) + sum_a m_an Z_a - m_mn Z
+// (h (x - A_m) . [r (n.rho) - rho (n.r)] with r = x - y, rho = y - B_n, summed term by term).
+// The distance comes as R^2 = R_c^2 + sigma with sigma from the scalars (two operations), and
+// R - R_c = (sigma - (R - R_c)^2) / (2 R_c), whose rounding is that of the small difference: the
+// phase of an evaluation is k (R - R_c) relative to the pair's e^{-jkR_c}, which is computed
+// once in two-float arithmetic.  An FP32 kR instead costs 1e-7 kR of phase per face pair,
+// which the cancellation between an entry's four face pairs raises to 1e-5 .. 6e-5 of it.
+//
+// Lanes of a packed register are the two orbits of the source rule; they are weighted and
+// added after the loop.  Bound: FMA pipe, 468 packed and ~600 scalar operations per pair.
+// ---------------------------------------------------------------------------------------
+__device__ __forceinline__ float lanes(float2 v, float wx, float wy) { return fmaf(v.x, wx, v.y * wy); }
+
+template <int NX>
+__global__ void __launch_bounds__(128, 2) far_pairs_kernel(const TierArgs args, int rows_per_block) {
+    __shared__ float4 s_rec[32 * (kRec / 4)];
+    const MeshRef m = find_mesh(args);
+    const int64_t col_tiles = (m.nf + 127) / 128;
+    const int64_t p0 = (m.block / col_tiles) * rows_per_block;
+    const int64_t q = (m.block % col_tiles) * 128 + threadIdx.x;
+    const int np = (int)min((int64_t)rows_per_block, m.nf - p0);
+    const float4* rec = reinterpret_cast<const float4*>(args.rec) + (kRec / 4) * m.f0;
+    for (int i = threadIdx.x; i < np * (kRec / 4); i += 128) s_rec[i] = __ldg(rec + (kRec / 4) * p0 + i);
+    __syncthreads();
+    if (q >= m.nf) return;
+    const float4* rq = rec + (kRec / 4) * q;
+    const float4 q0 = __ldg(rq), q1 = __ldg(rq + 1), q2 = __ldg(rq + 2), q3 = __ldg(rq + 3), q4 = __ldg(rq + 4),
+                 q5 = __ldg(rq + 5), q6 = __ldg(rq + 6);
+    const float B[3][3] = {{q2.x, q2.y, q2.z}, {q3.x, q3.y, q3.z}, {q4.x, q4.y, q4.z}};
+    const float BB[3] = {q6.x, q6.y, q6.z}, hq[3] = {q4.w, q5.w, q6.w};
+    const int col[3] = {__float_as_int(q1.w), __float_as_int(q2.w), __float_as_int(q3.w)};
+    const float k = (float)m.k, k2 = k * k;
+    const double kt = m.k * kInv2Pi;
+    const float kth = (float)kt, ktl = (float)(kt - (double)kth), four_k = 4.f / k;
+    constexpr float SA = -0.16666371f, SB = 0.00828212f;                     // sin
+    constexpr float CA = -0.49999997f, CB = 0.04166572f, CC = -0.00138007f;  // cos
+    const float wqx = kW1, wqy = kW2, wsx = kW1 * kS1, wsy = kW2 * kS2;
+#pragma unroll 1
+    for (int i = 0; i < np; ++i) {
+        const float4* rp = s_rec + (kRec / 4) * i;
+        const float4 p0v = rp[0];
+        const float dx = p0v.x - q0.x, dy = p0v.y - q0.y, dz = p0v.z - q0.z;
+        if (pair_tier<NX>(centre_dist2(dx, dy, dz), p0v.w, q0.w, k2) != 1) continue;
+        const float4 p1v = rp[1], p2v = rp[2], p3v = rp[3], p4v = rp[4], p5v = rp[5], p6v = rp[6], p7v = rp[7];
+        const float A[3][3] = {{p2v.x, p2v.y, p2v.z}, {p3v.x, p3v.y, p3v.z}, {p4v.x, p4v.y, p4v.z}};
+        const float AA[3] = {p6v.x, p6v.y, p6v.z};
+        const Centre ce = pair_centre(p0v, p1v, q0, q1, dx, dy, dz, kth, ktl, four_k);
+        const float Rc2 = ce.r2, R0 = ce.r, kp = k * (0.5f * ce.ri), C = ce.c, S = ce.s;
+        const float2 G0 = bc(ce.ri);
+        float mm[3][3], DA[3], nB[3];
+        float2 V[3];  // -(sigma's source part) per b, lanes the two orbits
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            DA[a] = fmaf(dz, A[a][2], fmaf(dy, A[a][1], dx * A[a][0]));
+            nB[a] = fmaf(p5v.z, B[a][2], fmaf(p5v.y, B[a][1], p5v.x * B[a][0]));
+            const float DB = fmaf(dz, B[a][2], fmaf(dy, B[a][1], dx * B[a][0]));
+            V[a] = make_float2(kS1 * (2.f * DB - kS1 * BB[a]), kS2 * (2.f * DB - kS2 * BB[a]));
+#pragma unroll
+            for (int b = 0; b < 3; ++b)
+                mm[a][b] = fmaf(A[a][2], B[b][2], fmaf(A[a][1], B[b][1], A[a][0] * B[b][0]));
+        }
+        const float nD = fmaf(p5v.z, dz, fmaf(p5v.y, dy, p5v.x * dx));
+
+        float2 Mr[3][3], Mi[3][3], M0r[3], M0i[3], Xr[3][3], Xi[3][3], X0r[3], X0i[3], Xgr[3], Xgi[3];
+#pragma unroll
+        for (int b = 0; b < 3; ++b) {
+            M0r[b] = M0i[b] = X0r[b] = X0i[b] = Xgr[b] = Xgi[b] = bc(0.f);
+#pragma unroll
+            for (int a = 0; a < 3; ++a) Mr[a][b] = Mi[a][b] = Xr[a][b] = Xi[a][b] = bc(0.f);
+        }
+#pragma unroll 1
+        for (int o = 0; o < 2; ++o) {
+            const float s = o ? kS2 : kS1, w = o ? kW2 : kW1;
+            const float2 W = bc(w), WS = bc(w * s), K2 = make_float2(2.f * s * kS1, 2.f * s * kS2);
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const float sd = s * DA[a], gam = fmaf(s * s, AA[a], sd);
+                const float2 U = bc(-(gam + sd)), WG = bc(w * gam);
+#pragma unroll
+                for (int b = 0; b < 3; ++b) {
+                    const float2 ns = fma2(bc(mm[a][b]), K2, add2(U, V[b]));  // -sigma
+                    const float2 r2 = sub2(bc(Rc2), ns);
+                    float2 rinv;
+                    rinv.x = rsqrtf(r2.x);
+                    rinv.y = rsqrtf(r2.y);
+                    const float2 R = mul2(r2, rinv), d0 = sub2(R, bc(R0));
+                    const float2 th = mul2(fma2(d0, d0, ns), bc(kp));  // -k (R - R_c)
+                    // |th| <= 0.43 by the rule of tier 1: polynomials (least squares on that range, off
+                    // by 5e-8 of th and 3e-10); the SFU's error, 4e-7 and alike over a pair, would not average out
+                    const float2 t = mul2(th, th);
+                    const float2 sn = mul2(th, fma2(t, fma2(t, bc(SB), bc(SA)), bc(1.f)));
+                    const float2 cs = fma2(t, fma2(t, fma2(t, bc(CC), bc(CB)), bc(CA)), bc(1.f));
+                    const float2 gr = mul2(rinv, cs), gi = mul2(rinv, sn), ri2 = mul2(rinv, rinv), kR = mul2(bc(k), R);
+                    const float2 hr = mul2(sub2(gr, mul2(gi, kR)), ri2), hi = mul2(fma2(gr, kR, gi), ri2);
+                    // sums of G - 1/R_c: the constant drops out of the first moments (the corners' sums
+                    // vanish) and is carried through M00 in two floats (ce.b)
+                    const float2 gd = sub2(gr, G0);
+                    Mr[a][b] = fma2(WS, gd, Mr[a][b]);
+                    Mi[a][b] = fma2(WS, gi, Mi[a][b]);
+                    M0r[b] = fma2(W, gd, M0r[b]);
+                    M0i[b] = fma2(W, gi, M0i[b]);
+                    Xr[a][b] = fma2(WS, hr, Xr[a][b]);
+                    Xi[a][b] = fma2(WS, hi, Xi[a][b]);
+                    X0r[b] = fma2(W, hr, X0r[b]);
+                    X0i[b] = fma2(W, hi, X0i[b]);
+                    Xgr[b] = fma2(WG, hr, Xgr[b]);
+                    Xgi[b] = fma2(WG, hi, Xgi[b]);
+                }
+            }
+        }
+        // sums over the source orbits; re and im in the lanes of the complex values below
+        float2 E[3][3], H[3][3];
+        {
+            float2 Tr = bc(0.f), Ti = bc(0.f), Ma[3], Mb[3], M00;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                Mb[a] = make_float2(lanes(M0r[a], wsx, wsy), lanes(M0i[a], wsx, wsy));
+                const float2 sr = add2(add2(Mr[a][0], Mr[a][1]), Mr[a][2]), si = add2(add2(Mi[a][0], Mi[a][1]), Mi[a][2]);
+                Ma[a] = make_float2(lanes(sr, wqx, wqy), lanes(si, wqx, wqy));
+#pragma unroll
+                for (int b = 0; b < 3; ++b) {
+                    Tr = fma2(bc(mm[a][b]), Mr[a][b], Tr);
+                    Ti = fma2(bc(mm[a][b]), Mi[a][b], Ti);
+                }
+            }
+            const float2 s0r = add2(add2(M0r[0], M0r[1]), M0r[2]), s0i = add2(add2(M0i[0], M0i[1]), M0i[2]);
+            M00 = make_float2(lanes(s0r, wqx, wqy), lanes(s0i, wqx, wqy));
+            const float2 M0f = add2(M00, make_float2(ce.ri, 0.f));
+            const float2 T = fma2(bc(-4.f / k2), M00, make_float2(lanes(Tr, wsx, wsy), lanes(Ti, wsx, wsy)));
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const float2 u = fma2(bc(mm[a][2]), Mb[2], fma2(bc(mm[a][1]), Mb[1], mul2(bc(mm[a][0]), Mb[0])));
+                const float2 Tu = sub2(T, u);
+#pragma unroll
+                for (int b = 0; b < 3; ++b) {
+                    const float2 v = fma2(bc(mm[2][b]), Ma[2], fma2(bc(mm[1][b]), Ma[1], mul2(bc(mm[0][b]), Ma[0])));
+                    E[a][b] = fma2(bc(mm[a][b]), M0f, sub2(Tu, v));
+                }
+            }
+        }
+        {
+            float2 Usr = bc(0.f), Usi = bc(0.f), Pa[3], Qa[3], X0[3];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                X0[a] = make_float2(lanes(X0r[a], wsx, wsy), lanes(X0i[a], wsx, wsy));
+                const float2 sr = add2(add2(Xr[a][0], Xr[a][1]), Xr[a][2]), si = add2(add2(Xi[a][0], Xi[a][1]), Xi[a][2]);
+                Qa[a] = make_float2(lanes(sr, wqx, wqy), lanes(si, wqx, wqy));
+                float2 pr = mul2(bc(nB[0]), Xr[a][0]), pi = mul2(bc(nB[0]), Xi[a][0]);
+                pr = fma2(bc(nB[2]), Xr[a][2], fma2(bc(nB[1]), Xr[a][1], pr));
+                pi = fma2(bc(nB[2]), Xi[a][2], fma2(bc(nB[1]), Xi[a][1], pi));
+                Pa[a] = make_float2(lanes(pr, wsx, wsy), lanes(pi, wsx, wsy));
+#pragma unroll
+                for (int b = 0; b < 3; ++b) {
+                    Usr = fma2(bc(mm[a][b]), Xr[a][b], Usr);
+                    Usi = fma2(bc(mm[a][b]), Xi[a][b], Usi);
+                }
+            }
+            const float2 Us = make_float2(lanes(Usr, wsx, wsy), lanes(Usi, wsx, wsy));
+            const float2 q0r = add2(add2(X0r[0], X0r[1]), X0r[2]), q0i = add2(add2(X0i[0], X0i[1]), X0i[2]);
+            const float2 Q = make_float2(lanes(q0r, wqx, wqy), lanes(q0i, wqx, wqy));
+            const float2 gr = add2(add2(Xgr[0], Xgr[1]), Xgr[2]), gi = add2(add2(Xgi[0], Xgi[1]), Xgi[2]);
+            const float2 Qg = make_float2(lanes(gr, wqx, wqy), lanes(gi, wqx, wqy));
+            const float2 pgr = fma2(bc(nB[2]), Xgr[2], fma2(bc(nB[1]), Xgr[1], mul2(bc(nB[0]), Xgr[0])));
+            const float2 pgi = fma2(bc(nB[2]), Xgi[2], fma2(bc(nB[1]), Xgi[1], mul2(bc(nB[0]), Xgi[0])));
+            const float2 Pg = make_float2(lanes(pgr, wsx, wsy), lanes(pgi, wsx, wsy));
+            const float2 P = fma2(bc(nB[2]), X0[2], fma2(bc(nB[1]), X0[1], mul2(bc(nB[0]), X0[0])));
+            const float2 Z = sub2(mul2(bc(nD), Q), P);
+            float2 Za[3], Y[3];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) Za[a] = sub2(mul2(bc(nD), Qa[a]), Pa[a]);
+#pragma unroll
+            for (int b = 0; b < 3; ++b)
+                Y[b] = fma2(bc(mm[2][b]), Za[2], fma2(bc(mm[1][b]), Za[1], mul2(bc(mm[0][b]), Za[0])));
+            const float G[3][3] = {{AA[0], p7v.x, p7v.z}, {p7v.x, AA[1], p7v.y}, {p7v.z, p7v.y, AA[2]}};
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const float2 nDA = bc(-DA[a]);
+                float2 R = fma2(nDA, P, Pg), Sm = fma2(nDA, Q, Qg);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    R = fma2(bc(-G[a][c]), Pa[c], R);
+                    Sm = fma2(bc(-G[a][c]), Qa[c], Sm);
+                }
+                const float2 um = fma2(bc(mm[a][2]), X0[2], fma2(bc(mm[a][1]), X0[1], mul2(bc(mm[a][0]), X0[0])));
+                const float2 du = sub2(Us, um);
+#pragma unroll
+                for (int b = 0; b < 3; ++b) {
+                    const float2 t = fma2(bc(nB[b] - nD), du, fma2(bc(-nB[b]), Sm, R));
+                    H[a][b] = add2(t, fma2(bc(-mm[a][b]), Z, Y[b]));
+                }
+            }
+        }
+        const float hp[3] = {p4v.w, p5v.w, p6v.w};
+        const int row[3] = {__float_as_int(p1v.w), __float_as_int(p2v.w), __float_as_int(p3v.w)};
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            float2* zr = reinterpret_cast<float2*>(m.z) + (int64_t)row[a] * m.pitch;
+            const float ha = hp[a] * float(kInv4Pi);
+#pragma unroll
+            for (int b = 0; b < 3; ++b) {
+                // jk E + H, times e^{-jkR_c}, and the charge term at the centroids
+                const float re = fmaf(-k, E[a][b].y, H[a][b].x), im = fmaf(k, E[a][b].x, H[a][b].y), c = ha * hq[b];
+                atomicAdd(zr + col[b], make_float2(fmaf(c, ce.br, c * fmaf(im, S, fmaf(re, C, ce.brl))),
+                                                   fmaf(c, ce.bi, c * fmaf(-re, S, fmaf(im, C, ce.bil)))));
+            }
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------------------
+// tiers 2 and 3: the three entries (m, e2), m = 0 .. 2, of one face pair -- nt shared test points,
+// the NY x NY source points anchored at local edge e2.  Distances and phases as in tier 1, in
+// units of 1/k: with y = B + r1 E1 + r2 E2 from the centroid, sigma takes three operations per
+// evaluation.  Per test point the sums over the source points are S0 = sum G, and of G y and h y
+// by the source's two barycentric coordinates; with the origin at the anchor,
+// P = sum G y, H = sum h y the entry is
+//   sum_i w_i [ (x_i - A_m) . (jk P_i - n x (H_i x x_i)) - (4j/k) S0_i ],
+// whose vector is e1 E1 + e2 E2 + e3 x_i.  Bound: FMA pipe, 26 packed operations per two evaluations.
+// ---------------------------------------------------------------------------------------
+template <int NY>
+__device__ __forceinline__ void shared_test_entries(const float* __restrict__ rp, const float* __restrict__ rq, int e2,
+                                                    const float (*s_b)[4], int nt, const float4* s_s, float k,
+                                                    float kth, float ktl, float wsum, int64_t pitch,
+                                                    float* __restrict__ z) {
+    constexpr int NS = NY * NY, NP = (NS + 1) / 2;  // an odd count is padded with a zero weight
+    const float4* r4p = reinterpret_cast<const float4*>(rp);
+    const float4* r4q = reinterpret_cast<const float4*>(rq);
+    const float4 cp = r4p[0], cq = r4q[0];
+    const float dx = cp.x - cq.x, dy = cp.y - cq.y, dz = cp.z - cq.z;
+    // charge term at the centroids: 4/k / R, the sums below being over G / k
+    const Centre ce = pair_centre(cp, r4p[1], cq, r4q[1], dx, dy, dz, kth, ktl, 4.f * wsum / (k * k));
+    const float k2 = k * k, Rc2 = k2 * ce.r2, R0 = k * ce.r, hc = 0.5f * ce.ri / k;
+    const float2 G0 = bc(-ce.ri / k);
+    const int b1 = e2 == 2 ? 0 : e2 + 1, b2 = e2 == 0 ? 2 : e2 - 1;
+    const V3<float> b0 = v3<float>(rq[kA + 4 * e2], rq[kA + 4 * e2 + 1], rq[kA + 4 * e2 + 2]);
+    const V3<float> E1 = v3<float>(rq[kA + 4 * b1], rq[kA + 4 * b1 + 1], rq[kA + 4 * b1 + 2]) - b0;
+    const V3<float> E2 = v3<float>(rq[kA + 4 * b2], rq[kA + 4 * b2 + 1], rq[kA + 4 * b2 + 2]) - b0;
+    const V3<float> D = v3<float>(dx, dy, dz), o = D - b0;  // x' + o: the test point from the anchor
+    const V3<float> n = v3<float>(rp[kN], rp[kN + 1], rp[kN + 2]);
+    float2 wn[NP];  // -k^2 (|y|^2 - 2 D.y)
+#pragma unroll
+    for (int j = 0; j < 2 * NP; ++j) {
+        const float4 r = s_s[j];
+        const V3<float> y = b0 + r.x * E1 + r.y * E2;
+        (reinterpret_cast<float*>(&wn[j / 2]) + (j & 1))[0] = k2 * (2.f * dot(D, y) - dot(y, y));
+    }
+    const float nB1 = dot(n, E1), nB2 = dot(n, E2);
+    V3<float> er = v3<float>(0.f, 0.f, 0.f), ei = v3<float>(0.f, 0.f, 0.f);  // sum w e3 x
+    float f1r = 0.f, f1i = 0.f, f2r = 0.f, f2i = 0.f;                         // sum w e1, w e2
+    float t0r = 0.f, t0i = 0.f;                                               // sum w x.E - (4j/k) w S0
+#pragma unroll 1
+    for (int i = 0; i < nt; ++i) {
+        V3<float> xc = v3<float>(0.f, 0.f, 0.f);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) xc = xc + s_b[i][a] * v3<float>(rp[kA + 4 * a], rp[kA + 4 * a + 1], rp[kA + 4 * a + 2]);
+        const V3<float> x = xc + o;
+        const float2 U = bc(k2 * (2.f * dot(xc, b0 - D) - dot(xc, xc))), X1 = bc(2.f * k2 * dot(xc, E1)),
+                     X2 = bc(2.f * k2 * dot(xc, E2));
+        float2 s0r = bc(0.f), s0i = bc(0.f), p1r = bc(0.f), p1i = bc(0.f), p2r = bc(0.f), p2i = bc(0.f), h1r = bc(0.f),
+               h1i = bc(0.f), h2r = bc(0.f), h2i = bc(0.f);
+#pragma unroll
+        for (int j = 0; j < NP; ++j) {
+            const float4 ra = s_s[2 * j], rb = s_s[2 * j + 1];  // (r1, r2, weight)
+            const float2 c1 = make_float2(ra.x, rb.x), c2 = make_float2(ra.y, rb.y), w = make_float2(ra.z, rb.z);
+            const float2 ns = fma2(c1, X1, fma2(c2, X2, add2(wn[j], U)));  // -k^2 sigma
+            const float2 r2 = sub2(bc(Rc2), ns);
+            float2 rinv;
+            rinv.x = rsqrtf(r2.x);
+            rinv.y = rsqrtf(r2.y);
+            const float2 kR = mul2(r2, rinv), d0 = sub2(kR, bc(R0));
+            const float2 th = mul2(fma2(d0, d0, ns), bc(hc));  // -k (R - R_c)
+            float2 sn, cs;
+            __sincosf(th.x, &sn.x, &cs.x);
+            __sincosf(th.y, &sn.y, &cs.y);
+            const float2 g = mul2(w, rinv), gr = mul2(g, cs), gi = mul2(g, sn), ri2 = mul2(rinv, rinv);
+            const float2 hr = mul2(sub2(gr, mul2(gi, kR)), ri2), hi = mul2(fma2(gr, kR, gi), ri2);
+            s0r = add2(s0r, fma2(w, G0, gr));  // of G - 1/R_c, as in tier 1
+            s0i = add2(s0i, gi);
+            p1r = fma2(c1, gr, p1r);
+            p1i = fma2(c1, gi, p1i);
+            p2r = fma2(c2, gr, p2r);
+            p2i = fma2(c2, gi, p2i);
+            h1r = fma2(c1, hr, h1r);
+            h1i = fma2(c1, hi, h1i);
+            h2r = fma2(c2, hr, h2r);
+            h2i = fma2(c2, hi, h2i);
+        }
+        const float w = s_b[i][3], wk = w * k, wk2 = w * k2, nx = dot(n, x), xx = dot(x, x), x1 = dot(x, E1), x2 = dot(x, E2);
+        const float u1r = h1r.x + h1r.y, u1i = h1i.x + h1i.y, u2r = h2r.x + h2r.y, u2i = h2i.x + h2i.y;
+        // E = e1 E1 + e2 E2 + e3 x:  e1 = jk p1 - k^2 h1 (n.x),  e3 = k^2 (h1 n.E1 + h2 n.E2)
+        const float e1r = -fmaf(wk2 * nx, u1r, wk * (p1i.x + p1i.y)), e1i = fmaf(-wk2 * nx, u1i, wk * (p1r.x + p1r.y));
+        const float e2r = -fmaf(wk2 * nx, u2r, wk * (p2i.x + p2i.y)), e2i = fmaf(-wk2 * nx, u2i, wk * (p2r.x + p2r.y));
+        const float e3r = wk2 * fmaf(nB1, u1r, nB2 * u2r), e3i = wk2 * fmaf(nB1, u1i, nB2 * u2i);
+        f1r += e1r;
+        f1i += e1i;
+        f2r += e2r;
+        f2i += e2i;
+        er = er + e3r * x;
+        ei = ei + e3i * x;
+        const float q = 4.f * w / k;
+        t0r += fmaf(x1, e1r, fmaf(x2, e2r, fmaf(xx, e3r, q * (s0i.x + s0i.y))));
+        t0i += fmaf(x1, e1i, fmaf(x2, e2i, fmaf(xx, e3i, -q * (s0r.x + s0r.y))));
+    }
+    er = er + f1r * E1 + f2r * E2;
+    ei = ei + f1i * E1 + f2i * E2;
+    const float sc = 2.f * k * rq[kHalf + 4 * e2];  // the sums lack a factor k (1/R -> 1/(kR))
+    const int64_t col = __float_as_int(rq[kEdge + 4 * e2]);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float c = sc * rp[kHalf + 4 * a];
+        const V3<float> A = v3<float>(rp[kA + 4 * a], rp[kA + 4 * a + 1], rp[kA + 4 * a + 2]) + o;
+        const float re = t0r - dot(A, er), im = t0i - dot(A, ei);
+        const int64_t row = __float_as_int(rp[kEdge + 4 * a]);
+        atomicAdd(reinterpret_cast<float2*>(z) + row * pitch + col,
+                  make_float2(fmaf(c, ce.br, c * fmaf(im, ce.s, fmaf(re, ce.c, ce.brl))),
+                              fmaf(c, ce.bi, c * fmaf(-re, ce.s, fmaf(im, ce.c, ce.bil)))));
+    }
+}
+
+// The pairs outside tier 1 of a block's tile of tp test x tq source faces (at most kTilePairs): sorted
+// into lists in shared memory, then worked off by all threads -- CLOSE: tier 4, one (pair, e1, e2)
+// entry per thread; else tiers 2 and 3, (pair, e2) items -- so that the few close pairs of a tile
+// leave no lanes idle.  A tile without such pairs ends after the tests.  Two launches: in one
+// kernel the two bodies spilled at 128 registers.
+constexpr int kTilePairs = 1024;
+
+template <int NX, int NY, bool CLOSE>
+__global__ void __launch_bounds__(128, NX <= 4 ? 4 : 3) close_pairs_kernel(const TierArgs args, int tp, int tq) {
+    __shared__ float4 s_t[NX * NX], s_s[NY * NY], s_src[(NY * NY + 1) / 2 * 2];
+    __shared__ float s_b[19][4];
+    __shared__ float4 s_p[256], s_q[256];
+    __shared__ uint16_t s_list[CLOSE ? 1 : 2][kTilePairs];
+    __shared__ int s_n[2], s_rho;
+    const MeshRef m = find_mesh(args);
+    const int64_t col_tiles = (m.nf + tq - 1) / tq;
+    const int64_t p0 = (m.block / col_tiles) * tp, q0 = (m.block % col_tiles) * tq;
+    const int np = (int)min((int64_t)tp, m.nf - p0), nq = (int)min((int64_t)tq, m.nf - q0);
+    const float4* rec4 = reinterpret_cast<const float4*>(args.rec) + (kRec / 4) * m.f0;
+    if (threadIdx.x < 2) s_n[threadIdx.x] = 0;
+    // the tile's largest rho^2 (a NaN wins: as bits it is above every finite value)
+    if (threadIdx.x == 0) s_rho = 0;
+    __syncthreads();
+    int top = 0;
+    for (int i = threadIdx.x; i < np + nq; i += 128) {
+        const float4 r = __ldg(rec4 + (kRec / 4) * (i < np ? p0 + i : q0 + (i - np)));
+        (i < np ? s_p[i] : s_q[i - np]) = r;
+        top = max(top, __float_as_int(r.w));
+    }
+    atomicMax(&s_rho, top);
+    const float k = (float)m.k, k2 = k * k;
+    __syncthreads();
+    // tq is a power of two up to 128: a thread keeps one source face and steps through the test faces
+    const float limit = CLOSE || NX > 3 ? far_limit(__int_as_float(s_rho), k2) : __int_as_float(0x7f800000);
+    const int b = threadIdx.x & (tq - 1);
+    if (b < nq) {
+        const float4 q = s_q[b];
+        for (int a = threadIdx.x / tq; a < np; a += 128 / tq) {
+            const float4 p = s_p[a];
+            const float r2 = centre_dist2(p.x - q.x, p.y - q.y, p.z - q.z);
+            if (r2 >= limit) continue;
+            const int t = pair_tier<NX>(r2, p.w, q.w, k2);
+            if (CLOSE ? t == 4 : (t == 2 || t == 3)) {
+                const int l = CLOSE ? 0 : t - 2;
+                s_list[l][atomicAdd(&s_n[l], 1)] = (uint16_t)(a * tq + b);
+            }
+        }
+    }
+    __syncthreads();
+    const int n0 = s_n[0], n1 = s_n[1];
+    if (n0 + n1 == 0) return;
+    stage_rules<NX, NY>(args.gpx, args.gwx, args.gpy, args.gwy, s_t, s_s);
+    if constexpr (!CLOSE)
+        if (threadIdx.x < 76) (&s_b[0][0])[threadIdx.x] = (&c_test[0][0])[threadIdx.x];
+    __syncthreads();
+    const float* rec = args.rec + kRec * m.f0;
+    if constexpr (CLOSE) {
+        for (int i = threadIdx.x; i < 9 * n0; i += 128) {
+            const int c = s_list[0][i / 9], e = i % 9;
+            const int64_t p = p0 + c / tq, q = q0 + (c & (tq - 1));
+            float re, im;
+            mom_entry_fast<NX, NY>(args.verts, args.faces, args.areas, args.normals, s_t, s_s, k, m.f0 + p, e / 3,
+                                   m.f0 + q, e % 3, &re, &im);
+            const int64_t row = __float_as_int(rec[kRec * p + kEdge + 4 * (e / 3)]);
+            const int64_t col = __float_as_int(rec[kRec * q + kEdge + 4 * (e % 3)]);
+            atomicAdd(reinterpret_cast<float2*>(m.z) + row * m.pitch + col, make_float2(re, im));
+        }
+    } else {
+        if (threadIdx.x < (NY * NY + 1) / 2 * 2) {  // barycentric form of the source rule: (r3 - r4, r4, weight)
+            const float4 r = threadIdx.x < NY * NY ? s_s[threadIdx.x] : make_float4(0.5f, 0.25f, 0.f, 0.f);
+            s_src[threadIdx.x] = make_float4(r.x - r.y, r.y, r.z, 0.f);
+        }
+        __syncthreads();
+        float wsum = 0.f;
+        for (int j = 0; j < NY * NY; ++j) wsum += s_s[j].z;
+        const double kt = m.k * kInv2Pi;
+        const float kth = (float)kt, ktl = (float)(kt - (double)kth);
+#pragma unroll 1
+        for (int t = 1; t >= 0; --t) {
+            const int n = 3 * (t ? n1 : n0);
+            for (int i = threadIdx.x; i < n; i += 128) {
+                const int c = s_list[t][i / 3];
+                shared_test_entries<NY>(rec + kRec * (p0 + c / tq), rec + kRec * (q0 + (c & (tq - 1))), i % 3,
+                                        t ? s_b + 7 : s_b, t ? 12 : 7, s_src, k, kth, ktl, wsum, m.pitch, m.z);
+            }
+        }
+    }
+}
+
+}  // namespace
+
+// Tile sizes: 32 test faces per block of tier 1 once that leaves 8 blocks per SM (its per-thread
+// source set-up is amortised over them), 8 below; the close pairs' tiles hold 1024 pairs on
+// large meshes, fewer on small ones: 8 times the chip's 608 resident blocks, so that the last
+// wave is a small part (1280 faces in tier 4: 2.83 ms with 2.6 waves of 1024-pair tiles, 2.56 ms as edge rows).
+void mom_tier_tiles(int64_t nf, int* rows, int* tp, int* tq) {
+    *rows = nf >= 5000 ? 32 : 8;
+    const double per_block = (double)nf * (double)nf / 4864.0;
+    *tp = per_block >= 1024 ? 16 : per_block >= 256 ? 8 : per_block >= 64 ? 4 : 7;
+    *tq = per_block >= 64 ? 4 * *tp : 2;  // the smallest, 14 pairs: 126 entries, one per thread
+}
+
+int64_t mom_tier_blocks(int64_t nf, int64_t tp, int64_t tq) { return ((nf + tp - 1) / tp) * ((nf + tq - 1) / tq); }
+
+template <int NX, int NY>
+static int launch_tiers(TierArgs a, int64_t far_blocks, int64_t close_blocks, int rows, int tp, int tq,
+                        const int64_t* far_off, const int64_t* close_off, cudaStream_t s) {
+    if (far_blocks > 0x7fffffffLL || close_blocks > 0x7fffffffLL)
+        return set_error(MB_ERR_SIZE, "mesh too large for one launch");
+    a.boff = close_off;
+    close_pairs_kernel<NX, NY, true><<<(unsigned)close_blocks, 128, 0, s>>>(a, tp, tq);
+    close_pairs_kernel<NX, NY, false><<<(unsigned)close_blocks, 128, 0, s>>>(a, tp, tq);
+    if (NX > 3) {
+        a.boff = far_off;
+        far_pairs_kernel<NX><<<(unsigned)far_blocks, 128, 0, s>>>(a, rows);
+    }
+    return check_launch("mom tiers");
+}
+
+static int tier_records(const float* verts, const int32_t* faces, const float* normals, const int32_t* fei, int64_t nf,
+                        const float* gpx, const float* gwx, int nx, const float* gpy, const float* gwy, int ny,
+                        float* rec, cudaStream_t s) {
+    face_record_kernel<<<(unsigned)((nf + 127) / 128), 128, 0, s>>>(verts, faces, normals, fei, nf, gpx, gwx, nx, gpy,
+                                                                    gwy, ny, rec);
+    return check_launch("face records");
+}
+
+bool mom_tier_rule(int nx, int ny) { return nx >= 3 && nx <= 5 && ny == nx - 1; }
+
+#define MB_TIERS(...)                                                    \
+    (nx == 4 ? launch_tiers<4, 3>(__VA_ARGS__) : nx == 3 ? launch_tiers<3, 2>(__VA_ARGS__) : launch_tiers<5, 4>(__VA_ARGS__))
+
+int launch_mom_tiers(const float* verts, const int32_t* faces, int64_t nf, const float* areas, const float* normals,
+                     const int32_t* fei, int64_t n_edges, const float* gpx, const float* gwx, int nx, const float* gpy,
+                     const float* gwy, int ny, double k, float* rec, float* z, cudaStream_t s) {
+    if (nf <= 0) return MB_OK;
+    if (int rc = tier_records(verts, faces, normals, fei, nf, gpx, gwx, nx, gpy, gwy, ny, rec, s)) return rc;
+    int rows, tp, tq;
+    mom_tier_tiles(nf, &rows, &tp, &tq);
+    const TierArgs a{verts, faces, areas, normals, rec, gpx, gwx, gpy, gwy, nullptr, nullptr, nullptr, 0, nf, n_edges, k, z};
+    return MB_TIERS(a, mom_tier_blocks(nf, rows, 128), mom_tier_blocks(nf, tp, tq), rows, tp, tq, nullptr, nullptr, s);
+}
+
+int launch_mom_tiers_batched(const float* verts, const int32_t* faces, int64_t total_faces, const float* areas,
+                             const float* normals, const int32_t* fei, const int64_t* desc, const int64_t* far_off,
+                             int64_t far_blocks, const int64_t* close_off, int64_t close_blocks, int rows, int tp, int tq,
+                             const double* ks, int n_mesh, const float* gpx, const float* gwx, int nx, const float* gpy,
+                             const float* gwy, int ny, float* rec, float* z, cudaStream_t s) {
+    if (total_faces <= 0) return MB_OK;
+    if (int rc = tier_records(verts, faces, normals, fei, total_faces, gpx, gwx, nx, gpy, gwy, ny, rec, s)) return rc;
+    const TierArgs a{verts, faces, areas, normals, rec, gpx, gwx, gpy, gwy, desc, nullptr, ks, n_mesh, 0, 0, 0.0, z};
+    return MB_TIERS(a, far_blocks, close_blocks, rows, tp, tq, far_off, close_off, s);
+}
+
+}  // namespace mb

@@ -174,8 +174,11 @@ def assemble_Z_rwg(verts, faces, face_areas, face_normals, face_edge_indices, n_
     contributions summed by one thread and stored once, no atomics and no zeroing; rows of
     ``out`` are OVERWRITTEN, not accumulated into (half the DRAM traffic of the edge order, but
     ~3 % slower at 20480 faces: neighbouring threads read scattered source faces).
-    ``order="auto"`` (default) takes the edge order when it applies (float32, a fast rule, no
-    ``rows``, every edge on at most two faces) and the face order otherwise.
+    ``order="tiers"`` (float32, gaussQR 3-5, no ``rows``): each face pair's quadrature sized by
+    its separation -- the reference's points on close pairs, one set of fewer points of the same
+    exactness for all nine entries of the others; equal to the other orders within FP32 rounding.
+    ``order="auto"`` (default) takes "tiers" when it applies, else the edge order when it applies
+    (float32, a fast rule, no ``rows``, every edge on at most two faces) and the face order otherwise.
     ``edge_rows_map``: ``edge_rows(face_edge_indices, F, E)`` computed once by the caller.
     ``out_host`` (complex64 [E, E] CPU tensor, pinned for overlap): Z goes to host memory,
     assembled in ``chunks`` Z-row ranges with each range's copy overlapping the next range's
@@ -206,12 +209,22 @@ def assemble_Z_rwg(verts, faces, face_areas, face_normals, face_edge_indices, n_
         return out_host
     if order == "auto":
         order = "faces"
-        if dt == torch.float32 and rows is None and (nx, ny) in _EDGE_RULES:
+        if dt == torch.float32 and rows is None and (nx, ny) in _TIER_RULES:
+            order = "tiers"
+        elif dt == torch.float32 and rows is None and (nx, ny) in _EDGE_RULES:
             try:
                 edge_rows_map = edge_rows(face_edge_indices, nf, n_edges) if edge_rows_map is None else edge_rows_map
                 order = "edges"
             except ValueError:
                 pass
+    if order == "tiers":
+        if dt != torch.float32 or rows is not None:
+            raise ValueError("order='tiers' needs a float32 mesh and no rows")
+        ws = torch.empty(max(1, int(_lib.load().mb_mom_tiers_workspace_bytes(nf))), dtype=torch.uint8, device=dev)
+        _lib.call("mb_mom_zmat_rwg_tiers_c64", _lib.ptr(verts), nv, _lib.ptr(faces), nf, _lib.ptr(face_areas),
+                  _lib.ptr(face_normals), _lib.ptr(face_edge_indices), n_edges, *rules, _lib.ptr(ws), ws.numel(),
+                  _lib.ptr(out), _lib.stream_of(verts))
+        return out
     if order == "gather":
         if dt != torch.float32:
             raise ValueError("order='gather' needs a float32 mesh")
@@ -231,7 +244,7 @@ def assemble_Z_rwg(verts, faces, face_areas, face_normals, face_edge_indices, n_
                   int(m1), _lib.ptr(out), _lib.stream_of(verts))
         return out
     if order != "faces":
-        raise ValueError("order must be 'auto', 'faces', 'edges' or 'gather'")
+        raise ValueError("order must be 'auto', 'tiers', 'faces', 'edges' or 'gather'")
     r0, r1 = (0, 3 * nf) if rows is None else rows
     _lib.call(f"mb_mom_zmat_rwg_{_lib.csfx(dt)}", _lib.ptr(verts), nv, _lib.ptr(faces), nf,
               _lib.ptr(face_areas), _lib.ptr(face_normals), _lib.ptr(face_edge_indices), n_edges, *rules,
@@ -239,6 +252,7 @@ def assemble_Z_rwg(verts, faces, face_areas, face_normals, face_edge_indices, n_
     return out
 
 
+_TIER_RULES = {(3, 2), (4, 3), (5, 4)}  # (n_x, n_y) with tiered kernels
 _EDGE_RULES = {(4, 3), (3, 2), (2, 1), (5, 4)}  # (n_x, n_y) with an edge-row kernel
 
 

@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "gmres_cycle.cuh"
 #include "packed.cuh"
 #include "spai_apply.cuh"
 
@@ -354,13 +355,15 @@ struct GmresWork {
     float* v32;     // [n] complex64
     double* h;      // [2 (m+1)] complex128 (dots), then [1] for norms
     double* nrm;    // [2]
+    void* cycle;    // the resident cycle's counters, sums and Hessenberg matrix
 };
 
 constexpr size_t al256(size_t b) { return (b + 255) & ~size_t(255); }
 
 constexpr size_t gmres_ws_bytes(int64_t n, int m) {
     return al256(sizeof(double) * 2 * (size_t)(m + 1) * n) + 2 * al256(sizeof(double) * 2 * n) +
-           al256(sizeof(float) * 2 * n) + al256(sizeof(double) * 2 * (m + 2)) + al256(sizeof(double) * 4);
+           al256(sizeof(float) * 2 * (n + 1)) + al256(sizeof(double) * 2 * (m + 2)) + al256(sizeof(double) * 4) +
+           GmresCycleRegion::bytes(m);
 }
 
 size_t gmres_workspace_bytes(int64_t n, int m) { return gmres_ws_bytes(n, m); }
@@ -376,10 +379,12 @@ static GmresWork carve(void* ws, int64_t n, int m) {
     g.r = reinterpret_cast<double*>(p);
     p += al(sizeof(double) * 2 * n);
     g.v32 = reinterpret_cast<float*>(p);
-    p += al(sizeof(float) * 2 * n);
+    p += al(sizeof(float) * 2 * (n + 1));
     g.h = reinterpret_cast<double*>(p);
     p += al(sizeof(double) * 2 * (m + 2));
     g.nrm = reinterpret_cast<double*>(p);
+    p += al(sizeof(double) * 4);
+    g.cycle = p;
     return g;
 }
 
@@ -464,10 +469,48 @@ int gmres_real(int kind, const void* a, int64_t n, const double* b, double* x, i
     return sync_check(s, "gmres real result");
 }
 
+// r = b - A x in FP64
+static void residual_of(const GmresMatrix& A, int64_t n, const double* x, const double* b, double* r, cudaStream_t s) {
+    const unsigned rblocks = (unsigned)((n + 7) / 8);
+    if (A.kind == 0)
+        residual_c128_kernel<<<rblocks, 256, 0, s>>>(static_cast<const float*>(A.a), x, b, n, r);
+    else if (A.kind == 1)
+        residual_real_kernel<float><<<rblocks, 256, 0, s>>>(static_cast<const float*>(A.a), x, b, n, r);
+    else
+        residual_real_kernel<double><<<rblocks, 256, 0, s>>>(static_cast<const double*>(A.a), x, b, n, r);
+}
+
+// Restart cycles as one resident kernel each (gmres_cycle.cu): two launches and one host
+// synchronisation per cycle.
+static int gmres_resident(const GmresMatrix& A, int64_t n, const double* b, double* x, int m, int max_iters, double tol,
+                          const GmresWork& g, const GmresCyclePlan& plan, int64_t* iters_out, int64_t* cycles_out,
+                          double* relres_out, int* status_out, cudaStream_t s) {
+    const GmresCycleRegion q(g.cycle, m);
+    cudaMemsetAsync(&q.head->st, 0, sizeof(GmresState), s);
+    GmresHead head{};
+    const GmresState& st = head.st;
+    for (long long c = 0; c < (long long)max_iters + 2 && !st.finished; ++c) {
+        residual_of(A, n, x, b, g.r, s);
+        int rc = gmres_cycle_launch(plan, A.a, n, b, x, g.r, m, tol, max_iters, g.v32, g.w, g.cycle, s);
+        if (rc) return rc;
+        cudaMemcpyAsync(&head, q.head, sizeof(head), cudaMemcpyDeviceToHost, s);
+        if ((rc = sync_check(s, "gmres cycle"))) return rc;
+        if (head.sync.error) return set_error(MB_ERR_CUDA, "gmres cycle: a wait between the grid's blocks ran out");
+    }
+    if (iters_out) *iters_out = st.iters;
+    if (cycles_out) *cycles_out = st.cycles;
+    if (relres_out) *relres_out = st.relres;
+    if (status_out) *status_out = st.converged ? 0 : 1;
+    return MB_OK;
+}
+
 static int gmres_core(const GmresMatrix& A, int64_t n, const double* b, double* x, int m, int max_iters,
                       double tol, void* workspace, const GmresHost& hs, int64_t* iters_out,
                       int64_t* cycles_out, double* relres_out, int* status_out, cudaStream_t s) {
     GmresWork g = carve(workspace, n, m);
+    GmresCyclePlan plan;
+    gmres_cycle_begin(&plan, A.kind, n, m);
+    if (plan.ok) return gmres_resident(A, n, b, x, m, max_iters, tol, g, plan, iters_out, cycles_out, relres_out, status_out, s);
     std::complex<double>* H = hs.H;
     std::complex<double>* cs = hs.cs;
     std::complex<double>* sn = hs.sn;
@@ -486,12 +529,7 @@ static int gmres_core(const GmresMatrix& A, int64_t n, const double* b, double* 
     int status = 1;
     while (true) {
         // FP64 residual of the current iterate
-        if (A.kind == 0)
-            residual_c128_kernel<<<rblocks, 256, 0, s>>>(static_cast<const float*>(A.a), x, b, n, g.r);
-        else if (A.kind == 1)
-            residual_real_kernel<float><<<rblocks, 256, 0, s>>>(static_cast<const float*>(A.a), x, b, n, g.r);
-        else
-            residual_real_kernel<double><<<rblocks, 256, 0, s>>>(static_cast<const double*>(A.a), x, b, n, g.r);
+        residual_of(A, n, x, b, g.r, s);
         double beta;
         if ((rc = norm_of(g.r, n, g.nrm, &beta, s))) return rc;
         relres = beta / bnorm;

@@ -19,6 +19,7 @@
 
 #include "common.cuh"
 #include "packed.cuh"
+#include "vertex_slots.cuh"
 
 namespace mb {
 
@@ -920,10 +921,87 @@ int launch_pack_rows(const T* m, const T* verts, const int32_t* faces, int64_t n
     return check_launch("pack_rows");
 }
 
+// FP32, P1 real: block rows of kPairRows test faces, a source face per thread, terms summed by
+// vertex_slots.cuh.  A warp's 32 panels of a row (1152 consecutive bytes) come by 4-byte asynchronous
+// copies (any alignment: a row starts at 36 F fy bytes), kPackStages - 1 rows ahead, into the
+// warp's own buffer, whose 9-float stride meets no bank twice.
+// Bound: HBM, each panel read once.  Measured (GB300, 5120 faces, 944 MB of panels): 680 us with the rows in
+// shared memory (the compare-and-swap loop of shared additions).
+constexpr int kPackStages = 3;
+constexpr int kPackSmem = kPairSumBytes + kPackStages * kPairThreads * 9 * (int)sizeof(float);
+
+__global__ void __launch_bounds__(kPairThreads)
+    pack_pairs_kernel(const float* __restrict__ m, const int32_t* __restrict__ faces, int64_t nf, int64_t nv,
+                      int rows_per_block, float* __restrict__ packed) {
+    __shared__ VertexSlots s_slots;
+    extern __shared__ float s_sum[];
+    const int64_t p0 = (int64_t)blockIdx.y * rows_per_block, col0 = (int64_t)blockIdx.x * kPairThreads;
+    const int64_t q = col0 + threadIdx.x;
+    const int np = (int)min((int64_t)rows_per_block, nf - p0);
+    if (threadIdx.x < 3 * np) s_slots.id[threadIdx.x] = __ldg(faces + 3 * p0 + threadIdx.x);
+    find_slots(s_slots, np);
+    clear_sums(s_sum, s_slots.n);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float* buf = s_sum + 3 * kPairVerts * kPairThreads + warp * kPackStages * 288;
+    const int64_t c0 = col0 + 32 * warp;
+    const int words = c0 < nf ? (int)min((int64_t)288, 9 * (nf - c0)) : 0;
+    auto fetch = [&](int i) {
+        if (i < np) {
+            const float* src = m + ((p0 + i) * nf + c0) * 9;
+            float* dst = buf + (i % kPackStages) * 288;
+#pragma unroll
+            for (int k = 0; k < 9; ++k) {
+                const int w = lane + 32 * k;
+                if (w < words) {
+                    const unsigned d = (unsigned)__cvta_generic_to_shared(dst + w);
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src + w) : "memory");
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int i = 0; i < kPackStages - 1; ++i) fetch(i);
+    int32_t col[3] = {0, 0, 0};
+    if (q < nf)
+        for (int b = 0; b < 3; ++b) col[b] = __ldg(faces + 3 * q + b);
+    for (int i = 0; i < np; ++i) {
+        fetch(i + kPackStages - 1);
+        asm volatile("cp.async.wait_group %0;" ::"n"(kPackStages - 1) : "memory");
+        __syncwarp();
+        if (q < nf) {
+            float acc[9];
+            const float* src = buf + (i % kPackStages) * 288 + 9 * lane;
+#pragma unroll
+            for (int c = 0; c < 9; ++c) acc[c] = src[c];
+            add_entries(s_slots, i, acc, col, nv, s_sum, packed);
+        }
+        __syncwarp();  // the next fetch overwrites the oldest buffer
+    }
+    if (q < nf) flush_sums(s_slots, col, nv, s_sum, packed);
+}
+
+// a float P1 packing; 0: not one
+static int pack_pairs(const double*, const double*, const int32_t*, int64_t, int64_t, int, double*, cudaStream_t) {
+    return 0;
+}
+static int pack_pairs(const float* m_r, const float* m_i, const int32_t* faces, int64_t nf, int64_t nv, int order,
+                      float* packed, cudaStream_t stream) {
+    const int64_t gx = (nf + kPairThreads - 1) / kPairThreads;
+    // fewer test faces per block where all of them would leave under two waves of 760 blocks
+    const int per = (int)(nf * gx / 1520 >= kPairRows ? kPairRows : nf * gx / 1520 >= 1 ? nf * gx / 1520 : 1);
+    const int64_t gy = (nf + per - 1) / per;
+    if (m_i != nullptr || order != 1 || gy > 65535) return 0;
+    pack_pairs_kernel<<<dim3((unsigned)gx, (unsigned)gy), kPairThreads, kPackSmem, stream>>>(m_r, faces, nf, nv, per,
+                                                                                             packed);
+    return 1;
+}
+
 template <typename T>
 int launch_pack_tight(const T* m_r, const T* m_i, const int32_t* faces, int64_t nf, int64_t nv,
                       int order, T* packed, cudaStream_t stream) {
     if (nf <= 0) return MB_OK;
+    if (pack_pairs(m_r, m_i, faces, nf, nv, order, packed, stream)) return check_launch("pack_pairs");
     if (m_i == nullptr && order == 1 && 3 * nv * (int64_t)sizeof(T) <= kPackRowSmemMax)
         return launch_pack_rows<T, false>(m_r, nullptr, faces, nf, nv, packed, stream);
     const int threads = 256;

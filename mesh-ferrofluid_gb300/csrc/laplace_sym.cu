@@ -21,9 +21,12 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "closed_form.cuh"
 #include "common.cuh"
 #include "packed.cuh"
+#include "vertex_slots.cuh"
 
 namespace mb {
 
@@ -88,79 +91,6 @@ __device__ __forceinline__ void sym_far_pair(const T (*s_rule)[4], const T (*s_y
                 for (int b = 0; b < 3; ++b) acc[3 * a + b] += sa[a] * (wx * s_rule[i][b]);
         } else {
             acc[0] += s0 * wx;
-        }
-    }
-}
-
-// Two separated pairs (fy, fxa) and (fy, fxb) at once in packed f32x2 arithmetic (lane .x
-// the first source face, .y the second): the same sums as sym_far_pair with half the FP32
-// instructions.  X0..X2 hold both faces' shifted corners per coordinate; acc as in
-// sym_far_pair, packed.
-template <int LAYER, int NPHI>
-__device__ __forceinline__ void sym_far_pair2(const float4 (*s_r4)[2], const float4 (*s_y4)[2], const float3& ny,
-                                              const float2 X0[3], const float2 X1[3], const float2 X2[3],
-                                              float2 acc[9]) {
-    // s_r4[j] = {(r0, r0, r1, r1), (r2, r2, w, w)}, s_y4[j] = {(y.x, y.x, y.y, y.y),
-    // (y.z, y.z, wA, wA)}: every value already duplicated, so one 16-byte shared load yields two
-    // packed operands and no register moves are needed to broadcast them
-    float2 e1[3], e2[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        e1[c] = sub2(X1[c], X0[c]);
-        e2[c] = sub2(X2[c], X1[c]);
-    }
-    const float2 nx0 = fma2(e1[1], e2[2], mul2(bc(-1.f), mul2(e1[2], e2[1])));
-    const float2 nx1 = fma2(e1[2], e2[0], mul2(bc(-1.f), mul2(e1[0], e2[2])));
-    const float2 nx2 = fma2(e1[0], e2[1], mul2(bc(-1.f), mul2(e1[1], e2[0])));
-    const float2 n2 = fma2(nx0, nx0, fma2(nx1, nx1, mul2(nx2, nx2)));
-    const float2 ax = make_float2(0.5f * sqrtf(n2.x), 0.5f * sqrtf(n2.y));
-#pragma unroll 1
-    for (int i = 0; i < 7; ++i) {
-        // re-read the tables every outer point instead of holding all 28 of them in registers
-        asm volatile("" ::: "memory");
-        const float4 ra = s_r4[i][0], rb = s_r4[i][1];
-        const float2 r0 = make_float2(ra.x, ra.y), r1 = make_float2(ra.z, ra.w), r2 = make_float2(rb.x, rb.y);
-        float2 x[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) x[c] = fma2(r0, X0[c], fma2(r1, X1[c], mul2(r2, X2[c])));
-        float2 s0 = bc(0.f), s1 = bc(0.f), s2 = bc(0.f);
-#pragma unroll
-        for (int j = 0; j < 7; ++j) {
-            const float4 ya = s_y4[j][0], yb = s_y4[j][1];
-            const float2 dx = sub2(x[0], make_float2(ya.x, ya.y));
-            const float2 dy = sub2(x[1], make_float2(ya.z, ya.w));
-            const float2 dz = sub2(x[2], make_float2(yb.x, yb.y));
-            const float2 d2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
-            const float2 ri = make_float2(rsqrtf(d2.x), rsqrtf(d2.y));
-            float2 g = mul2(ri, make_float2(yb.z, yb.w));
-            if constexpr (LAYER == 2) g = mul2(g, mul2(ri, ri));
-            if constexpr (NPHI == 3) {
-                const float4 qa = s_r4[j][0], qb = s_r4[j][1];
-                s0 = fma2(g, make_float2(qa.x, qa.y), s0);
-                s1 = fma2(g, make_float2(qa.z, qa.w), s1);
-                s2 = fma2(g, make_float2(qb.x, qb.y), s2);
-            } else {
-                s0 = add2(s0, g);
-            }
-        }
-        if constexpr (LAYER == 2) {
-            const float2 dn = fma2(x[0], bc(ny.x), fma2(x[1], bc(ny.y), mul2(x[2], bc(ny.z))));
-            s0 = mul2(s0, dn);
-            s1 = mul2(s1, dn);
-            s2 = mul2(s2, dn);
-        }
-        const float2 wx = mul2(make_float2(rb.z, rb.w), ax);
-        if constexpr (NPHI == 3) {
-            const float2 sa[3] = {s0, s1, s2};
-            const float2 rr[3] = {r0, r1, r2};
-#pragma unroll
-            for (int b = 0; b < 3; ++b) {
-                const float2 wb = mul2(wx, rr[b]);
-#pragma unroll
-                for (int a = 0; a < 3; ++a) acc[3 * a + b] = fma2(sa[a], wb, acc[3 * a + b]);
-            }
-        } else {
-            acc[0] = fma2(s0, wx, acc[0]);
         }
     }
 }
@@ -243,20 +173,19 @@ __device__ __forceinline__ void tri_curls(const V3<T>& p0, const V3<T>& p1, cons
 
 // Packed operators [V, V] without the [F, F, 3, 3] panels: OP 1 single layer, 2 double layer
 // (P1 x P1), 3 hypersingular (Maue: curl phi_a(fy) . curl phi_b(fx) times the P0 single
-// layer).  One block per test face fy sweeps every source face fx, accumulates the three
+// layer).  FP64: one block per test face fy sweeps every source face fx, accumulates the three
 // packed rows faces[fy, a] in shared memory (3 V values) and adds them to `packed` at the
 // end.  Pairs sharing a vertex are skipped here and added by lap_sym_near_kernel.
-template <typename T, int OP>
-__global__ void __launch_bounds__(kSymThreads, sizeof(T) == 4 ? (OP == 3 ? 6 : 4) : 1)
-    lap_sym_tight_kernel(const T* __restrict__ verts, const int32_t* __restrict__ faces, int64_t nf, int64_t nv,
-                         int64_t row_begin, T* __restrict__ packed) {
+template <int OP>
+__global__ void __launch_bounds__(kSymThreads, 1)
+    lap_sym_tight_kernel(const double* __restrict__ verts, const int32_t* __restrict__ faces, int64_t nf, int64_t nv,
+                         int64_t row_begin, double* __restrict__ packed) {
+    using T = double;
     constexpr int LAYER = OP == 2 ? 2 : 1;
     constexpr int NPHI = OP == 3 ? 1 : 3;
     __shared__ T s_rule[7][4];
     __shared__ T s_y[7][4];
     __shared__ T s_n[3];
-    __shared__ float4 s_r4[7][2];  // the same tables with every value duplicated (float path)
-    __shared__ float4 s_y4[7][2];
     extern __shared__ __align__(16) unsigned char tight_smem[];
     T* rows = reinterpret_cast<T*>(tight_smem);
     const int64_t fy = row_begin + blockIdx.x;
@@ -268,17 +197,6 @@ __global__ void __launch_bounds__(kSymThreads, sizeof(T) == 4 ? (OP == 3 ? 6 : 4
     V3<T> cy[3];
     if constexpr (OP == 3) tri_curls(v3<T>(0, 0, 0), Y1, Y2, cy);
     __syncthreads();
-    if (threadIdx.x < 7) {
-        const int j = threadIdx.x;
-        const float r0 = (float)s_rule[j][0], r1 = (float)s_rule[j][1], r2 = (float)s_rule[j][2];
-        const float rw = (float)s_rule[j][3];
-        s_r4[j][0] = make_float4(r0, r0, r1, r1);
-        s_r4[j][1] = make_float4(r2, r2, rw, rw);
-        const float y0 = (float)s_y[j][0], y1 = (float)s_y[j][1], y2 = (float)s_y[j][2], yw = (float)s_y[j][3];
-        s_y4[j][0] = make_float4(y0, y0, y1, y1);
-        s_y4[j][1] = make_float4(y2, y2, yw, yw);
-    }
-    __syncthreads();
     const V3<T> ny = v3<T>(s_n[0], s_n[1], s_n[2]);
     // each thread sweeps its own strip of consecutive source faces: neighbouring faces share
     // vertices, and lanes of a warp working on neighbours would collide in the shared-memory
@@ -286,46 +204,6 @@ __global__ void __launch_bounds__(kSymThreads, sizeof(T) == 4 ? (OP == 3 ? 6 : 4
     const int64_t strip = (nf + blockDim.x - 1) / blockDim.x;
     const int64_t strip0 = (int64_t)threadIdx.x * strip;
     const int64_t strip1 = strip0 + strip < nf ? strip0 + strip : nf;
-    if constexpr (sizeof(T) == 4 && OP != 3) {
-        // two source faces per thread and iteration (fxa, fxa + 1), packed arithmetic
-        // (the P0 sums of OP 3 are light enough that occupancy matters more)
-        const float3 nyf = make_float3(ny.x, ny.y, ny.z);
-#pragma unroll 1
-        for (int64_t k = 0; k < strip; k += 2) {
-            const int64_t fxa = strip0 + k;
-            if (fxa >= strip1) break;
-            const int64_t fxb_raw = fxa + 1;
-            const bool has_b = fxb_raw < strip1;
-            const int64_t fxb = has_b ? fxb_raw : fxa;
-            const bool use_a = !share_vertex(faces, fy, fxa);
-            const bool use_b = has_b && !share_vertex(faces, fy, fxb);
-            if (!use_a && !use_b) continue;
-            const int32_t va[3] = {__ldg(faces + 3 * fxa), __ldg(faces + 3 * fxa + 1), __ldg(faces + 3 * fxa + 2)};
-            const int32_t vb[3] = {__ldg(faces + 3 * fxb), __ldg(faces + 3 * fxb + 1), __ldg(faces + 3 * fxb + 2)};
-            float2 X[3][3];  // corner, coordinate
-#pragma unroll
-            for (int v = 0; v < 3; ++v) {
-                const V3<T> pa = load3(verts, va[v]) - o;
-                const V3<T> pb = load3(verts, vb[v]) - o;
-                X[v][0] = make_float2(pa.x, pb.x);
-                X[v][1] = make_float2(pa.y, pb.y);
-                X[v][2] = make_float2(pa.z, pb.z);
-            }
-            float2 acc[9];
-#pragma unroll
-            for (int c = 0; c < 9; ++c) acc[c] = bc(0.f);
-            sym_far_pair2<LAYER, NPHI>(s_r4, s_y4, nyf, X[0], X[1], X[2], acc);
-            {
-#pragma unroll
-                for (int a = 0; a < 3; ++a)
-#pragma unroll
-                    for (int b = 0; b < 3; ++b) {
-                        if (use_a) atomicAdd(rows + a * nv + va[b], acc[3 * a + b].x * T(kInv4Pi));
-                        if (use_b) atomicAdd(rows + a * nv + vb[b], acc[3 * a + b].y * T(kInv4Pi));
-                    }
-            }
-        }
-    } else {
 #pragma unroll 1
     for (int64_t fx = strip0; fx < strip1; ++fx) {
         if (share_vertex(faces, fy, fx)) continue;
@@ -352,12 +230,254 @@ __global__ void __launch_bounds__(kSymThreads, sizeof(T) == 4 ? (OP == 3 ? 6 : 4
                 for (int b = 0; b < 3; ++b) atomicAdd(rows + a * nv + vx[b], acc[3 * a + b] * T(kInv4Pi));
         }
     }
-    }
     __syncthreads();
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         T* dst = packed + (int64_t)__ldg(faces + 3 * fy + a) * nv;
         for (int64_t j = threadIdx.x; j < nv; j += blockDim.x) atomicAdd(dst + j, rows[a * nv + j]);
+    }
+}
+
+// FP32: a thread keeps one source face fx and meets the block's test faces.  The 7-point rule is its
+// centroid and two orbits s A_a of the corners A_a relative to the centroid (s = 1 - 3 q), so with
+// D the difference of the centroids
+//     R^2 = |D|^2 + 2 s D.A_a - 2 s' D.B_b + s^2 |A_a|^2 + s'^2 |B_b|^2 - 2 s s' A_a.B_b
+// comes from 15 dot products of the pair at three operations per evaluation instead of six, and the
+// hat functions at the points are (1 - s)/3 + s [corner], so two sums per evaluation (over all
+// corners of fy, and corner by corner) hold all nine entries.  n_y.(x - y) depends on x alone.
+// Lanes of a packed register are the two orbits of fx.  The sums are over k(R) - k(R_c): the
+// constant's integrals are known, and the rounding is that of the differences.  Entries are added by
+// vertex_slots.cuh.  Bound: SFU (49 reciprocal roots per pair, 0.28 ms at 5120 faces) and issue
+// slots.  Measured (GB300, 5120 faces): single / double / hypersingular 982 / 1020 / 757 ->
+// 485 / 541 / 421 us.
+// Pairs whose centroids are closer than twice the sum of the corner distances, where the
+// expansion of R^2 would cancel, are listed and evaluated from coordinate differences.
+constexpr int kRowRec = 28;  // floats per staged test face
+
+struct FaceLocal {
+    V3<float> v0, off, A[3];  // first corner; centroid - v0; corners - centroid
+    float area, rho;
+    int32_t id[3];
+};
+
+__device__ __forceinline__ FaceLocal face_local(const float* __restrict__ verts, const int32_t* __restrict__ faces,
+                                                int64_t f) {
+    FaceLocal o;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) o.id[a] = __ldg(faces + 3 * f + a);
+    o.v0 = load3(verts, o.id[0]);
+    const V3<float> e1 = load3(verts, o.id[1]) - o.v0, e2 = load3(verts, o.id[2]) - o.v0;
+    o.off = (1.f / 3.f) * (e1 + e2);
+    o.A[0] = -1.f * o.off;
+    o.A[1] = e1 - o.off;
+    o.A[2] = e2 - o.off;
+    const V3<float> n = cross(e1, e2);
+    o.area = 0.5f * sqrtf(dot(n, n));
+    o.rho = sqrtf(fmaxf(dot(o.A[0], o.A[0]), fmaxf(dot(o.A[1], o.A[1]), dot(o.A[2], o.A[2]))));
+    return o;
+}
+
+// a close separated pair: coordinate differences, as lap_sym_far_kernel
+template <int OP>
+__device__ void close_pair_entries(const float* __restrict__ verts, const int32_t* __restrict__ faces, int64_t fy,
+                                   int64_t fx, int64_t nv, float* __restrict__ packed) {
+    constexpr int LAYER = OP == 2 ? 2 : 1, NPHI = OP == 3 ? 1 : 3;
+    const int32_t row[3] = {faces[3 * fy], faces[3 * fy + 1], faces[3 * fy + 2]};
+    const int32_t col[3] = {faces[3 * fx], faces[3 * fx + 1], faces[3 * fx + 2]};
+    const V3<float> o = load3(verts, row[0]);
+    const V3<float> Y1 = load3(verts, row[1]) - o, Y2 = load3(verts, row[2]) - o;
+    const V3<float> X0 = load3(verts, col[0]) - o, X1 = load3(verts, col[1]) - o, X2 = load3(verts, col[2]) - o;
+    float rule[7][4], y[7][4];
+    const V3<float> n = cross(Y1, Y2 - Y1);
+    const float l = sqrtf(dot(n, n));
+#pragma unroll
+    for (int j = 0; j < 7; ++j) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) rule[j][c] = (float)c_d7[j][c];
+        const V3<float> p = rule[j][1] * Y1 + rule[j][2] * Y2;
+        y[j][0] = p.x;
+        y[j][1] = p.y;
+        y[j][2] = p.z;
+        y[j][3] = rule[j][3] * 0.5f * l;
+    }
+    float acc[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    sym_far_pair<float, LAYER, NPHI>(rule, y, (1.f / l) * n, X0, X1, X2, acc);
+    if constexpr (OP == 3) {
+        V3<float> cy[3], cx[3];
+        tri_curls(v3<float>(0.f, 0.f, 0.f), Y1, Y2, cy);
+        tri_curls(X0, X1, X2, cx);
+        const float w = acc[0];
+#pragma unroll
+        for (int c = 0; c < 9; ++c) acc[c] = dot(cy[c / 3], cx[c % 3]) * w;
+    }
+#pragma unroll
+    for (int c = 0; c < 9; ++c) atomicAdd(packed + (int64_t)row[c / 3] * nv + col[c % 3], acc[c] * float(kInv4Pi));
+}
+
+template <int OP>
+__global__ void __launch_bounds__(kPairThreads, 5)
+    lap_sym_pairs_kernel(const float* __restrict__ verts, const int32_t* __restrict__ faces, int64_t nf, int64_t nv,
+                         int64_t row_begin, int64_t row_end, int rows_per_block, float* __restrict__ packed) {
+    constexpr float s1 = (float)(1.0 - 3.0 * 0.10128650732345634), s2 = (float)(1.0 - 3.0 * 0.47014206410511509);
+    constexpr float w0 = 0.225f, w1 = 0.12593918054482715f, w2 = 0.13239415278850619f;
+    constexpr float a1 = (1.f - s1) / 3.f, a2 = (1.f - s2) / 3.f;
+    __shared__ __align__(16) float s_rec[kPairRows][kRowRec];
+    __shared__ VertexSlots s_slots;
+    __shared__ uint16_t s_close[kPairRows * kPairThreads];
+    __shared__ int s_n;
+    extern __shared__ float s_sum[];
+    const int64_t p0 = row_begin + (int64_t)blockIdx.y * rows_per_block;
+    const int64_t q = (int64_t)blockIdx.x * kPairThreads + threadIdx.x;
+    const int np = (int)min((int64_t)rows_per_block, row_end - p0);
+    if (threadIdx.x == 0) s_n = 0;
+    if (threadIdx.x < np) {
+        const FaceLocal f = face_local(verts, faces, p0 + threadIdx.x);
+        float* r = s_rec[threadIdx.x];
+        const V3<float> n = cross(f.A[1] - f.A[0], f.A[2] - f.A[1]);
+        const float inv = 1.f / sqrtf(dot(n, n));
+        const float v[kRowRec] = {f.v0.x, f.v0.y, f.v0.z, f.rho, f.off.x, f.off.y, f.off.z, f.area,
+                                  f.A[0].x, f.A[0].y, f.A[0].z, 0.f, f.A[1].x, f.A[1].y, f.A[1].z, 0.f,
+                                  f.A[2].x, f.A[2].y, f.A[2].z, 0.f, n.x * inv, n.y * inv, n.z * inv, 0.f,
+                                  dot(f.A[0], f.A[0]), dot(f.A[1], f.A[1]), dot(f.A[2], f.A[2]), 0.f};
+#pragma unroll
+        for (int c = 0; c < kRowRec; ++c) r[c] = v[c];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) s_slots.id[3 * threadIdx.x + a] = f.id[a];
+    }
+    find_slots(s_slots, np);
+    clear_sums(s_sum, s_slots.n);
+    if (q < nf) {
+        const FaceLocal x = face_local(verts, faces, q);
+        float BB[3];
+#pragma unroll
+        for (int b = 0; b < 3; ++b) BB[b] = dot(x.A[b], x.A[b]);
+#pragma unroll 1
+        for (int i = 0; i < np; ++i) {
+            const float4* r = reinterpret_cast<const float4*>(s_rec[i]);
+            const float4 c0 = r[0], c1 = r[1], r2v = r[2], r3v = r[3], r4v = r[4], nv4 = r[5], aav = r[6];
+            const float dx = (c0.x - x.v0.x) + (c1.x - x.off.x), dy = (c0.y - x.v0.y) + (c1.y - x.off.y),
+                        dz = (c0.z - x.v0.z) + (c1.z - x.off.z);
+            const float Rc2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx)), lim = 2.f * (c0.w + x.rho);
+            if (!(Rc2 >= lim * lim)) {  // faces sharing a vertex are here, too: closed forms
+                int shared = 0;
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    const int id = s_slots.id[3 * i + a];
+                    shared |= (id == x.id[0]) | (id == x.id[1]) | (id == x.id[2]);
+                }
+                if (!shared) s_close[atomicAdd(&s_n, 1)] = (uint16_t)(i * kPairThreads + threadIdx.x);
+                continue;
+            }
+            const float A[3][3] = {{r2v.x, r2v.y, r2v.z}, {r3v.x, r3v.y, r3v.z}, {r4v.x, r4v.y, r4v.z}};
+            const float AA[3] = {aav.x, aav.y, aav.z};
+            float m[3][3], DA[3];
+            float2 V[3];
+#pragma unroll
+            for (int b = 0; b < 3; ++b) {
+                const float DB = fmaf(dz, x.A[b].z, fmaf(dy, x.A[b].y, dx * x.A[b].x));
+                V[b] = make_float2(s1 * (2.f * DB - s1 * BB[b]), s2 * (2.f * DB - s2 * BB[b]));
+            }
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                DA[a] = fmaf(dz, A[a][2], fmaf(dy, A[a][1], dx * A[a][0]));
+#pragma unroll
+                for (int b = 0; b < 3; ++b)
+                    m[a][b] = fmaf(A[a][2], x.A[b].z, fmaf(A[a][1], x.A[b].y, A[a][0] * x.A[b].x));
+            }
+            // sums over fy's points, lanes fx's orbits: S[a][b] with w s (corner a), S0[b] with
+            // w (1 - s)/3 (OP 3: w); c[a], cc the same at fx's centroid; fy's centroid first
+            float2 S[3][3], S0[3];
+            float c[3] = {0.f, 0.f, 0.f}, cc = 0.f;
+            const float ri = rsqrtf(Rc2), kc = OP == 2 ? ri * ri * ri : ri;
+#pragma unroll
+            for (int b = 0; b < 3; ++b) {
+                const float2 d2 = sub2(bc(Rc2), V[b]);
+                float2 h = make_float2(rsqrtf(d2.x), rsqrtf(d2.y));
+                if constexpr (OP == 2) h = mul2(h, mul2(h, h));
+                S0[b] = mul2(bc(OP == 3 ? w0 : w0 / 3.f), sub2(h, bc(kc)));
+#pragma unroll
+                for (int a = 0; a < 3; ++a) S[a][b] = bc(0.f);
+            }
+#pragma unroll
+            for (int o = 0; o < 2; ++o) {
+                const float s = o ? s2 : s1, w = o ? w2 : w1, al = o ? a2 : a1;
+                const float2 K = make_float2(2.f * s * s1, 2.f * s * s2);
+                const float2 W0 = bc(OP == 3 ? w : w * al), WS = bc(w * s);
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    const float u = fmaf(s * s, AA[a], 2.f * s * DA[a]);
+                    {
+                        float g = rsqrtf(Rc2 + u);
+                        if constexpr (OP == 2) g = g * g * g;
+                        g -= kc;
+                        cc = fmaf(OP == 3 ? w : w * al, g, cc);
+                        c[a] = fmaf(w * s, g, c[a]);
+                    }
+#pragma unroll
+                    for (int b = 0; b < 3; ++b) {
+                        const float2 d2 = sub2(bc(Rc2 + u), fma2(bc(m[a][b]), K, V[b]));
+                        float2 h = make_float2(rsqrtf(d2.x), rsqrtf(d2.y));
+                        if constexpr (OP == 2) h = mul2(h, mul2(h, h));
+                        h = sub2(h, bc(kc));
+                        S0[b] = fma2(W0, h, S0[b]);
+                        if constexpr (OP != 3) S[a][b] = fma2(WS, h, S[a][b]);
+                    }
+                }
+            }
+            float acc[9];
+            if constexpr (OP == 3) {
+                const float2 t = add2(add2(S0[0], S0[1]), S0[2]);
+                // curl_a . curl_b = (A_{a+1} - A_{a+2}).(B_{b+1} - B_{b+2}) / (4 area area)
+                const float v0 = (kc + fmaf(w1, t.x, fmaf(w2, t.y, w0 * cc))) * (0.25f * float(kInv4Pi));
+#pragma unroll
+                for (int a = 0; a < 3; ++a)
+#pragma unroll
+                    for (int b = 0; b < 3; ++b) {
+                        const int p = (a + 1) % 3, e = (a + 2) % 3, u = (b + 1) % 3, v = (b + 2) % 3;
+                        acc[3 * a + b] = ((m[p][u] - m[p][v]) - (m[e][u] - m[e][v])) * v0;
+                    }
+            } else {
+                const float sc = c1.w * x.area * float(kInv4Pi);
+                float k0[3] = {kc / 9.f, kc / 9.f, kc / 9.f};  // the constant's share of column b
+                if constexpr (OP == 2) {                       // n_y.(x - y) at fx's points
+                    const float nD = fmaf(nv4.z, dz, fmaf(nv4.y, dy, nv4.x * dx));
+#pragma unroll
+                    for (int b = 0; b < 3; ++b) {
+                        const float nB = fmaf(nv4.z, x.A[b].z, fmaf(nv4.y, x.A[b].y, nv4.x * x.A[b].x));
+                        const float2 dn = make_float2(fmaf(s1, nB, -nD), fmaf(s2, nB, -nD));
+                        S0[b] = mul2(S0[b], dn);
+                        k0[b] = (kc / 3.f) * fmaf(w1 * s1 * s1 + w2 * s2 * s2, nB, -nD / 3.f);
+#pragma unroll
+                        for (int a = 0; a < 3; ++a) S[a][b] = mul2(S[a][b], dn);
+                    }
+                    cc *= -nD;
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) c[a] *= -nD;
+                }
+                // fx's weights: w' s' at corner b, w' (1 - s')/3 over all points
+                const float2 t0 = add2(add2(S0[0], S0[1]), S0[2]);
+                const float C0 = fmaf(w1 * a1, t0.x, fmaf(w2 * a2, t0.y, (w0 / 3.f) * cc));
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    const float2 t = add2(add2(S[a][0], S[a][1]), S[a][2]);
+                    const float Ca = fmaf(w1 * a1, t.x, fmaf(w2 * a2, t.y, fmaf(w0 / 3.f, c[a], C0)));
+#pragma unroll
+                    for (int b = 0; b < 3; ++b) {
+                        const float2 v = add2(S[a][b], S0[b]);
+                        acc[3 * a + b] = sc * (k0[b] + fmaf(w1 * s1, v.x, fmaf(w2 * s2, v.y, Ca)));
+                    }
+                }
+            }
+            add_entries(s_slots, i, acc, x.id, nv, s_sum, packed);
+        }
+        flush_sums(s_slots, x.id, nv, s_sum, packed);
+    }
+    __syncthreads();
+    const int n = s_n;
+    for (int i = threadIdx.x; i < n; i += kPairThreads) {
+        const int e = s_close[i];
+        close_pair_entries<OP>(verts, faces, p0 + e / kPairThreads, (int64_t)blockIdx.x * kPairThreads + e % kPairThreads,
+                               nv, packed);
     }
 }
 
@@ -643,30 +763,45 @@ int launch_laplace_sym(const T* verts, const int32_t* faces, int64_t nf, int lay
 // [row_begin, row_end), added to packed [nv, nv].
 constexpr int64_t kTightSmemMax = 160 * 1024;
 
+static int launch_sym_pairs(const double* verts, const int32_t* faces, int64_t nf, int64_t nv, int op, int64_t row_begin,
+                            int64_t row_end, double* packed, cudaStream_t s) {
+    const int64_t smem = 3 * nv * (int64_t)sizeof(double);
+    if (row_end - row_begin > 0x7fffffffLL) return set_error(MB_ERR_SIZE, "mesh too large for one launch");
+    const unsigned blocks = (unsigned)(row_end - row_begin);
+    auto go = [&](auto kernel) -> int {
+        if (smem > 48 * 1024) {
+            const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (e != cudaSuccess) return set_error(MB_ERR_CUDA, cudaGetErrorString(e));
+        }
+        kernel<<<blocks, kSymThreads, (size_t)smem, s>>>(verts, faces, nf, nv, row_begin, packed);
+        return MB_OK;
+    };
+    return op == 1 ? go(lap_sym_tight_kernel<1>) : op == 2 ? go(lap_sym_tight_kernel<2>) : go(lap_sym_tight_kernel<3>);
+}
+
+static int launch_sym_pairs(const float* verts, const int32_t* faces, int64_t nf, int64_t nv, int op, int64_t row_begin,
+                            int64_t row_end, float* packed, cudaStream_t s) {
+    const int64_t gx = (nf + kPairThreads - 1) / kPairThreads, rows = row_end - row_begin;
+    // fewer test faces per block where all of them would leave under two waves of 760 blocks
+    const int per = (int)std::max<int64_t>(1, std::min<int64_t>(kPairRows, rows * gx / 1520));
+    const int64_t gy = (rows + per - 1) / per;
+    if (gx > 0x7fffffffLL || gy > 65535) return set_error(MB_ERR_SIZE, "mesh too large for one launch");
+    auto go = [&](auto kernel) -> int {
+        kernel<<<dim3((unsigned)gx, (unsigned)gy), kPairThreads, kPairSumBytes, s>>>(verts, faces, nf, nv, row_begin,
+                                                                                     row_end, per, packed);
+        return MB_OK;
+    };
+    return op == 1 ? go(lap_sym_pairs_kernel<1>) : op == 2 ? go(lap_sym_pairs_kernel<2>) : go(lap_sym_pairs_kernel<3>);
+}
+
 template <typename T>
 int launch_laplace_sym_tight(const T* verts, const int32_t* faces, int64_t nf, int64_t nv, int op,
                              const int32_t* pairs, int64_t n_pairs, int64_t row_begin, int64_t row_end, T* packed,
                              cudaStream_t s) {
     if (nf <= 0 || row_end <= row_begin) return MB_OK;
     if (op < 1 || op > 3) return set_error(MB_ERR_ARG, "op must be 1 (single), 2 (double) or 3 (hypersingular)");
-    const int64_t smem = 3 * nv * (int64_t)sizeof(T);
-    if (smem > kTightSmemMax) return set_error(MB_ERR_SIZE, "too many vertices for the packed assembly");
-    if (row_end - row_begin > 0x7fffffffLL) return set_error(MB_ERR_SIZE, "mesh too large for one launch");
-    const unsigned blocks = (unsigned)(row_end - row_begin);
-#define MB_TIGHT(OP)                                                                                          \
-    do {                                                                                                      \
-        if (smem > 48 * 1024) {                                                                               \
-            const cudaError_t e = cudaFuncSetAttribute(lap_sym_tight_kernel<T, OP>,                          \
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-            if (e != cudaSuccess) return set_error(MB_ERR_CUDA, cudaGetErrorString(e));                     \
-        }                                                                                                     \
-        lap_sym_tight_kernel<T, OP><<<blocks, kSymThreads, (size_t)smem, s>>>(verts, faces, nf, nv, row_begin, \
-                                                                              packed);                        \
-    } while (0)
-    if (op == 1) MB_TIGHT(1);
-    else if (op == 2) MB_TIGHT(2);
-    else MB_TIGHT(3);
-#undef MB_TIGHT
+    if (3 * nv * (int64_t)sizeof(T) > kTightSmemMax) return set_error(MB_ERR_SIZE, "too many vertices for the packed assembly");
+    if (int rc = launch_sym_pairs(verts, faces, nf, nv, op, row_begin, row_end, packed, s)) return rc;
     if (n_pairs > 0) {
         const int64_t near_blocks = (n_pairs * kNearLanes + 127) / 128;
         if (near_blocks > 0x7fffffffLL) return set_error(MB_ERR_SIZE, "near-pair list too long for one launch");

@@ -25,6 +25,7 @@
 
 #include "closed_form.cuh"
 #include "common.cuh"
+#include "face_record.cuh"
 #include "packed.cuh"
 
 namespace mb {
@@ -316,13 +317,17 @@ __device__ __forceinline__ void sym_regular_pair<float>(const float* __restrict_
 // Single-mesh float separated pairs: a block owns kSymRows test faces (their vertices, RWG
 // constants and edge ids staged in shared memory) and 128 source faces; each thread sets up
 // its source face once and evaluates it against every test face of the block.
+// REST: only the pairs that sym_pairs_kernel leaves (rec: the face records).
 constexpr int kSymRows = 32;
+template <bool REST>
 __global__ void __launch_bounds__(128) mom_sym_regular_rows_kernel(const float* __restrict__ verts,
                                                                    const int32_t* __restrict__ faces,
                                                                    const int32_t* __restrict__ fei,
                                                                    int64_t n_edges, float k, int64_t nf,
                                                                    int64_t p_begin, int64_t p_end,
-                                                                   float* __restrict__ z) {
+                                                                   float* __restrict__ z,
+                                                                   const float* __restrict__ rec) {
+    __shared__ float4 s_c[REST ? kSymRows : 1];
     __shared__ float s_b[7][4];
     __shared__ float s_A[kSymRows][9], s_cm[kSymRows][3], s_ap[kSymRows];
     __shared__ int32_t s_v[kSymRows][3], s_row[kSymRows][3];
@@ -346,15 +351,29 @@ __global__ void __launch_bounds__(128) mom_sym_regular_rows_kernel(const float* 
         s_cm[threadIdx.x][1] = cm[1];
         s_cm[threadIdx.x][2] = cm[2];
         s_ap[threadIdx.x] = ap;
+        if constexpr (REST) s_c[threadIdx.x] = reinterpret_cast<const float4*>(rec)[(kRec / 4) * p];
     }
     __syncthreads();
     const int64_t q = (int64_t)blockIdx.x * 128 + threadIdx.x;
     if (q >= nf) return;
+    float4 cq = make_float4(0.f, 0.f, 0.f, 0.f);
+    uint32_t mine = 0xffffffffu;  // test faces left to this kernel
+    if constexpr (REST) {
+        const int nr = (int)min((int64_t)kSymRows, p_end - p0);
+        cq = __ldg(reinterpret_cast<const float4*>(rec) + (kRec / 4) * q);
+        mine = 0;
+        for (int r = 0; r < nr; ++r) {
+            const float4 c = s_c[r];
+            if (!sym_pair_far(centre_dist2(c.x - cq.x, c.y - cq.y, c.z - cq.z), c.w, cq.w, k)) mine |= 1u << r;
+        }
+        if (mine == 0) return;
+    }
     SymSource S;
     sym_source(verts, faces, fei, k, q, s_b, S);
     const int nr = (int)min((int64_t)kSymRows, p_end - p0);
 #pragma unroll 1
     for (int r = 0; r < nr; ++r) {
+        if (REST && !(mine >> r & 1)) continue;
         int shared = 0;
 #pragma unroll
         for (int a = 0; a < 3; ++a)
@@ -862,8 +881,8 @@ int launch_mom_sym_regular(const T* verts, const int32_t* faces, const int32_t* 
     if constexpr (sizeof(T) == 4) {
         const int64_t py = (p_end - p_begin + kSymRows - 1) / kSymRows;
         if (q_blocks > 0x7fffffffLL || py > 65535) return set_error(MB_ERR_SIZE, "mesh too large for one launch");
-        mom_sym_regular_rows_kernel<<<dim3((unsigned)q_blocks, (unsigned)py), 128, 0, s>>>(
-            verts, faces, fei, n_edges, (float)k, nf, p_begin, p_end, z);
+        mom_sym_regular_rows_kernel<false><<<dim3((unsigned)q_blocks, (unsigned)py), 128, 0, s>>>(
+            verts, faces, fei, n_edges, (float)k, nf, p_begin, p_end, z, nullptr);
         return check_launch("mom_sym_regular");
     }
     const int64_t blocks = (p_end - p_begin) * q_blocks;
@@ -871,6 +890,16 @@ int launch_mom_sym_regular(const T* verts, const int32_t* faces, const int32_t* 
     mom_sym_regular_kernel<T><<<(unsigned)blocks, 128, 0, s>>>(verts, faces, fei, n_edges, (T)k, nf, p_begin,
                                                                 q_blocks, z);
     return check_launch("mom_sym_regular");
+}
+
+// The separated pairs that sym_pairs_kernel leaves, all test faces.
+int launch_mom_sym_rest(const float* verts, const int32_t* faces, const int32_t* fei, int64_t n_edges, double k, int64_t nf,
+                        const float* rec, float* z, cudaStream_t s) {
+    const int64_t q_blocks = (nf + 127) / 128, py = (nf + kSymRows - 1) / kSymRows;
+    if (q_blocks > 0x7fffffffLL || py > 65535) return set_error(MB_ERR_SIZE, "mesh too large for one launch");
+    mom_sym_regular_rows_kernel<true><<<dim3((unsigned)q_blocks, (unsigned)py), 128, 0, s>>>(verts, faces, fei, n_edges,
+                                                                                             (float)k, nf, 0, nf, z, rec);
+    return check_launch("mom_sym_rest");
 }
 
 template <typename T>

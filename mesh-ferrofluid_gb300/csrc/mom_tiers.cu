@@ -38,6 +38,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "face_record.cuh"
 #include "mom_entry.cuh"
 #include "packed.cuh"
 
@@ -48,19 +49,6 @@ namespace {
 // ---------------------------------------------------------------------------------------
 // face records: 32 floats per face
 // ---------------------------------------------------------------------------------------
-constexpr int kRec = 32;
-enum {
-    kC = 0,      // centroid (hi)
-    kRho2 = 3,   // max |corner - centroid|^2; NaN: the face takes part in tier 4 only
-    kCl = 4,     // centroid (lo): hi + lo carries ~48 bits
-    kEdge = 7,   // RWG edge id of local edge e at 7 + 4 e (int bits)
-    kA = 8,      // corner a - centroid at 8 + 4 a
-    kHalf = 19,  // +-l / 2 of local edge e at 19 + 4 e (RWG sign of the reference)
-    kN = 20,     // normal
-    kAA = 24,    // |A_0|^2, |A_1|^2, |A_2|^2
-    kAB = 28     // A_0.A_1, A_1.A_2, A_2.A_0
-};
-
 // degree-4 rule: corners (1 - 2 q, q, q) of two orbits lie at s A_a from the centroid
 constexpr float kS1 = (float)(1.0 - 3.0 * 0.445948490915965), kW1 = 0.223381589678011f;
 constexpr float kS2 = (float)(1.0 - 3.0 * 0.091576213509771), kW2 = 0.109951743655322f;
@@ -117,7 +105,7 @@ __global__ void face_record_kernel(const float* __restrict__ verts, const int32_
     float n[3];
     for (int a = 0; a < 3; ++a) {
         id[a] = faces[3 * f + a];
-        n[a] = normals[3 * f + a];
+        n[a] = normals ? normals[3 * f + a] : 0.f;
         for (int d = 0; d < 3; ++d) v[a][d] = (double)verts[3 * (int64_t)id[a] + d];
     }
     float r[kRec];
@@ -130,7 +118,7 @@ __global__ void face_record_kernel(const float* __restrict__ verts, const int32_
         r[kN + d] = n[d];
     }
     float rho2 = 0.f;
-    bool ok = is_gauss(gpx, gwx, nx) && is_gauss(gpy, gwy, ny);
+    bool ok = !gpx || (is_gauss(gpx, gwx, nx) && is_gauss(gpy, gwy, ny));
     const float nn = n[0] * n[0] + n[1] * n[1] + n[2] * n[2];
     for (int a = 0; a < 3; ++a) {
         const int b = (a + 1) % 3, c = (a + 2) % 3;
@@ -155,10 +143,6 @@ __global__ void face_record_kernel(const float* __restrict__ verts, const int32_
 // the rule of a pair.  Both kernels below evaluate it and take disjoint sets of pairs, so its
 // arithmetic is spelled out with rounding intrinsics (no contraction that differs by context).
 // ---------------------------------------------------------------------------------------
-__device__ __forceinline__ float centre_dist2(float dx, float dy, float dz) {
-    return __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
-}
-
 template <int NX>
 __device__ __forceinline__ int pair_tier(float r2, float rho2p, float rho2q, float k2) {
     // fmaxf drops a NaN operand; the sum does not
@@ -688,6 +672,207 @@ __global__ void __launch_bounds__(128, NX <= 4 ? 4 : 3) close_pairs_kernel(const
     }
 }
 
+// ---------------------------------------------------------------------------------------
+// the 7-point-rule EFIE (mom_sym.cu) on separated pairs, in the same arithmetic: the rule's points
+// are the centroid and two orbits s A_a, so all 49 evaluations come from the pair's scalar products.
+// The operator is symmetric and both faces carry the same rule: a pair is evaluated once, p < q,
+// and added at (m, n) and (n, m).  The terms of kEdgeRows test faces are summed per thread in shared
+// memory by distinct test edge (8 faces of the sphere have 16 to 18 of 24), so that about 2 edges
+// x 3 of a face remain of 9 reductions per ordered pair: a reduction costs a cycle of its SM, which
+// with 9 bounds the whole at 13 ms for 20480 faces.
+// Measured (GB300): 20480 faces 22.35 -> 13.66 ms + 0.9 ms for the pairs left, 5120 faces 1.44 -> 0.77 + 0.17 ms;
+// (rows, slots, blocks per SM) 8/16/4 best of 4/8/5 15.4, 8/16/3 14.1, 12/22/3 14.1, 16/28/2 14.8 ms.  Bound: FMA pipe and
+// the reductions together.  Entry errors against 64 bits 0.45 .. 0.65 of the former kernel's beyond 4 edges.
+// Pairs with |D| >= 2 (rho_p + rho_q) and k (rho_p + rho_q) <= 0.6 (the phases' polynomials); the
+// others are left to mom_sym_regular_rows_kernel, which applies the same test.
+// ---------------------------------------------------------------------------------------
+constexpr int kEdgeRows = 8, kEdgeSlots = 16;
+constexpr int kEdgeSumBytes = 3 * kEdgeSlots * 128 * (int)sizeof(float2);
+
+struct EdgeSlots {
+    int id[3 * kEdgeRows], first[3 * kEdgeRows], edge[kEdgeSlots], n;
+    uint8_t slot[4 * kEdgeRows];
+};
+
+__global__ void __launch_bounds__(128, 4)
+    sym_pairs_kernel(const float* __restrict__ rec, int64_t nf, int64_t n_edges, double kd, float* __restrict__ z) {
+    constexpr float s1 = (float)(1.0 - 3.0 * 0.10128650732345634), s2 = (float)(1.0 - 3.0 * 0.47014206410511509);
+    constexpr float w0 = 0.225f, w1 = 0.12593918054482715f, w2 = 0.13239415278850619f;
+    constexpr float SA = -0.16666371f, SB = 0.00828212f;                     // sin, as in far_pairs_kernel
+    constexpr float CA = -0.49999997f, CB = 0.04166572f, CC = -0.00138007f;  // cos
+    __shared__ float4 s_rec[kEdgeRows * (kRec / 4)];
+    __shared__ EdgeSlots s_e;
+    extern __shared__ float2 s_sum[];  // [kEdgeSlots][3][128]
+    const int64_t p0 = (int64_t)blockIdx.x * kEdgeRows, q0i = (int64_t)blockIdx.y * 128, q = q0i + threadIdx.x;
+    if (q0i + 127 <= p0) return;  // no pair p < q in the tile
+    const int np = (int)min((int64_t)kEdgeRows, nf - p0), t = threadIdx.x;
+    const float4* rec4 = reinterpret_cast<const float4*>(rec);
+    for (int i = t; i < np * (kRec / 4); i += 128) s_rec[i] = __ldg(rec4 + (kRec / 4) * p0 + i);
+    if (t < 3 * np) s_e.id[t] = __float_as_int(__ldg(rec + kRec * (p0 + t / 3) + kEdge + 4 * (t % 3)));
+    __syncthreads();
+    int first = 0;
+    if (t < 3 * np) {
+        while (s_e.id[first] != s_e.id[t]) ++first;
+        s_e.first[t] = first == t;
+    }
+    __syncthreads();
+    if (t < 3 * np) {
+        int rank = 0;
+        for (int j = 0; j < first; ++j) rank += s_e.first[j];
+        s_e.slot[4 * (t / 3) + t % 3] = (uint8_t)rank;
+        if (rank < kEdgeSlots) s_e.edge[rank] = s_e.id[t];
+    }
+    if (t == 0) {
+        int n = 0;
+        for (int j = 0; j < 3 * np; ++j) n += s_e.first[j];
+        s_e.n = min(n, kEdgeSlots);
+    }
+    __syncthreads();
+    const int nslot = s_e.n;
+    float2* mine = s_sum + t;
+    for (int u = 0; u < 3 * nslot; ++u) mine[u * 128] = bc(0.f);
+    if (q >= nf) return;
+    const float4* rq = rec4 + (kRec / 4) * q;
+    const float4 q0 = __ldg(rq), q1 = __ldg(rq + 1), q2 = __ldg(rq + 2), q3 = __ldg(rq + 3), q4 = __ldg(rq + 4),
+                 q5 = __ldg(rq + 5), q6 = __ldg(rq + 6);
+    const float B[3][3] = {{q2.x, q2.y, q2.z}, {q3.x, q3.y, q3.z}, {q4.x, q4.y, q4.z}};
+    const float BB[3] = {q6.x, q6.y, q6.z}, hq[3] = {q4.w, q5.w, q6.w};
+    const int col[3] = {__float_as_int(q1.w), __float_as_int(q2.w), __float_as_int(q3.w)};
+    const float k = (float)kd, four_k = 4.f / k;
+    const double kt = kd * kInv2Pi;
+    const float kth = (float)kt, ktl = (float)(kt - (double)kth);
+    float2* z2 = reinterpret_cast<float2*>(z);
+#pragma unroll 1
+    for (int i = 0; i < np && p0 + i < q; ++i) {
+        const float4* rp = s_rec + (kRec / 4) * i;
+        const float4 p0v = rp[0];
+        const float dx = p0v.x - q0.x, dy = p0v.y - q0.y, dz = p0v.z - q0.z;
+        if (!sym_pair_far(centre_dist2(dx, dy, dz), p0v.w, q0.w, k)) continue;
+        const float4 p1v = rp[1], p2v = rp[2], p3v = rp[3], p4v = rp[4], p5v = rp[5], p6v = rp[6];
+        const float A[3][3] = {{p2v.x, p2v.y, p2v.z}, {p3v.x, p3v.y, p3v.z}, {p4v.x, p4v.y, p4v.z}};
+        const float AA[3] = {p6v.x, p6v.y, p6v.z};
+        const Centre ce = pair_centre(p0v, p1v, q0, q1, dx, dy, dz, kth, ktl, four_k);
+        const float Rc2 = ce.r2, R0 = ce.r, kp = k * (0.5f * ce.ri);
+        float mm[3][3], DA[3];
+        float2 V[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            DA[a] = fmaf(dz, A[a][2], fmaf(dy, A[a][1], dx * A[a][0]));
+            const float DB = fmaf(dz, B[a][2], fmaf(dy, B[a][1], dx * B[a][0]));
+            V[a] = make_float2(s1 * (2.f * DB - s1 * BB[a]), s2 * (2.f * DB - s2 * BB[a]));
+#pragma unroll
+            for (int b = 0; b < 3; ++b)
+                mm[a][b] = fmaf(A[a][2], B[b][2], fmaf(A[a][1], B[b][1], A[a][0] * B[b][0]));
+        }
+        // (G - 1/R_c) e^{jkR_c} at squared distance Rc2 - ns
+        auto green = [&](float2 ns, float2& gr, float2& gi) {
+            const float2 r2 = sub2(bc(Rc2), ns);
+            float2 rinv;
+            rinv.x = rsqrtf(r2.x);
+            rinv.y = rsqrtf(r2.y);
+            const float2 d0 = sub2(mul2(r2, rinv), bc(R0));
+            const float2 th = mul2(fma2(d0, d0, ns), bc(kp)), x2 = mul2(th, th);
+            const float2 sn = mul2(th, fma2(x2, fma2(x2, bc(SB), bc(SA)), bc(1.f)));
+            const float2 cs = fma2(x2, fma2(x2, fma2(x2, bc(CC), bc(CB)), bc(CA)), bc(1.f));
+            gr = sub2(mul2(rinv, cs), bc(ce.ri));
+            gi = mul2(rinv, sn);
+        };
+        float2 M0r[3], M0i[3], Ma[3], Mb[3], M00;
+        float2 Tr = bc(0.f), Ti = bc(0.f);
+#pragma unroll
+        for (int b = 0; b < 3; ++b) {  // p's centroid
+            float2 gr, gi;
+            green(V[b], gr, gi);
+            M0r[b] = mul2(bc(w0), gr);
+            M0i[b] = mul2(bc(w0), gi);
+        }
+        float c0r = 0.f, c0i = 0.f;
+        // corner by corner of p, its sums folded at once (fewer registers)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            float2 Mr[3], Mi[3];
+#pragma unroll
+            for (int o = 0; o < 2; ++o) {
+                const float s = o ? s2 : s1, w = o ? w2 : w1;
+                const float2 W = bc(w), WS = bc(w * s), K2 = make_float2(2.f * s * s1, 2.f * s * s2);
+                const float2 U = bc(-s * fmaf(s, AA[a], 2.f * DA[a]));
+#pragma unroll
+                for (int b = 0; b < 3; ++b) {
+                    float2 gr, gi;
+                    green(fma2(bc(mm[a][b]), K2, add2(U, V[b])), gr, gi);
+                    Mr[b] = o ? fma2(WS, gr, Mr[b]) : mul2(WS, gr);
+                    Mi[b] = o ? fma2(WS, gi, Mi[b]) : mul2(WS, gi);
+                    M0r[b] = fma2(W, gr, M0r[b]);
+                    M0i[b] = fma2(W, gi, M0i[b]);
+                }
+            }
+            // q's centroid: lanes p's two orbits
+            float2 cr, ci;
+            green(make_float2(-s1 * (2.f * DA[a] + s1 * AA[a]), -s2 * (2.f * DA[a] + s2 * AA[a])), cr, ci);
+            c0r += lanes(cr, w1, w2);
+            c0i += lanes(ci, w1, w2);
+            const float2 sr = add2(add2(Mr[0], Mr[1]), Mr[2]), si = add2(add2(Mi[0], Mi[1]), Mi[2]);
+            Ma[a] = make_float2(fmaf(w0, lanes(cr, w1 * s1, w2 * s2), lanes(sr, w1, w2)),
+                                fmaf(w0, lanes(ci, w1 * s1, w2 * s2), lanes(si, w1, w2)));
+#pragma unroll
+            for (int b = 0; b < 3; ++b) {
+                Tr = fma2(bc(mm[a][b]), Mr[b], Tr);
+                Ti = fma2(bc(mm[a][b]), Mi[b], Ti);
+            }
+        }
+        {
+            const float2 s0r = add2(add2(M0r[0], M0r[1]), M0r[2]), s0i = add2(add2(M0i[0], M0i[1]), M0i[2]);
+            M00 = make_float2(fmaf(w0, c0r, lanes(s0r, w1, w2)), fmaf(w0, c0i, lanes(s0i, w1, w2)));
+        }
+#pragma unroll
+        for (int b = 0; b < 3; ++b)
+            Mb[b] = make_float2(lanes(M0r[b], w1 * s1, w2 * s2), lanes(M0i[b], w1 * s1, w2 * s2));
+        const float2 M0f = add2(M00, make_float2(ce.ri, 0.f));
+        const float2 T = fma2(bc(-four_k / k), M00,
+                              make_float2(lanes(Tr, w1 * s1, w2 * s2), lanes(Ti, w1 * s1, w2 * s2)));
+        float2 v[3];
+#pragma unroll
+        for (int b = 0; b < 3; ++b)
+            v[b] = fma2(bc(mm[2][b]), Ma[2], fma2(bc(mm[1][b]), Ma[1], mul2(bc(mm[0][b]), Ma[0])));
+        const float hp[3] = {p4v.w, p5v.w, p6v.w};
+        const uint32_t slots = *reinterpret_cast<const uint32_t*>(s_e.slot + 4 * i);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const float2 u = fma2(bc(mm[a][2]), Mb[2], fma2(bc(mm[a][1]), Mb[1], mul2(bc(mm[a][0]), Mb[0])));
+            const float2 Tu = sub2(T, u);
+            const float ha = hp[a] * float(kInv4Pi);
+            const int slot = (slots >> (8 * a)) & 255;
+#pragma unroll
+            for (int b = 0; b < 3; ++b) {
+                const float2 E = fma2(bc(mm[a][b]), M0f, sub2(Tu, v[b]));
+                const float re = -k * E.y, im = k * E.x, c = ha * hq[b];
+                const float2 e = make_float2(fmaf(c, ce.br, c * fmaf(im, ce.s, fmaf(re, ce.c, ce.brl))),
+                                             fmaf(c, ce.bi, c * fmaf(-re, ce.s, fmaf(im, ce.c, ce.bil))));
+                if (slot < kEdgeSlots) {
+                    float2* d = mine + (3 * slot + b) * 128;
+                    *d = add2(*d, e);
+                } else {
+                    const int64_t m = s_e.id[3 * i + a], n = col[b];
+                    atomicAdd(z2 + m * n_edges + n, e);
+                    atomicAdd(z2 + n * n_edges + m, e);
+                }
+            }
+        }
+    }
+    for (int u = 0; u < nslot; ++u) {
+        const int64_t m = s_e.edge[u];
+#pragma unroll
+        for (int b = 0; b < 3; ++b) {
+            const float2 e = mine[(3 * u + b) * 128];
+            if (e.x != 0.f || e.y != 0.f) {
+                const int64_t n = col[b];
+                atomicAdd(z2 + m * n_edges + n, e);
+                atomicAdd(z2 + n * n_edges + m, e);
+            }
+        }
+    }
+}
+
 }  // namespace
 
 // Tile sizes: 32 test faces per block of tier 1 once that leaves 8 blocks per SM (its per-thread
@@ -751,6 +936,25 @@ int launch_mom_tiers_batched(const float* verts, const int32_t* faces, int64_t t
     if (int rc = tier_records(verts, faces, normals, fei, total_faces, gpx, gwx, nx, gpy, gwy, ny, rec, s)) return rc;
     const TierArgs a{verts, faces, areas, normals, rec, gpx, gwx, gpy, gwy, desc, nullptr, ks, n_mesh, 0, 0, 0.0, z};
     return MB_TIERS(a, far_blocks, close_blocks, rows, tp, tq, far_off, close_off, s);
+}
+
+// The separated pairs of the 7-point-rule EFIE over the whole mesh: records, sym_pairs_kernel, then the
+// pairs it leaves (mom_sym.cu).
+int launch_mom_sym_rest(const float* verts, const int32_t* faces, const int32_t* fei, int64_t n_edges, double k, int64_t nf,
+                        const float* rec, float* z, cudaStream_t s);
+
+int launch_mom_sym_pairs(const float* verts, const int32_t* faces, const int32_t* fei, int64_t nf, int64_t n_edges, double k,
+                         float* rec, float* z, cudaStream_t s) {
+    if (nf <= 0) return MB_OK;
+    if (int rc = tier_records(verts, faces, nullptr, fei, nf, nullptr, nullptr, 0, nullptr, nullptr, 0, rec, s)) return rc;
+    const int64_t gx = (nf + kEdgeRows - 1) / kEdgeRows, gy = (nf + 127) / 128;
+    if (gx > 0x7fffffffLL || gy > 65535) return set_error(MB_ERR_SIZE, "mesh too large for one launch");
+    const cudaError_t e = cudaFuncSetAttribute(sym_pairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kEdgeSumBytes);
+    if (e != cudaSuccess) return set_error(MB_ERR_CUDA, "%s", cudaGetErrorString(e));
+    // test groups fastest: blocks in flight share the rows of one source tile for the transposed terms
+    sym_pairs_kernel<<<dim3((unsigned)gx, (unsigned)gy), 128, kEdgeSumBytes, s>>>(rec, nf, n_edges, k, z);
+    if (int rc = check_launch("mom sym pairs")) return rc;
+    return launch_mom_sym_rest(verts, faces, fei, n_edges, k, nf, rec, z, s);
 }
 
 }  // namespace mb

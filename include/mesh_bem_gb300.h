@@ -577,8 +577,8 @@ int mb_spai_apply_c64(const int32_t* m_cols, const float* m_vals, int64_t n, con
  * residual b - Z x, solves (Z M) u = r and adds M u to x.  The whole cycle runs on the device
  * (CGS2 Arnoldi, Givens rotations, the residual estimate and the back substitution in
  * kernels; Hessenberg matrix, rotations and x in FP64; deterministic block reductions);
- * use_graph = 1 captures it once as a CUDA graph and replays it.  The host reads the solver
- * state once per cycle.
+ * use_graph = 1 captures a group of its steps once as a CUDA graph and replays it.  The host
+ * reads the solver state after every group.
  * mb_pgmres_c64: Z interleaved complex64 [n, n]; FP32 products, complex64 Krylov basis with
  * FP32 Gram-Schmidt products and FP64 sums; the refinement residual by compensated FP32 dot
  * products (exact products and sums, ~1e-13 of sum |Z_ij x_j|).  With z_half (from

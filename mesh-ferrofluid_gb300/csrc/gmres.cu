@@ -713,9 +713,9 @@ int launch_residual_c128(const float* z, const double* x, const double* b, int64
 // substitution and x stay in FP64, in one-warp kernels on a device state record.  Sums over
 // the vector run as block partials that the last block to finish adds in a fixed order
 // (deterministic, no FP64 atomics).  A cycle is a fixed sequence of launches: once the state
-// says the cycle has ended, the remaining steps' launches return at once.  With use_graph the
-// cycle is captured once as a CUDA graph and replayed; the host reads the state once per
-// cycle.
+// says the cycle has ended, the remaining steps' launches return at once.  With use_graph a group of
+// steps is captured once as a CUDA graph and replayed; the host reads the state after every
+// group.
 //
 // Three matrix kinds:
 //   0  complex64 Z: FP32 products; the Krylov basis is complex64 and the Gram-Schmidt
@@ -906,11 +906,15 @@ __global__ void pg_start_basis_kernel(const double2* __restrict__ r, int64_t n, 
     v0[k] = PgB<B>::make(r[k].x * s, r[k].y * s);
 }
 
+// A step's kernels take its number from the state: st->jdone steps are done, V_jdone is the newest basis
+// vector (pg_givens_kernel advances it), so one captured group of steps serves every part of a cycle.
+
 // V_{j+1} = w / h_{j+1,j}
 template <typename B>
 __global__ void pg_scale_kernel(const B* __restrict__ w, int64_t n, const PgState* __restrict__ st,
-                                B* __restrict__ dst) {
+                                B* __restrict__ V) {
     if (!st->active) return;
+    B* __restrict__ dst = V + (int64_t)st->jdone * n;
     const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     using S = typename PgB<B>::S;
@@ -927,9 +931,10 @@ __global__ void pg_scale_kernel(const B* __restrict__ w, int64_t n, const PgStat
 template <typename B>
 __global__ void __launch_bounds__(256) pg_precond_kernel(const int32_t* __restrict__ cols,
                                                          const float2* __restrict__ vals, int64_t n,
-                                                         const B* __restrict__ v, B* __restrict__ z,
+                                                         const B* __restrict__ V, B* __restrict__ z,
                                                          const PgState* __restrict__ st) {
     if (!st->active) return;
+    const B* __restrict__ v = V + (int64_t)st->jdone * n;
     using S = typename PgB<B>::S;
     const int64_t row = (int64_t)blockIdx.x * kPgRowsPerBlock + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
@@ -1144,10 +1149,13 @@ __global__ void __launch_bounds__(256) residual_c64x_kernel(const float2* __rest
 // chunks).
 template <typename B>
 __global__ void __launch_bounds__(256) pg_dots_kernel(const B* __restrict__ V, const B* __restrict__ w, int64_t n,
-                                                      int nb, int64_t chunk, double2* __restrict__ part, int ldp,
+                                                      int64_t chunk, double2* __restrict__ part, int ldp,
                                                       unsigned* cnt, double2* __restrict__ h,
-                                                      const int* __restrict__ active) {
-    if (!*active) return;
+                                                      const PgState* __restrict__ st) {
+    if (!st->active) return;
+    const int nb = st->jdone + 1;
+    const unsigned groups = (unsigned)(nb + 7) / 8;  // the grid is sized for the restart length
+    if (blockIdx.y >= groups) return;
     using S = typename PgB<B>::S;
     __shared__ bool s_last;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1176,7 +1184,7 @@ __global__ void __launch_bounds__(256) pg_dots_kernel(const B* __restrict__ V, c
     }
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd(cnt, 1u) == gridDim.x * gridDim.y - 1;
+    if (threadIdx.x == 0) s_last = atomicAdd(cnt, 1u) == gridDim.x * groups - 1;
     __syncthreads();
     if (!s_last) return;
     for (int ii = warp; ii < nb; ii += 8) {
@@ -1197,9 +1205,10 @@ __global__ void __launch_bounds__(256) pg_dots_kernel(const B* __restrict__ V, c
 // unrolled by four); with npart, also |w|^2 into *hn2 (FP64 block partials + last block).
 template <typename B>
 __global__ void __launch_bounds__(128) pg_sub_kernel(const B* __restrict__ V, const double2* __restrict__ h, int64_t n,
-                                                     int nb, B* __restrict__ w, double* __restrict__ npart,
-                                                     unsigned* cnt, double* hn2, const int* __restrict__ active) {
-    if (!*active) return;
+                                                     B* __restrict__ w, double* __restrict__ npart, unsigned* cnt,
+                                                     double* hn2, const PgState* __restrict__ st) {
+    if (!st->active) return;
+    const int nb = st->jdone + 1;
     using S = typename PgB<B>::S;
     __shared__ B sh[kGmresMaxRestart + 1];
     __shared__ double s[4];
@@ -1240,11 +1249,13 @@ __global__ void __launch_bounds__(128) pg_sub_kernel(const B* __restrict__ V, co
 // memory with the previous rotations; lane 0 applies them, forms the new rotation, updates
 // the residual estimate and decides whether the cycle ends.
 __global__ void __launch_bounds__(32) pg_givens_kernel(PgState* st, double2* g, double2* cs, double2* sn,
-                                                       double2* H, const double2* h1, const double2* h2, int j) {
+                                                       double2* H, const double2* h1, const double2* h2) {
     if (!st->active) return;
+    const int j = st->jdone;
     __shared__ double2 col[kGmresMaxRestart + 1], scs[kGmresMaxRestart], ssn[kGmresMaxRestart];
     const int lane = threadIdx.x;
     const int m = st->m;
+    __syncwarp();  // every lane has read the step's number before lane 0 advances it
     for (int i = lane; i <= j; i += 32) col[i] = make_double2(h1[i].x + h2[i].x, h1[i].y + h2[i].y);
     for (int i = lane; i < j; i += 32) {
         scs[i] = cs[i];
@@ -1343,20 +1354,17 @@ struct PgMatrix {
     const float* scale;  // kind 2: its scale (device)
 };
 
+// Steps per captured group.  A cycle usually ends well before its m steps (kind 2 stops once it has gained
+// inner_rtol), and the launches of a step after that, each returning at once, cost a microsecond
+// each: with whole cycles of 50 captured, 1.8 of 13.6 ms at 7680 unknowns, and 1.5 ms of capturing,
+// instantiating and launching 400 nodes.  The host reads the state after every group.
+constexpr int kPgGroup = 8;
+
 template <typename B>
-static void pg_cycle_t(const PgMatrix& A, int64_t n, const int32_t* cols, const float2* vals, const double2* b,
-                       double2* x, int m, const PgWork& W, unsigned* cnt, cudaStream_t s) {
+static void pg_head_t(const PgMatrix& A, int64_t n, const double2* b, const double2* x, const PgWork& W, unsigned* cnt,
+                      cudaStream_t s) {
     const unsigned vb = (unsigned)((n + 255) / 256), rb = (unsigned)((n + 7) / 8);
     const int nblk = (int)std::min<int64_t>(vb, kPgMaxBlocks);
-    const int sblk = (int)std::min<int64_t>((n + 127) / 128, kPgMaxBlocks);
-    // dot-product chunks: at least 1024 elements, at most kPgMaxBlocks chunks
-    int64_t chunk = 1024;
-    while ((n + chunk - 1) / chunk > kPgMaxBlocks) chunk *= 2;
-    const unsigned nchunk = (unsigned)((n + chunk - 1) / chunk);
-    const int* act = &W.st->active;
-    B* V = static_cast<B*>(W.V);
-    B* w = static_cast<B*>(W.w);
-    B* z = reinterpret_cast<B*>(W.z);
     if (A.kind == 1) {
         residual_z128_kernel<<<rb, 256, 0, s>>>(static_cast<const double2*>(A.z), x, b, n, W.r);
     } else {
@@ -1366,11 +1374,25 @@ static void pg_cycle_t(const PgMatrix& A, int64_t n, const int32_t* cols, const 
     }
     pg_norm2_kernel<<<nblk, 256, 0, s>>>(W.r, n, W.npart, cnt, &W.st->rn2);
     pg_cycle_start_kernel<<<1, 1, 0, s>>>(W.st, W.g);
-    pg_start_basis_kernel<B><<<vb, 256, 0, s>>>(W.r, n, W.st, V);
-    for (int j = 0; j < m; ++j) {
-        const B* vj = V + (int64_t)j * n;
-        const dim3 dgrid(nchunk, (unsigned)((j + 1 + 7) / 8));
-        pg_precond_kernel<B><<<rb, 256, 0, s>>>(cols, vals, n, vj, z, W.st);
+    pg_start_basis_kernel<B><<<vb, 256, 0, s>>>(W.r, n, W.st, static_cast<B*>(W.V));
+}
+
+template <typename B>
+static void pg_steps_t(const PgMatrix& A, int64_t n, const int32_t* cols, const float2* vals, int m, const PgWork& W,
+                       unsigned* cnt, cudaStream_t s) {
+    const unsigned vb = (unsigned)((n + 255) / 256), rb = (unsigned)((n + 7) / 8);
+    const int sblk = (int)std::min<int64_t>((n + 127) / 128, kPgMaxBlocks);
+    // dot-product chunks: at least 1024 elements, at most kPgMaxBlocks chunks
+    int64_t chunk = 1024;
+    while ((n + chunk - 1) / chunk > kPgMaxBlocks) chunk *= 2;
+    const unsigned nchunk = (unsigned)((n + chunk - 1) / chunk);
+    const dim3 dgrid(nchunk, (unsigned)((m + 7) / 8));
+    const int* act = &W.st->active;
+    B* V = static_cast<B*>(W.V);
+    B* w = static_cast<B*>(W.w);
+    B* z = reinterpret_cast<B*>(W.z);
+    for (int j = 0; j < kPgGroup; ++j) {
+        pg_precond_kernel<B><<<rb, 256, 0, s>>>(cols, vals, n, V, z, W.st);
         if constexpr (sizeof(B) == 8) {
             if (A.kind == 2)
                 pg_matvec_h16_kernel<<<rb, 256, 0, s>>>(A.zh, A.scale, reinterpret_cast<const float2*>(z), n,
@@ -1384,22 +1406,21 @@ static void pg_cycle_t(const PgMatrix& A, int64_t n, const int32_t* cols, const 
                                                   reinterpret_cast<const double2*>(z), n,
                                                   reinterpret_cast<double2*>(w), act);
         }
-        pg_dots_kernel<B><<<dgrid, 256, 0, s>>>(V, w, n, j + 1, chunk, W.part, m + 1, cnt, W.h1, act);
-        pg_sub_kernel<B><<<sblk, 128, 0, s>>>(V, W.h1, n, j + 1, w, nullptr, cnt, nullptr, act);
-        pg_dots_kernel<B><<<dgrid, 256, 0, s>>>(V, w, n, j + 1, chunk, W.part, m + 1, cnt, W.h2, act);
-        pg_sub_kernel<B><<<sblk, 128, 0, s>>>(V, W.h2, n, j + 1, w, W.npart, cnt, &W.st->hn2, act);
-        pg_givens_kernel<<<1, 32, 0, s>>>(W.st, W.g, W.cs, W.sn, W.H, W.h1, W.h2, j);
-        pg_scale_kernel<B><<<vb, 256, 0, s>>>(w, n, W.st, V + (int64_t)(j + 1) * n);
+        pg_dots_kernel<B><<<dgrid, 256, 0, s>>>(V, w, n, chunk, W.part, m + 1, cnt, W.h1, W.st);
+        pg_sub_kernel<B><<<sblk, 128, 0, s>>>(V, W.h1, n, w, nullptr, cnt, nullptr, W.st);
+        pg_dots_kernel<B><<<dgrid, 256, 0, s>>>(V, w, n, chunk, W.part, m + 1, cnt, W.h2, W.st);
+        pg_sub_kernel<B><<<sblk, 128, 0, s>>>(V, W.h2, n, w, W.npart, cnt, &W.st->hn2, W.st);
+        pg_givens_kernel<<<1, 32, 0, s>>>(W.st, W.g, W.cs, W.sn, W.H, W.h1, W.h2);
+        pg_scale_kernel<B><<<vb, 256, 0, s>>>(w, n, W.st, V);
     }
-    pg_backsub_kernel<<<1, 32, 0, s>>>(W.st, W.H, W.g, W.y);
-    pg_combine_kernel<B><<<vb, 256, 0, s>>>(V, W.y, W.st, n, W.r);
-    pg_update_kernel<<<vb, 256, 0, s>>>(cols, vals, W.r, W.st, n, x);
 }
 
-static void pg_cycle(const PgMatrix& A, int64_t n, const int32_t* cols, const float2* vals, const double2* b,
-                     double2* x, int m, const PgWork& W, unsigned* cnt, cudaStream_t s) {
-    if (A.kind == 1) pg_cycle_t<double2>(A, n, cols, vals, b, x, m, W, cnt, s);
-    else pg_cycle_t<float2>(A, n, cols, vals, b, x, m, W, cnt, s);
+template <typename B>
+static void pg_tail_t(int64_t n, const int32_t* cols, const float2* vals, double2* x, const PgWork& W, cudaStream_t s) {
+    const unsigned vb = (unsigned)((n + 255) / 256);
+    pg_backsub_kernel<<<1, 32, 0, s>>>(W.st, W.H, W.g, W.y);
+    pg_combine_kernel<B><<<vb, 256, 0, s>>>(static_cast<const B*>(W.V), W.y, W.st, n, W.r);
+    pg_update_kernel<<<vb, 256, 0, s>>>(cols, vals, W.r, W.st, n, x);
 }
 
 int pgmres(int kind, const void* z, const void* z_half, const float* half_scale, double inner_rtol, int64_t n,
@@ -1443,27 +1464,41 @@ int pgmres(int kind, const void* z, const void* z_half, const float* half_scale,
         if (graph) cudaGraphDestroy(graph);
         if (cap) cudaStreamDestroy(cap);
     };
+    auto steps = [&](cudaStream_t t) {
+        if (kind == 1) pg_steps_t<double2>(A, n, m_cols, vals, m, W, cnt, t);
+        else pg_steps_t<float2>(A, n, m_cols, vals, m, W, cnt, t);
+    };
     if (use_graph) {
         if (cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking) != cudaSuccess ||
             cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
             return cleanup(), set_error(MB_ERR_CUDA, "pgmres: stream capture failed");
-        pg_cycle(A, n, m_cols, vals, b2, x2, m, W, cnt, cap);
+        steps(cap);
         cudaError_t ce = cudaStreamEndCapture(cap, &graph);
         if (ce != cudaSuccess || cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess)
             return cleanup(), set_error(MB_ERR_CUDA, "pgmres: graph capture / instantiate failed");
     }
     PgState hs{};
     const long long max_cycles = (long long)max_iters + 2;
-    for (long long c = 0; c < max_cycles; ++c) {
-        if (use_graph) {
-            if (cudaGraphLaunch(exec, s) != cudaSuccess)
-                return cleanup(), set_error(MB_ERR_CUDA, "pgmres: graph launch failed");
-        } else {
-            pg_cycle(A, n, m_cols, vals, b2, x2, m, W, cnt, s);
-        }
+    auto read_state = [&]() -> int {
         cudaMemcpyAsync(&hs, W.st, sizeof(PgState), cudaMemcpyDeviceToHost, s);
-        if ((rc = sync_check(s, "pgmres cycle"))) return cleanup(), rc;
+        return sync_check(s, "pgmres cycle");
+    };
+    for (long long c = 0; c < max_cycles; ++c) {
+        if (kind == 1) pg_head_t<double2>(A, n, b2, x2, W, cnt, s);
+        else pg_head_t<float2>(A, n, b2, x2, W, cnt, s);
+        for (int j = 0; j < m; j += kPgGroup) {
+            if (use_graph) {
+                if (cudaGraphLaunch(exec, s) != cudaSuccess)
+                    return cleanup(), set_error(MB_ERR_CUDA, "pgmres: graph launch failed");
+            } else {
+                steps(s);
+            }
+            if ((rc = read_state())) return cleanup(), rc;
+            if (!hs.active) break;
+        }
         if (hs.converged || hs.jdone == 0) break;
+        if (kind == 1) pg_tail_t<double2>(n, m_cols, vals, x2, W, s);
+        else pg_tail_t<float2>(n, m_cols, vals, x2, W, s);
     }
     cleanup();
     if (iters_out) *iters_out = hs.iters;

@@ -462,19 +462,25 @@ int zmat_edges_to_host(const float* verts, const int32_t* faces, const float* ar
     return check_launch("zmat to host");
 }
 
-// Launches the fast path for float and supported rule sizes; returns false otherwise.
-template <typename T>
-bool launch_fast_zmat(const T*, const int32_t*, const T*, const T*, const int32_t*, int64_t, const T*,
-                      const T*, int, const T*, const T*, int, double, int64_t, int64_t, int64_t, int64_t,
-                      unsigned, T*, T*, cudaStream_t) {
-    return false;
+bool launch_mom_f64(const double* verts, const int32_t* faces, const double* areas, const double* normals,
+                    const int32_t* fei, int64_t n_edges, const double* gpx, const double* gwx, int nx,
+                    const double* gpy, const double* gwy, int ny, double k, int64_t nf, int64_t batch,
+                    int64_t row_begin, int64_t row_end, double* zr, double* zi, cudaStream_t stream);
+
+// Launches the kernel made for the type and rule sizes; returns false if there is none.
+bool launch_fast_zmat(const double* verts, const int32_t* faces, const double* areas, const double* normals,
+                      const int32_t* fei, int64_t n_edges, const double* gpx, const double* gwx, int nx,
+                      const double* gpy, const double* gwy, int ny, double k, int64_t nf, int64_t batch,
+                      int64_t row_begin, int64_t row_end, int64_t, unsigned, double* zr, double* zi,
+                      cudaStream_t stream) {
+    return launch_mom_f64(verts, faces, areas, normals, fei, n_edges, gpx, gwx, nx, gpy, gwy, ny, k, nf, batch,
+                          row_begin, row_end, zr, zi, stream);
 }
-template <>
-bool launch_fast_zmat<float>(const float* verts, const int32_t* faces, const float* areas,
-                             const float* normals, const int32_t* fei, int64_t n_edges, const float* gpx,
-                             const float* gwx, int nx, const float* gpy, const float* gwy, int ny, double k,
-                             int64_t nf, int64_t batch, int64_t row_begin, int64_t col_blocks,
-                             unsigned blocks, float* zr, float* zi, cudaStream_t stream) {
+bool launch_fast_zmat(const float* verts, const int32_t* faces, const float* areas, const float* normals,
+                      const int32_t* fei, int64_t n_edges, const float* gpx, const float* gwx, int nx,
+                      const float* gpy, const float* gwy, int ny, double k, int64_t nf, int64_t batch,
+                      int64_t row_begin, int64_t, int64_t col_blocks, unsigned blocks, float* zr, float* zi,
+                      cudaStream_t stream) {
 #define MB_FAST(NXV, NYV)                                                                          \
     if (nx == NXV && ny == NYV) {                                                                  \
         if (fei)                                                                                   \
@@ -646,10 +652,9 @@ int launch_mom_ref_zmat(const T* verts, int64_t nv, const int32_t* faces, int64_
     const int64_t blocks = rows * col_blocks;
     if (blocks <= 0) return MB_OK;
     if (blocks > 0x7fffffffLL) return set_error(MB_ERR_SIZE, "mesh too large for one launch");
-    if (launch_fast_zmat<T>(verts, faces, areas, normals, fei, n_edges, gpx, gwx, nx, gpy, gwy, ny, k, nf,
-                            batch, row_begin, col_blocks, (unsigned)blocks, zr, zi, stream))
+    if (launch_fast_zmat(verts, faces, areas, normals, fei, n_edges, gpx, gwx, nx, gpy, gwy, ny, k, nf, batch,
+                         row_begin, row_end, col_blocks, (unsigned)blocks, zr, zi, stream))
         return check_launch("mom_ref_zmat");
-    const int ns = ny * ny;
 #define MB_ZMAT_LAUNCH(NSV)                                                                              \
     do {                                                                                                \
         if (fei == nullptr)                                                                             \
@@ -661,12 +666,16 @@ int launch_mom_ref_zmat(const T* verts, int64_t nv, const int32_t* faces, int64_
                 verts, faces, areas, normals, fei, n_edges, gpx, gwx, nx, gpy, gwy, ny, (T)k, nf,        \
                 row_begin, col_blocks, zr);                                                             \
     } while (0)
-    switch (ns) {
-        case 1: MB_ZMAT_LAUNCH(1); break;
-        case 4: MB_ZMAT_LAUNCH(4); break;
-        case 9: MB_ZMAT_LAUNCH(9); break;
-        case 16: MB_ZMAT_LAUNCH(16); break;
-        default: MB_ZMAT_LAUNCH(0); break;
+    if constexpr (sizeof(T) == 4) {
+        switch (ny * ny) {
+            case 1: MB_ZMAT_LAUNCH(1); break;
+            case 4: MB_ZMAT_LAUNCH(4); break;
+            case 9: MB_ZMAT_LAUNCH(9); break;
+            case 16: MB_ZMAT_LAUNCH(16); break;
+            default: MB_ZMAT_LAUNCH(0); break;
+        }
+    } else {
+        MB_ZMAT_LAUNCH(0);  // FP64 with ny <= 4 went to launch_mom_f64
     }
 #undef MB_ZMAT_LAUNCH
     return check_launch("mom_ref_zmat");

@@ -111,6 +111,17 @@ int mb_shared_vertex_pairs_count(const int32_t* faces, int64_t n_faces, int64_t 
 int mb_shared_vertex_pairs_fill(const int32_t* faces, int64_t n_faces, int64_t n_verts, void* workspace,
                                 int32_t* pairs, void* stream);
 
+/* Face areas [F] and unit normals [F, 3] (face_normals may be NULL) of the reference's compute_face_areas /
+ * compute_face_normals (mesh_utils.py:158-310): |e0 x e1| / 2 and e0 x e1 / max(|e0 x e1|, 1e-12).  A face with an
+ * index outside [0, n_verts) gets zeros. */
+int mb_face_geometry_f32(const float* verts, int64_t n_verts, const int32_t* faces, int64_t n_faces,
+                         float* face_areas, float* face_normals, void* stream);
+int mb_face_geometry_f64(const double* verts, int64_t n_verts, const int32_t* faces, int64_t n_faces,
+                         double* face_areas, double* face_normals, void* stream);
+/* *outside (host) = 1 if one of the indices is not in [0, limit), else 0; waits for the stream.  work: 4 bytes of
+ * device memory. */
+int mb_index_range_i32(const int32_t* indices, int64_t count, int64_t limit, int32_t* work, int32_t* outside,
+                       void* stream);
 /* No counterpart in the reference (its scatter_add_ runs after the whole face-edge matrix
  * exists).  edge_rows [2 n_edges + 1] int32: for Z row m (edge m) the face-edge rows 3f + e
  * of its faces (smaller first; -1 for a missing second face); edge_rows[2 n_edges] = 1 when

@@ -88,6 +88,10 @@ int gnn_aggregate_bwd(const float* dcat, const int32_t* nbr, int64_t N, int F, f
 int gnn_relu_bwd(const void* y, const float* dy, int64_t count, float* dz, cudaStream_t s);
 int gnn_adam(float* w, float* m1, float* m2, const float* g, int64_t count, float lr, float b1, float b2, float eps,
              int step, void* w16, cudaStream_t s);
+template <typename T>
+int launch_face_geometry(const T* verts, int64_t nv, const int32_t* faces, int64_t nf, T* areas, T* normals,
+                         cudaStream_t s);
+int index_range(const int32_t* idx, int64_t count, int64_t limit, int32_t* work, int32_t* outside, cudaStream_t s);
 int launch_edge_rows(const int32_t* fei, int64_t nf, int64_t n_edges, int32_t* er, cudaStream_t s);
 bool mom_tier_rule(int nx, int ny);
 int launch_mom_sym_pairs(const float* verts, const int32_t* faces, const int32_t* fei, int64_t nf, int64_t n_edges, double k,
@@ -289,6 +293,25 @@ int mb_mom_zmat_rwg_edges_c64(const float* verts, int64_t n_verts, const int32_t
                                 as_stream(stream)))
         return set_error(MB_ERR_UNSUPPORTED, "edge-row assembly: no instance for rule sizes (%d, %d)", n_x, n_y);
     return check_launch("mom_ref_zmat_edges");
+}
+
+#define MB_FACE_GEOMETRY(SFX, T)                                                                          \
+    int mb_face_geometry_##SFX(const T* verts, int64_t n_verts, const int32_t* faces, int64_t n_faces,      \
+                               T* face_areas, T* face_normals, void* stream) {                              \
+        MB_REQUIRE(n_verts >= 0 && n_faces >= 0, "negative size");                                          \
+        if (n_faces == 0) return MB_OK;                                                                     \
+        MB_REQUIRE(faces && face_areas && (verts || n_verts == 0), "null pointer argument");                \
+        return launch_face_geometry<T>(verts, n_verts, faces, n_faces, face_areas, face_normals,            \
+                                       as_stream(stream));                                                  \
+    }
+MB_FACE_GEOMETRY(f32, float)
+MB_FACE_GEOMETRY(f64, double)
+#undef MB_FACE_GEOMETRY
+
+int mb_index_range_i32(const int32_t* indices, int64_t count, int64_t limit, int32_t* work, int32_t* outside,
+                       void* stream) {
+    MB_REQUIRE(count >= 0 && outside && (count == 0 || (indices && work)), "null pointer argument or negative count");
+    return index_range(indices, count, limit, work, outside, as_stream(stream));
 }
 
 int64_t mb_mom_tiers_workspace_bytes(int64_t n_faces) { return n_faces > 0 ? 128 * n_faces : 0; }

@@ -50,6 +50,7 @@ from .mesh_MOM_3d import (
     assemble_rhs_rwg_sym,
     assemble_Z_rwg,
     assemble_Z_rwg_sym,
+    face_geometry,
     gmres,
     gmres_real,
     interpolate_vert_js,
@@ -59,8 +60,6 @@ from .utils import (
     BEMType,
     BoundaryType,
     OrderType,
-    compute_face_areas,
-    compute_face_normals,
     compute_panel_relation,
     compute_vert_areas,
     get_gaussion_integration_points_and_weights,
@@ -160,18 +159,17 @@ class MeshBEMSolver3d:
         faces = faces.to(torch.int32).contiguous()
         fei = face_edge_indices.to(torch.int32).reshape(-1).contiguous()
         dev, dt = verts.device, verts.dtype
-        areas = compute_face_areas(vertices=verts, faces=faces, keepdim=True).contiguous()
+        areas, normals = face_geometry(verts, faces)
         if waves is None:
             waves = reference_plane_wave(self.wavenumber, device=dev)
         if self.rule == "dunavant7":
             Z = assemble_Z_rwg_sym(verts, faces, fei, n_edges, self.wavenumber)
-            rhs = assemble_rhs_rwg_sym(verts, faces, fei, n_edges, waves)
+            rhs = assemble_rhs_rwg_sym(verts, faces, fei, n_edges, waves, check_indices=False)  # as for Z
             return Z, rhs, areas
         gpx, gwx, gpy, gwy, gp, gw = self._rules_on(dev, dt)
-        normals = compute_face_normals(vertices=verts, faces=faces).contiguous()
         Z = assemble_Z_rwg(verts, faces, areas, normals, fei, n_edges, gpx, gwx, gpy, gwy,
                            self.wavenumber)
-        rhs = assemble_rhs_rwg(verts, faces, areas, normals, fei, n_edges, gp, gw, waves)
+        rhs = assemble_rhs_rwg(verts, faces, areas, normals, fei, n_edges, gp, gw, waves, check_indices=False)  # as for Z
         return Z, rhs, areas
 
     def solve_MOM(self, verts: torch.Tensor, faces: torch.Tensor, edges: torch.Tensor,
@@ -201,8 +199,7 @@ class MeshBEMSolver3d:
         sym = self.rule == "dunavant7" and not BEMType.belong_Helmholtz(self.BEM_type)
         areas = normals = None
         if not sym:  # the reference rule's layers take them
-            areas = compute_face_areas(vertices=verts, faces=faces, keepdim=True).contiguous()
-            normals = compute_face_normals(vertices=verts, faces=faces).contiguous()
+            areas, normals = face_geometry(verts, faces)
         # the symmetric rule needs only the face pairs sharing a vertex (O(F)), not the
         # dense [F, F] relation of the reference rule
         near = shared_vertex_pairs(faces, n_verts) if sym else None

@@ -24,6 +24,8 @@ import math
 import torch
 
 from . import _lib
+from .utils import compute_face_areas, compute_face_normals
+from .utils import indices_outside as _indices_outside
 
 _FLOATS = (torch.float32, torch.float64)
 
@@ -47,6 +49,30 @@ def _mesh_args(verts, faces, face_areas, face_normals):
     return dt, dev, verts.shape[0], nf
 
 
+def face_geometry(verts, faces):
+    """Face areas [F, 1] and unit normals [F, 3] of a mesh, as ``utils.compute_face_areas`` and
+    ``utils.compute_face_normals`` give them.
+
+    One kernel for what a kernel can take: a CUDA mesh of float32 or float64 vertices [V, 3] and int32 faces [F, 3],
+    contiguous, whose vertices carry no gradient and no tangent.  Everything else goes to those two functions.  Face
+    indices are not checked here: a face with one out of range gets zeros."""
+    plain = (type(verts) in (torch.Tensor, torch.nn.Parameter) and type(faces) is torch.Tensor and verts.is_cuda
+             and verts.dtype in _FLOATS and verts.dim() == 2 and verts.shape[1] == 3 and verts.is_contiguous()
+             and faces.device == verts.device and faces.dtype == torch.int32 and faces.dim() == 2
+             and faces.shape[1] == 3 and faces.is_contiguous()
+             and not (verts.requires_grad and torch.is_grad_enabled())
+             and torch.autograd.forward_ad.unpack_dual(verts).tangent is None)
+    if not plain:
+        areas = compute_face_areas(verts, faces, keepdim=True).contiguous()
+        return areas, compute_face_normals(verts, faces).contiguous()
+    nf = faces.shape[0]
+    areas = torch.empty((nf, 1), dtype=verts.dtype, device=verts.device)
+    normals = torch.empty((nf, 3), dtype=verts.dtype, device=verts.device)
+    _lib.call(f"mb_face_geometry_{_lib.sfx(verts.dtype)}", _lib.ptr(verts), verts.shape[0], _lib.ptr(faces), nf,
+              _lib.ptr(areas), _lib.ptr(normals), _lib.stream_of(verts))
+    return areas, normals
+
+
 # face tensors already checked: (tensor, version counter, vertex count); an entry holds its
 # tensor, so the identity cannot be taken by another tensor while the entry lives
 _CHECKED_FACES: list = []
@@ -54,14 +80,13 @@ _CHECKED_FACES_MAX = 8
 
 
 def check_face_range(faces, n_verts):
-    """Vertex ids must index ``verts``; the kernels trust them (one reduction, one sync -- once
+    """Vertex ids must index ``verts``; the kernels trust them (one kernel, one sync -- once
     per face tensor and vertex count while the tensor is not modified in place)."""
     if faces.numel():
         for held, ver, nv in _CHECKED_FACES:
             if held is faces and ver == faces._version and nv == n_verts:
                 return
-        lo, hi = torch.aminmax(faces)
-        if int(lo) < 0 or int(hi) >= n_verts:
+        if _indices_outside(faces, n_verts):
             raise ValueError(f"faces reference vertex ids outside [0, {n_verts})")
         _CHECKED_FACES.append((faces, faces._version, int(n_verts)))
         del _CHECKED_FACES[:-_CHECKED_FACES_MAX]
@@ -138,8 +163,7 @@ def interpolate_Icoeff_to_Js_3d_forward(verts, faces, face_edge_indices, face_ar
         if t.numel() != batch * 9 * nf:
             raise ValueError(f"{nm} must be [B, 3F, 3]")
     if nf:
-        fei_max = int(face_edge_indices.max().item())
-        if fei_max >= n_edges or int(face_edge_indices.min().item()) < 0:
+        if _indices_outside(face_edge_indices, n_edges):
             raise ValueError("face_edge_indices out of range of the edge coefficients")
     _lib.call(f"mb_mom_interp_js_{_lib.sfx(dt)}", _lib.ptr(verts), verts.shape[0], _lib.ptr(faces), nf,
               _lib.ptr(face_edge_indices), _lib.ptr(face_areas), _lib.ptr(edge_I_coeff_real),
@@ -154,7 +178,7 @@ def _check_fei(face_edge_indices, nf, n_edges, dev):
     _lib.check_tensor(face_edge_indices, "face_edge_indices", dtype=torch.int32, device=dev)
     if face_edge_indices.numel() != 3 * nf:
         raise ValueError("face_edge_indices must have 3F entries")
-    if nf and (int(face_edge_indices.max().item()) >= n_edges or int(face_edge_indices.min().item()) < 0):
+    if nf and _indices_outside(face_edge_indices, n_edges):
         raise ValueError("face_edge_indices out of range [0, n_edges)")
 
 
@@ -288,11 +312,12 @@ def reference_plane_wave(wavenumber: float, device=None) -> torch.Tensor:
 
 
 def assemble_rhs_rwg(verts, faces, face_areas, face_normals, face_edge_indices, n_edges,
-                     gaussian_points_1d, gaussian_weights_1d, waves, out=None):
+                     gaussian_points_1d, gaussian_weights_1d, waves, out=None, check_indices=True):
     """Excitation vectors [E, n_rhs] complex for the plane waves ``waves`` ([n_rhs, 9] float64)."""
     dt, dev, nv, nf = _mesh_args(verts, faces, face_areas, face_normals)
     n = _rule(gaussian_points_1d, gaussian_weights_1d, "rule", dt, dev)
-    _check_fei(face_edge_indices, nf, n_edges, dev)
+    if check_indices:
+        _check_fei(face_edge_indices, nf, n_edges, dev)
     waves = waves.to(device=dev, dtype=torch.float64).contiguous()
     _lib.check_tensor(waves, "waves", dtype=torch.float64, device=dev, ndim=2)
     if waves.shape[1] != 9:
@@ -399,14 +424,15 @@ def assemble_Z_rwg_sym(verts, faces, face_edge_indices, n_edges, wavenumber, out
     return out
 
 
-def assemble_rhs_rwg_sym(verts, faces, face_edge_indices, n_edges, waves, out=None):
+def assemble_rhs_rwg_sym(verts, faces, face_edge_indices, n_edges, waves, out=None, check_indices=True):
     """EFIE excitation [E, n_rhs] with the 7-point rule for plane waves [n_rhs, 9] float64."""
     _lib.check_tensor(verts, "verts", dtype=_FLOATS, ndim=2)
     dt, dev = verts.dtype, verts.device
     _lib.check_tensor(faces, "faces", dtype=torch.int32, device=dev, ndim=2)
     nf = faces.shape[0]
     check_face_range(faces, verts.shape[0])
-    _check_fei(face_edge_indices, nf, n_edges, dev)
+    if check_indices:
+        _check_fei(face_edge_indices, nf, n_edges, dev)
     waves = waves.to(device=dev, dtype=torch.float64).contiguous()
     if waves.dim() != 2 or waves.shape[1] != 9:
         raise ValueError("waves must be [n_rhs, 9]")

@@ -349,13 +349,27 @@ def shape_function(dim: int, order_type: int, r1: torch.Tensor, r2: torch.Tensor
     raise RuntimeError("We only accept 2D/3D for calculating shape function")
 
 
+def indices_outside(idx: torch.Tensor, limit: int) -> bool:
+    """Whether an index lies outside [0, limit): one kernel and one sync for contiguous int32 CUDA tensors."""
+    if idx.numel() == 0:
+        return False
+    if not (idx.is_cuda and idx.dtype == torch.int32 and idx.is_contiguous()):
+        lo, hi = torch.aminmax(idx)
+        return int(lo) < 0 or int(hi) >= limit
+    work = torch.empty(1, dtype=torch.int32, device=idx.device)
+    bad = ctypes.c_int32(0)
+    _lib.call("mb_index_range_i32", _lib.ptr(idx), idx.numel(), int(limit), _lib.ptr(work), ctypes.byref(bad),
+              _lib.stream_of(idx))
+    return bool(bad.value)
+
+
 def pack_matrix_tight(order_type: int, unpacked_matrix: torch.Tensor, verts: torch.Tensor,
                       faces: torch.Tensor) -> torch.Tensor:
     """[F, F, nphi, nphi] -> [V, V]: packed[faces[fy,a], faces[fx,b]] += M[fy, fx, a, b]."""
     n_verts = verts.shape[-2]
     faces = _lib.check_tensor(faces.contiguous(), "faces", dtype=torch.int32, ndim=2)
     nf = faces.shape[0]
-    if nf and (int(faces.min()) < 0 or int(faces.max()) >= n_verts):
+    if nf and indices_outside(faces, n_verts):
         raise ValueError(f"faces reference vertex ids outside [0, {n_verts})")
     m = unpacked_matrix.contiguous()
     if m.shape[:2] != (nf, nf) or m.shape[2] != m.shape[3] or m.shape[2] not in (1, 3):

@@ -71,6 +71,77 @@ __device__ __forceinline__ void potential_integrals(const V3<R>& x, const V3<R> 
     *Iv = sv - (d * s1) * n;
 }
 
+// The same integrals at many points of one triangle, in FP64.  The pipe's 2 lanes a clock and SM bound them, so
+// they take few instructions: the edges' directions once per triangle; a corner's distance once (it is R+ of one
+// edge and R- of the next); sum (beta+ - beta-) as the solid angle, which is one arc tangent of
+//   2 area |d| / (r0 r1 r2 + (r0.r1) r2 + (r1.r2) r0 + (r2.r0) r1),  r_i.r_j = (r_i^2 + r_j^2 - L_ij^2) / 2
+// instead of six; roots and quotients from the hardware's approximations (about 2^-20) by one third-order step.
+struct FaceEdges {
+    V3<double> n, l[3], u[3];
+    double len[3], area2;  // edge lengths, twice the area
+};
+
+__device__ __forceinline__ double rsqrt_step(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double t = fma(-(x * y), y, 1.0);
+    return fma(t * y, fma(t, 0.375, 0.5), y);
+}
+__device__ __forceinline__ double sqrt_step(double x) { return x > 0.0 ? x * rsqrt_step(x) : sqrt(x); }
+__device__ __forceinline__ double quotient_step(double a, double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    const double e = fma(-b, y, 1.0);
+    y = fma(y, fma(e, e, e), y);
+    const double q = a * y;
+    return fma(fma(-b, q, a), y, q);
+}
+
+__device__ __forceinline__ FaceEdges face_edges(const V3<double> P[3]) {
+    FaceEdges f;
+    f.n = cross(P[1] - P[0], P[2] - P[1]);
+    f.area2 = sqrt(dot(f.n, f.n));
+    f.n = (1.0 / f.area2) * f.n;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const V3<double> e = P[(i + 1) % 3] - P[i];
+        f.len[i] = sqrt(dot(e, e));
+        f.l[i] = (1.0 / f.len[i]) * e;
+        f.u[i] = cross(f.l[i], f.n);
+    }
+    return f;
+}
+
+__device__ __forceinline__ void potential_integrals(const V3<double>& x, const V3<double> P[3], const FaceEdges& f,
+                                                    double* I1, V3<double>* Iv) {
+    const double d = dot(x - P[0], f.n), ad = fabs(d);
+    double lm[3], p0[3], q0[3], r2[3], r[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const V3<double> v = P[i] - x;
+        lm[i] = dot(v, f.l[i]);
+        p0[i] = dot(v, f.u[i]);
+        q0[i] = fma(p0[i], p0[i], d * d);
+        r2[i] = fma(lm[i], lm[i], q0[i]);
+        r[i] = sqrt_step(r2[i]);
+    }
+    double s1 = 0.0, den = r[0] * r[1] * r[2];
+    V3<double> sv = v3<double>(0, 0, 0);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const int j = (i + 1) % 3;
+        const double lp = lm[i] + f.len[i], rp = r[j], rm = r[i];
+        const bool ahead = (lm[i] >= 0.0 || lp >= 0.0) && rm + lm[i] > 0.0;
+        const double lg = log(quotient_step(ahead ? rp + lp : rm - lm[i], ahead ? rm + lm[i] : rp - lp));
+        s1 = fma(p0[i], lg, s1);
+        sv = sv + (0.5 * fma(q0[i], lg, fma(lp, rp, -lm[i] * rm))) * f.u[i];
+        den = fma(0.5 * (r2[i] + r2[j] - f.len[i] * f.len[i]), r[(i + 2) % 3], den);
+    }
+    s1 -= 2.0 * ad * atan2(f.area2 * ad, den);
+    *I1 = s1;
+    *Iv = sv - (d * s1) * f.n;
+}
+
 // Double-layer integrals: *omega = int_T n.(y - x)/R^3 dS (signed solid angle) and
 // *J = int_T (rho_y - rho)/R^3 dS (in-plane vector); *d = n.(x - P0).  When |d| is below
 // dtol the point lies in the triangle's plane, where n.(x - y) vanishes: omega = 0 (the

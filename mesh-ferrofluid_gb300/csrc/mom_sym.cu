@@ -405,8 +405,20 @@ __global__ void __launch_bounds__(128) mom_sym_regular_kernel(const T* __restric
 }
 
 // ---------------------------------------------------------------------------------------
-// pairs sharing a vertex: FP64 with the singular part in closed form; one thread per pair
+// pairs sharing a vertex: FP64 with the singular part in closed form; one thread per pair.
+// Bound: the FP64 pipe.  For complex64 the closed form takes one arc tangent and three roots a point
+// instead of six each, its edges' directions and the source points (two floats each) once a
+// pair (closed_form.cuh): 266 240 pairs 3.10 -> 1.56 ms, 66 560 pairs 0.90 -> 0.45 ms, the entries'
+// errors against complex128 the same (1.3e-7 .. 2.4e-7 rms).  complex128 keeps the edge-by-edge form.
 // ---------------------------------------------------------------------------------------
+// a rule point, rounded alike for both faces (a self pair's points coincide exactly)
+__device__ __forceinline__ V3<double> rule_point(int i, const V3<double> (&P)[3]) {
+    const double a = c_d7[i][0], b = c_d7[i][1], c = c_d7[i][2];
+    return v3<double>(__fma_rn(a, P[0].x, __fma_rn(b, P[1].x, __dmul_rn(c, P[2].x))),
+                      __fma_rn(a, P[0].y, __fma_rn(b, P[1].y, __dmul_rn(c, P[2].y))),
+                      __fma_rn(a, P[0].z, __fma_rn(b, P[1].z, __dmul_rn(c, P[2].z))));
+}
+
 template <typename T>
 __device__ __forceinline__ void sym_near_pair(const T* __restrict__ verts, const int32_t* __restrict__ faces,
                                               const int32_t* __restrict__ fei, int64_t n_edges, double k, int64_t p,
@@ -427,23 +439,39 @@ __device__ __forceinline__ void sym_near_pair(const T* __restrict__ verts, const
     double t0r = 0, t0i = 0, txyr = 0, txyi = 0;
     V3<double> txr = v3<double>(0, 0, 0), txi = v3<double>(0, 0, 0), tyr = v3<double>(0, 0, 0),
                tyi = v3<double>(0, 0, 0);
+    const float kf = (float)k;
+    V3<float> yh[7], yl[7];  // complex64 output: the source points from B0, in two floats each
+    float wq[7];
+    FaceEdges fe;
+    if constexpr (sizeof(T) == 4) {
+#pragma unroll
+        for (int j = 0; j < 7; ++j) {
+            const V3<double> y = rule_point(j, B) - B[0];
+            yh[j] = v3<float>((float)y.x, (float)y.y, (float)y.z);
+            yl[j] = v3<float>((float)(y.x - yh[j].x), (float)(y.y - yh[j].y), (float)(y.z - yh[j].z));
+            wq[j] = (float)(c_d7[j][3] * aq * inv4pi);
+        }
+        fe = face_edges(B);
+    }
+#pragma unroll 1
     for (int i = 0; i < 7; ++i) {
-        const V3<double> x = c_d7[i][0] * A[0] + c_d7[i][1] * A[1] + c_d7[i][2] * A[2];
+        const V3<double> x = rule_point(i, A);
         double g0r = 0, g0i = 0;
         V3<double> gyr = v3<double>(0, 0, 0), gyi = v3<double>(0, 0, 0);
         if constexpr (sizeof(T) == 4) {
-            // complex64 output: the smooth part (e^{-jkR} - 1) / (4 pi R) in FP32 (point
-            // differences taken in FP64, moments relative to B0), the singular 1/R part below
-            // in FP64 and closed form
-            const float kf = (float)k;
+            // complex64 output: the smooth part (e^{-jkR} - 1) / (4 pi R) in FP32 (point differences
+            // from two floats each, moments relative to B0), the singular 1/R part below in FP64
+            // and closed form
+            const V3<double> xd = x - B[0];
+            const V3<float> xh = v3<float>((float)xd.x, (float)xd.y, (float)xd.z);
+            const V3<float> xl = v3<float>((float)(xd.x - xh.x), (float)(xd.y - xh.y), (float)(xd.z - xh.z));
             float s0r = 0.f, s0i = 0.f, syr[3] = {0.f, 0.f, 0.f}, syi[3] = {0.f, 0.f, 0.f};
 #pragma unroll
             for (int j = 0; j < 7; ++j) {
-                const V3<double> y = c_d7[j][0] * B[0] + c_d7[j][1] * B[1] + c_d7[j][2] * B[2];
-                const V3<double> dd = x - y;
-                const float dx = (float)dd.x, dy = (float)dd.y, dz = (float)dd.z;
+                const float dx = (xh.x - yh[j].x) + (xl.x - yl[j].x), dy = (xh.y - yh[j].y) + (xl.y - yl[j].y),
+                            dz = (xh.z - yh[j].z) + (xl.z - yl[j].z);
                 const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-                const float wj = (float)(c_d7[j][3] * aq * inv4pi);
+                const float wj = wq[j];
                 float gr, gi;
                 if (r2 <= 0.f) {  // coincident points of the self pair: limit of the smooth part
                     gr = 0.f;
@@ -457,13 +485,13 @@ __device__ __forceinline__ void sym_near_pair(const T* __restrict__ verts, const
                     gr = -2.f * sh * sh * rinv * wj;  // (cos kR - 1) / R without cancellation
                     gi = -sn * rinv * wj;
                 }
-                const float yl[3] = {(float)(y.x - B[0].x), (float)(y.y - B[0].y), (float)(y.z - B[0].z)};
                 s0r += gr;
                 s0i += gi;
+                const float yj[3] = {yh[j].x, yh[j].y, yh[j].z};
 #pragma unroll
                 for (int a = 0; a < 3; ++a) {
-                    syr[a] = fmaf(gr, yl[a], syr[a]);
-                    syi[a] = fmaf(gi, yl[a], syi[a]);
+                    syr[a] = fmaf(gr, yj[a], syr[a]);
+                    syi[a] = fmaf(gi, yj[a], syi[a]);
                 }
             }
             g0r = s0r;
@@ -472,7 +500,7 @@ __device__ __forceinline__ void sym_near_pair(const T* __restrict__ verts, const
             gyi = v3<double>(syi[0], syi[1], syi[2]) + g0i * B[0];
         } else {
             for (int j = 0; j < 7; ++j) {
-                const V3<double> y = c_d7[j][0] * B[0] + c_d7[j][1] * B[1] + c_d7[j][2] * B[2];
+                const V3<double> y = rule_point(j, B);
                 const V3<double> dd = x - y;
                 const double R = sqrt(dot(dd, dd));
                 double gr, gi;
@@ -495,7 +523,8 @@ __device__ __forceinline__ void sym_near_pair(const T* __restrict__ verts, const
         }
         double I1;
         V3<double> Iv;
-        potential_integrals(x, B, &I1, &Iv);
+        if constexpr (sizeof(T) == 4) potential_integrals(x, B, fe, &I1, &Iv);
+        else potential_integrals(x, B, &I1, &Iv);
         g0r += inv4pi * I1;
         gyr = gyr + inv4pi * (Iv + I1 * x);
         const double wi = c_d7[i][3] * ap;

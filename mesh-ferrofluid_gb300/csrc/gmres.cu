@@ -1273,9 +1273,16 @@ __global__ void __launch_bounds__(32) pg_givens_kernel(PgState* st, double2* g, 
             col[i] = make_double2(t1.x + t2.x, t1.y + t2.y);
             col[i + 1] = make_double2(u2.x - u1.x, u2.y - u1.y);
         }
-        const double rr = hypot(sqrt(cabs2(col[j])), hn);
+        // one reciprocal root in place of hypot, a root and three quotients, unless the squares leave the range
+        const double s2 = cabs2(col[j]) + hn * hn;
+        const bool plain = s2 > 1e-280 && s2 < 1e280;
+        const double ri = plain ? rsqrt(s2) : 0.0;
+        const double rr = plain ? s2 * ri : hypot(sqrt(cabs2(col[j])), hn);
         double2 c, sv;
-        if (rr == 0.0) {
+        if (plain) {
+            c = make_double2(col[j].x * ri, col[j].y * ri);
+            sv = make_double2(hn * ri, 0.0);
+        } else if (rr == 0.0) {
             c = make_double2(1.0, 0.0);
             sv = make_double2(0.0, 0.0);
         } else {
@@ -1382,8 +1389,8 @@ static void pg_steps_t(const PgMatrix& A, int64_t n, const int32_t* cols, const 
                        unsigned* cnt, cudaStream_t s) {
     const unsigned vb = (unsigned)((n + 255) / 256), rb = (unsigned)((n + 7) / 8);
     const int sblk = (int)std::min<int64_t>((n + 127) / 128, kPgMaxBlocks);
-    // dot-product chunks: at least 1024 elements, at most kPgMaxBlocks chunks
-    int64_t chunk = 1024;
+    // dot-product chunks: at least 256 elements (8 a lane), at most kPgMaxBlocks chunks
+    int64_t chunk = 256;
     while ((n + chunk - 1) / chunk > kPgMaxBlocks) chunk *= 2;
     const unsigned nchunk = (unsigned)((n + chunk - 1) / chunk);
     const dim3 dgrid(nchunk, (unsigned)((m + 7) / 8));

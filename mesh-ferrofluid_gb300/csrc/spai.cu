@@ -65,8 +65,26 @@ __device__ __forceinline__ int find_mesh(const int64_t* d, int n_mesh, int col, 
     return lo;
 }
 
+// ranges[2 f], [2 f + 1]: the near-pair rows of face f (pairs sorted by first face; ranges zeroed).  Searched in
+// the column kernel instead, a range is 32 dependent fetches, twice in each block's way.
+__global__ void __launch_bounds__(256) pair_ranges_kernel(const int32_t* __restrict__ pairs, int64_t n,
+                                                          int64_t n_faces, int32_t* __restrict__ ranges) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int32_t f = __ldg(pairs + 2 * i);
+    if (f < 0 || f >= n_faces) return;
+    if (i == 0 || __ldg(pairs + 2 * i - 2) != f) ranges[2 * f] = (int32_t)i;
+    if (i == n - 1 || __ldg(pairs + 2 * i + 2) != f) ranges[2 * f + 1] = (int32_t)(i + 1);
+}
+
 // [begin, end) of the near-pair rows whose first face is f (pairs sorted by first face)
-__device__ __forceinline__ void pair_range(const int32_t* pairs, int64_t n, int32_t f, int64_t* b, int64_t* e) {
+__device__ __forceinline__ void pair_range(const int32_t* pairs, int64_t n, const int32_t* ranges, int32_t f,
+                                           int64_t* b, int64_t* e) {
+    if (ranges) {
+        *b = __ldg(ranges + 2 * (int64_t)f);
+        *e = max((int)*b, __ldg(ranges + 2 * (int64_t)f + 1));
+        return;
+    }
     int64_t lo = 0, hi = n;
     while (lo < hi) {
         const int64_t mid = (lo + hi) >> 1;
@@ -188,8 +206,8 @@ __device__ __forceinline__ float warp_sumf(float v) {
 __global__ void __launch_bounds__(kSpaiThreads) spai_column_kernel(
     const float* __restrict__ verts, const int32_t* __restrict__ faces, const int32_t* __restrict__ fei,
     const int32_t* __restrict__ edge_fe, const int32_t* __restrict__ pairs, int64_t n_pairs,
-    const int64_t* __restrict__ desc, int n_mesh, const float* __restrict__ z, int32_t* __restrict__ out_cols,
-    float2* __restrict__ out_vals, int* __restrict__ status) {
+    const int32_t* __restrict__ ranges, const int64_t* __restrict__ desc, int n_mesh, const float* __restrict__ z,
+    int32_t* __restrict__ out_cols, float2* __restrict__ out_vals, int* __restrict__ status) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SpaiSmem& S = *reinterpret_cast<SpaiSmem*>(smem_raw);
     const int64_t g = blockIdx.x;
@@ -218,7 +236,7 @@ __global__ void __launch_bounds__(kSpaiThreads) spai_column_kernel(
     if (tid < 2) {
         const int32_t r = tid == 0 ? ra : rb;
         int64_t b = 0, e = 0;
-        if (r >= 0) pair_range(pairs, n_pairs, r / 3, &b, &e);
+        if (r >= 0) pair_range(pairs, n_pairs, ranges, r / 3, &b, &e);
         S.s1_off[tid] = (int)(e - b);
         S.s1_off[2 + tid] = (int)b;  // scratch: range starts
     }
@@ -262,7 +280,7 @@ __global__ void __launch_bounds__(kSpaiThreads) spai_column_kernel(
     // ---- 1c. S2 = faces sharing a vertex with a face of S1 ---------------------------------
     for (int i = tid; i < n1; i += kSpaiThreads) {
         int64_t b, e;
-        pair_range(pairs, n_pairs, S.s1[i], &b, &e);
+        pair_range(pairs, n_pairs, ranges, S.s1[i], &b, &e);
         S.s1_off[i + 1] = (int)(e - b);
         S.cand[kSpaiCand - 1 - i] = (int)b;  // range starts kept at the buffer's end
     }
@@ -595,7 +613,14 @@ int spai_build(const float* verts, const int32_t* faces, const int32_t* fei, con
     edge_fe_kernel<<<(unsigned)((total_faces + 255) / 256), 256, 0, s>>>(fei, desc, n_mesh, total_faces, w.ef,
                                                                        w.status);
     edge_fe_order_kernel<<<(unsigned)((total_edges + 255) / 256), 256, 0, s>>>(total_edges, w.ef, w.status);
-    spai_column_kernel<<<(unsigned)total_edges, kSpaiThreads, smem, s>>>(verts, faces, fei, w.ef, pairs, n_pairs, desc,
+    // the ranges live in m_cols until spai_rows_kernel writes it (48 entries an edge; two a face)
+    int32_t* ranges = 2 * total_faces <= kSpaiWidth * total_edges ? m_cols : nullptr;
+    if (ranges) {
+        cudaMemsetAsync(ranges, 0, sizeof(int32_t) * 2 * (size_t)total_faces, s);
+        pair_ranges_kernel<<<(unsigned)((n_pairs + 255) / 256), 256, 0, s>>>(pairs, n_pairs, total_faces, ranges);
+    }
+    spai_column_kernel<<<(unsigned)total_edges, kSpaiThreads, smem, s>>>(verts, faces, fei, w.ef, pairs, n_pairs,
+                                                                        ranges, desc,
                                                                         n_mesh, z, w.ccols, w.cvals, w.status);
     const int64_t nt = total_edges * kSpaiWidth;
     spai_rows_kernel<<<(unsigned)((nt + 255) / 256), 256, 0, s>>>(desc, n_mesh, total_edges, w.ccols, w.cvals,

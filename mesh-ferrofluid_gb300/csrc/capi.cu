@@ -95,7 +95,7 @@ int index_range(const int32_t* idx, int64_t count, int64_t limit, int32_t* work,
 int launch_edge_rows(const int32_t* fei, int64_t nf, int64_t n_edges, int32_t* er, cudaStream_t s);
 bool mom_tier_rule(int nx, int ny);
 int launch_mom_sym_pairs(const float* verts, const int32_t* faces, const int32_t* fei, int64_t nf, int64_t n_edges, double k,
-                         float* rec, float* z, cudaStream_t s);
+                         bool overwrite, float* rec, float* z, cudaStream_t s);
 int launch_mom_tiers(const float* verts, const int32_t* faces, int64_t nf, const float* areas, const float* normals,
                      const int32_t* fei, int64_t n_edges, const float* gpx, const float* gwx, int nx, const float* gpy,
                      const float* gwy, int ny, double k, float* rec, float* z, cudaStream_t s);
@@ -317,16 +317,21 @@ int mb_index_range_i32(const int32_t* indices, int64_t count, int64_t limit, int
 int64_t mb_mom_tiers_workspace_bytes(int64_t n_faces) { return n_faces > 0 ? 128 * n_faces : 0; }
 
 int mb_mom_sym_zmat_rwg_pairs_c64(const float* verts, int64_t n_verts, const int32_t* faces, int64_t n_faces,
-                                  const int32_t* face_edge_indices, int64_t n_edges, double wavenumber, void* workspace,
-                                  int64_t workspace_bytes, float* z, void* stream) {
+                                  const int32_t* face_edge_indices, int64_t n_edges, double wavenumber, int overwrite,
+                                  void* workspace, int64_t workspace_bytes, float* z, void* stream) {
     (void)n_verts;
     MB_REQUIRE(n_faces >= 0 && n_edges >= 0, "bad sizes");
-    if (n_faces == 0) return MB_OK;
+    if (n_faces == 0) {
+        if (!overwrite || n_edges == 0) return MB_OK;
+        MB_REQUIRE(z, "null pointer argument");
+        const cudaError_t e = cudaMemsetAsync(z, 0, (size_t)n_edges * n_edges * 8, as_stream(stream));
+        return e == cudaSuccess ? MB_OK : set_error(MB_ERR_CUDA, "%s", cudaGetErrorString(e));
+    }
     MB_REQUIRE(verts && faces && face_edge_indices && workspace && z, "null pointer argument");
     MB_REQUIRE(wavenumber > 0, "wavenumber must be > 0");
     MB_REQUIRE(workspace_bytes >= mb_mom_tiers_workspace_bytes(n_faces) && (uintptr_t)workspace % 16 == 0,
                "workspace too small or not 16-byte aligned");
-    return launch_mom_sym_pairs(verts, faces, face_edge_indices, n_faces, n_edges, wavenumber,
+    return launch_mom_sym_pairs(verts, faces, face_edge_indices, n_faces, n_edges, wavenumber, overwrite != 0,
                                 static_cast<float*>(workspace), z, as_stream(stream));
 }
 

@@ -675,14 +675,16 @@ __global__ void __launch_bounds__(128, NX <= 4 ? 4 : 3) close_pairs_kernel(const
 // ---------------------------------------------------------------------------------------
 // the 7-point-rule EFIE (mom_sym.cu) on separated pairs, in the same arithmetic: the rule's points
 // are the centroid and two orbits s A_a, so all 49 evaluations come from the pair's scalar products.
-// The operator is symmetric and both faces carry the same rule: a pair is evaluated once, p < q,
-// and added at (m, n) and (n, m).  The terms of kEdgeRows test faces are summed per thread in shared
-// memory by distinct test edge (8 faces of the sphere have 16 to 18 of 24), so that about 2 edges
+// The operator is symmetric and both faces carry the same rule: a pair is evaluated once, p < q, and
+// its entries belong at (m, n) and (n, m).  The terms of kEdgeRows test faces are summed per thread in
+// shared memory by distinct test edge (8 faces of the sphere have 16 to 18 of 24), so that about 2 edges
 // x 3 of a face remain of 9 reductions per ordered pair: a reduction costs a cycle of its SM, which
-// with 9 bounds the whole at 13 ms for 20480 faces.
-// Measured (GB300): 20480 faces 22.35 -> 13.66 ms + 0.9 ms for the pairs left, 5120 faces 1.44 -> 0.77 + 0.17 ms;
-// (rows, slots, blocks per SM) 8/16/4 best of 4/8/5 15.4, 8/16/3 14.1, 12/22/3 14.1, 16/28/2 14.8 ms.  Bound: FMA pipe and
-// the reductions together.  Entry errors against 64 bits 0.45 .. 0.65 of the former kernel's beyond 4 edges.
+// with 9 bounds the whole at 13 ms for 20480 faces.  Into a matrix of its own (not one that is added
+// to) the kernel sums above the diagonal only, half the reductions, and mirror_kernel copies.
+// Measured (GB300), 20480 faces: 22.35 (every ordered pair, row by row) -> 13.66 (both sides) -> 10.05 ms + 1.48 ms for
+// the mirror, 0.49 instead of 0.96 for the zeros, 0.9 ms for the pairs left.  (rows, slots, blocks per SM), both
+// sides: 8/16/4 best of 4/8/5 15.4, 8/16/3 14.1, 12/22/3 14.1, 16/28/2 14.8 ms.  Bound: FMA pipe.  Entry errors
+// against 64 bits 0.45 .. 0.65 of the row kernel's beyond 4 edges.
 // Pairs with |D| >= 2 (rho_p + rho_q) and k (rho_p + rho_q) <= 0.6 (the phases' polynomials); the
 // others are left to mom_sym_regular_rows_kernel, which applies the same test.
 // ---------------------------------------------------------------------------------------
@@ -694,6 +696,35 @@ struct EdgeSlots {
     uint8_t slot[4 * kEdgeRows];
 };
 
+// e at (m, n) and (n, m); UPPER: at the one of them above the diagonal, for mirror_kernel to copy
+template <bool UPPER>
+__device__ __forceinline__ void add_both(float2* __restrict__ z, int64_t m, int64_t n, int64_t n_edges, float2 e) {
+    atomicAdd(z + (UPPER ? min(m, n) : m) * n_edges + (UPPER ? max(m, n) : n), e);
+    if (!UPPER || m == n) atomicAdd(z + n * n_edges + m, e);
+}
+
+// Zeros from the diagonal's 32 x 32 tiles to the right, a row per block.
+__global__ void __launch_bounds__(256) zero_upper_kernel(float2* __restrict__ z, int64_t n) {
+    float2* row = z + (int64_t)blockIdx.x * n;
+    for (int64_t c = (int64_t)blockIdx.x / 32 * 32 + threadIdx.x; c < n; c += 256) row[c] = make_float2(0.f, 0.f);
+}
+
+// z[n, m] = z[m, n] for m < n, a 32 x 32 tile above the diagonal per block.  Tile rows y and t - 1 - y together
+// have t + 1 tiles: the grid is (t + 1) x ceil(t / 2).
+__global__ void __launch_bounds__(256) mirror_kernel(float2* __restrict__ z, int64_t n, int t) {
+    __shared__ float2 s[32][33];
+    const int x = blockIdx.x, y = blockIdx.y;
+    if (x <= y && 2 * y == t - 1) return;  // the middle row pairs with itself
+    const int64_t i0 = 32 * (int64_t)(x > y ? y : t - 1 - y), j0 = 32 * (int64_t)(x > y ? x - 1 : t - 1 - x);
+    const int c = threadIdx.x & 31;
+    for (int r = threadIdx.x >> 5; r < 32; r += 8)
+        if (i0 + r < n && j0 + c < n) s[r][c] = z[(i0 + r) * n + j0 + c];
+    __syncthreads();
+    for (int r = threadIdx.x >> 5; r < 32; r += 8)
+        if (j0 + r < n && i0 + c < n && j0 + r > i0 + c) z[(j0 + r) * n + i0 + c] = s[c][r];
+}
+
+template <bool UPPER>
 __global__ void __launch_bounds__(128, 4)
     sym_pairs_kernel(const float* __restrict__ rec, int64_t nf, int64_t n_edges, double kd, float* __restrict__ z) {
     constexpr float s1 = (float)(1.0 - 3.0 * 0.10128650732345634), s2 = (float)(1.0 - 3.0 * 0.47014206410511509);
@@ -853,8 +884,7 @@ __global__ void __launch_bounds__(128, 4)
                     *d = add2(*d, e);
                 } else {
                     const int64_t m = s_e.id[3 * i + a], n = col[b];
-                    atomicAdd(z2 + m * n_edges + n, e);
-                    atomicAdd(z2 + n * n_edges + m, e);
+                    add_both<UPPER>(z2, m, n, n_edges, e);
                 }
             }
         }
@@ -865,9 +895,7 @@ __global__ void __launch_bounds__(128, 4)
         for (int b = 0; b < 3; ++b) {
             const float2 e = mine[(3 * u + b) * 128];
             if (e.x != 0.f || e.y != 0.f) {
-                const int64_t n = col[b];
-                atomicAdd(z2 + m * n_edges + n, e);
-                atomicAdd(z2 + n * n_edges + m, e);
+                add_both<UPPER>(z2, m, col[b], n_edges, e);
             }
         }
     }
@@ -944,15 +972,24 @@ int launch_mom_sym_rest(const float* verts, const int32_t* faces, const int32_t*
                         const float* rec, float* z, cudaStream_t s);
 
 int launch_mom_sym_pairs(const float* verts, const int32_t* faces, const int32_t* fei, int64_t nf, int64_t n_edges, double k,
-                         float* rec, float* z, cudaStream_t s) {
+                         bool overwrite, float* rec, float* z, cudaStream_t s) {
     if (nf <= 0) return MB_OK;
     if (int rc = tier_records(verts, faces, nullptr, fei, nf, nullptr, nullptr, 0, nullptr, nullptr, 0, rec, s)) return rc;
     const int64_t gx = (nf + kEdgeRows - 1) / kEdgeRows, gy = (nf + 127) / 128;
     if (gx > 0x7fffffffLL || gy > 65535) return set_error(MB_ERR_SIZE, "mesh too large for one launch");
-    const cudaError_t e = cudaFuncSetAttribute(sym_pairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kEdgeSumBytes);
+    // a matrix that is not added to is summed above the diagonal only, half the reductions, and mirrored
+    const auto kernel = overwrite ? sym_pairs_kernel<true> : sym_pairs_kernel<false>;
+    const int64_t tiles = (n_edges + 31) / 32;
+    if (overwrite && (n_edges > 0x7fffffffLL || (tiles + 1) / 2 > 65535))
+        return set_error(MB_ERR_SIZE, "matrix too large for one launch");
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kEdgeSumBytes);
     if (e != cudaSuccess) return set_error(MB_ERR_CUDA, "%s", cudaGetErrorString(e));
+    float2* z2 = reinterpret_cast<float2*>(z);
+    if (overwrite && n_edges > 0) zero_upper_kernel<<<(unsigned)n_edges, 256, 0, s>>>(z2, n_edges);
     // test groups fastest: blocks in flight share the rows of one source tile for the transposed terms
-    sym_pairs_kernel<<<dim3((unsigned)gx, (unsigned)gy), 128, kEdgeSumBytes, s>>>(rec, nf, n_edges, k, z);
+    kernel<<<dim3((unsigned)gx, (unsigned)gy), 128, kEdgeSumBytes, s>>>(rec, nf, n_edges, k, z);
+    if (overwrite && n_edges > 0)
+        mirror_kernel<<<dim3((unsigned)(tiles + 1), (unsigned)((tiles + 1) / 2)), 256, 0, s>>>(z2, n_edges, (int)tiles);
     if (int rc = check_launch("mom sym pairs")) return rc;
     return launch_mom_sym_rest(verts, faces, fei, n_edges, k, nf, rec, z, s);
 }

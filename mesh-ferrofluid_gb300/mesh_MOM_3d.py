@@ -388,8 +388,9 @@ def assemble_Z_rwg_sym(verts, faces, face_edge_indices, n_edges, wavenumber, out
     if check_indices:
         _check_fei(face_edge_indices, nf, n_edges, dev)
     cdt = torch.complex64 if dt == torch.float32 else torch.complex128
+    fresh = out is None and out_host is None and dt == torch.float32 and faces_range is None  # written whole below
     if out is None:
-        out = torch.zeros((n_edges, n_edges), dtype=cdt, device=dev)
+        out = (torch.empty if fresh else torch.zeros)((n_edges, n_edges), dtype=cdt, device=dev)
     else:
         _lib.check_tensor(out, "out", dtype=cdt, device=dev, shape=(n_edges, n_edges))
     st = _lib.stream_of(verts)
@@ -409,7 +410,8 @@ def assemble_Z_rwg_sym(verts, faces, face_edge_indices, n_edges, wavenumber, out
     if dt == torch.float32 and faces_range is None:
         ws = torch.empty(max(1, int(_lib.load().mb_mom_tiers_workspace_bytes(nf))), dtype=torch.uint8, device=dev)
         _lib.call("mb_mom_sym_zmat_rwg_pairs_c64", _lib.ptr(verts), verts.shape[0], _lib.ptr(faces), nf,
-                  _lib.ptr(face_edge_indices), n_edges, float(wavenumber), _lib.ptr(ws), ws.numel(), _lib.ptr(out), st)
+                  _lib.ptr(face_edge_indices), n_edges, float(wavenumber), int(fresh), _lib.ptr(ws), ws.numel(),
+                  _lib.ptr(out), st)
     else:
         f0, f1 = (0, nf) if faces_range is None else faces_range
         _lib.call(f"mb_mom_sym_zmat_rwg_{_lib.csfx(dt)}", _lib.ptr(verts), verts.shape[0], _lib.ptr(faces), nf,

@@ -47,3 +47,23 @@ def test_pairs_equal_rows_and_float64(pkg, kind, k):
     assert _rel(Z, ref) <= 1.1 * _rel(rows, ref)
     again = ops.assemble_Z_rwg_sym(v, f, fei, n, k, out=Z.clone())  # accumulates
     assert _rel(again, 2 * Z) < TOL
+
+
+# a part of a 32 x 32 tile, one tile, an even and an odd number of tile rows, a partial last one
+@pytest.mark.parametrize("n_faces", [0, 1, 10, 20, 21, 42, 64, 107])
+def test_fresh_matrix_equals_one_added_to_zeros(pkg, n_faces):
+    """A matrix that is not passed in is summed above the diagonal and mirrored; one that is passed in is added to
+    on both sides: the same additions in another order (a few 6e-8 of an entry's terms)."""
+    ops = pkg.mesh_MOM_3d
+    v, f = pkg.meshes.icosphere(2)
+    v = torch.tensor(v, dtype=torch.float32, device="cuda")
+    f = torch.tensor(f[:n_faces], dtype=torch.int32, device="cuda").reshape(-1, 3)
+    fei = pkg.utils.get_edge_unique(v, f)[1] if n_faces else torch.zeros((0, 3), dtype=torch.int32, device="cuda")
+    n = int(fei.max()) + 1 if n_faces else 5
+    if n_faces == 107:  # edges that far faces share: terms on the diagonal
+        fei = fei % (n - 40)
+        n -= 40
+    torch.full((n, n), float("nan"), device="cuda", dtype=torch.complex64)  # what the allocator may hand out
+    Z = ops.assemble_Z_rwg_sym(v, f, fei, n, 0.4)
+    ref = ops.assemble_Z_rwg_sym(v, f, fei, n, 0.4, out=torch.zeros((n, n), dtype=torch.complex64, device="cuda"))
+    assert torch.linalg.norm(Z - ref) <= 5e-7 * torch.linalg.norm(ref)

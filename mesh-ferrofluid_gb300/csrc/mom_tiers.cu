@@ -682,7 +682,7 @@ __global__ void __launch_bounds__(128, NX <= 4 ? 4 : 3) close_pairs_kernel(const
 // with 9 bounds the whole at 13 ms for 20480 faces.  Into a matrix of its own (not one that is added
 // to) the kernel sums above the diagonal only, half the reductions, and mirror_kernel copies.
 // Measured (GB300), 20480 faces: 22.35 (every ordered pair, row by row) -> 13.66 (both sides) -> 10.05 ms + 1.48 ms for
-// the mirror, 0.49 instead of 0.96 for the zeros, 0.9 ms for the pairs left.  (rows, slots, blocks per SM), both
+// the mirror, 0.49 instead of 0.96 for the zeros, 0.5 ms for the pairs left.  (rows, slots, blocks per SM), both
 // sides: 8/16/4 best of 4/8/5 15.4, 8/16/3 14.1, 12/22/3 14.1, 16/28/2 14.8 ms.  Bound: FMA pipe.  Entry errors
 // against 64 bits 0.45 .. 0.65 of the row kernel's beyond 4 edges.
 // Pairs with |D| >= 2 (rho_p + rho_q) and k (rho_p + rho_q) <= 0.6 (the phases' polynomials); the

@@ -988,8 +988,7 @@ static int pack_pairs(const double*, const double*, const int32_t*, int64_t, int
 static int pack_pairs(const float* m_r, const float* m_i, const int32_t* faces, int64_t nf, int64_t nv, int order,
                       float* packed, cudaStream_t stream) {
     const int64_t gx = (nf + kPairThreads - 1) / kPairThreads;
-    // fewer test faces per block where all of them would leave under two waves of 760 blocks
-    const int per = (int)(nf * gx / 1520 >= kPairRows ? kPairRows : nf * gx / 1520 >= 1 ? nf * gx / 1520 : 1);
+    const int per = pair_rows(nf, gx);
     const int64_t gy = (nf + per - 1) / per;
     if (m_i != nullptr || order != 1 || gy > 65535) return 0;
     pack_pairs_kernel<<<dim3((unsigned)gx, (unsigned)gy), kPairThreads, kPackSmem, stream>>>(m_r, faces, nf, nv, per,

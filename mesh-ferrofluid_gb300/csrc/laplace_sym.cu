@@ -782,8 +782,7 @@ static int launch_sym_pairs(const double* verts, const int32_t* faces, int64_t n
 static int launch_sym_pairs(const float* verts, const int32_t* faces, int64_t nf, int64_t nv, int op, int64_t row_begin,
                             int64_t row_end, float* packed, cudaStream_t s) {
     const int64_t gx = (nf + kPairThreads - 1) / kPairThreads, rows = row_end - row_begin;
-    // fewer test faces per block where all of them would leave under two waves of 760 blocks
-    const int per = (int)std::max<int64_t>(1, std::min<int64_t>(kPairRows, rows * gx / 1520));
+    const int per = pair_rows(rows, gx);
     const int64_t gy = (rows + per - 1) / per;
     if (gx > 0x7fffffffLL || gy > 65535) return set_error(MB_ERR_SIZE, "mesh too large for one launch");
     auto go = [&](auto kernel) -> int {

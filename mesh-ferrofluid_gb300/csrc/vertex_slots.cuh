@@ -21,6 +21,25 @@ constexpr int kPairVerts = 20;  // distinct vertices with a place; terms of the 
 constexpr int kPairThreads = 128;
 constexpr int kPairSumBytes = 3 * kPairVerts * kPairThreads * (int)sizeof(float);
 
+// Test faces per block (host) for `rows` test faces and gx blocks of source faces.  An SM's time is that of its share
+// of the blocks, each worth its faces and about 0.6 more for its start; fewer than five blocks an SM leave it waiting
+// (676 faces: 8 a block 35 us, 5 27.5, 2 28.7).  Among those within 1 % the most faces: fewer reductions.
+inline int pair_rows(int64_t rows, int64_t gx) {
+    constexpr int64_t kSms = 152;
+    int best = 1;
+    double cost = 0.0;
+    for (int per = 1; per <= kPairRows; ++per) {
+        const int64_t blocks = (rows + per - 1) / per * gx;
+        if (per > 1 && blocks < 5 * kSms) break;
+        const double c = (double)((blocks + kSms - 1) / kSms) * (per + 0.6);
+        if (per == 1 || c <= 1.01 * cost) {
+            best = per;
+            cost = per == 1 || c < cost ? c : cost;
+        }
+    }
+    return best;
+}
+
 struct VertexSlots {
     int id[3 * kPairRows];        // vertex of each corner
     int first[3 * kPairRows];     // 1 at a vertex's first corner
@@ -32,6 +51,12 @@ struct VertexSlots {
 // before.  At most 48 corners: the searches are short.
 __device__ __forceinline__ void find_slots(VertexSlots& s, int np) {
     const int t = threadIdx.x, n = 3 * np;
+    if (np == 1) {  // nothing to share: its terms are reduced directly
+        if (t < 3) s.slot[t] = 255;
+        if (t == 0) s.n = 0;
+        __syncthreads();
+        return;
+    }
     __syncthreads();
     int first = 0;
     if (t < n) {

@@ -1303,7 +1303,7 @@ def main_lapmixed(args, rank, world, local_rank):
                              "schur_solve_blocks": t_schur,
                              "not_on_the_path": {"V_panels": t_vp, "pack_V_panels": t_pack,
                                                  "lu_solve_block_system": t_lu}},
-            "roofline": {"kernel": "lap_sym_tight_kernel<float, 1> + lap_sym_near_kernel (packed V)",
+            "roofline": {"kernel": "lap_sym_pairs_kernel<1> + lap_sym_near_kernel (packed V)",
                          "bound": "fp32" if dts == "f32" else "fp64", "achieved": ach,
                          "peak": fp32_peak if dts == "f32" else R.FP64_NOMINAL_TFLOPS, "unit": "TFLOP/s",
                          "frac": ach / (fp32_peak if dts == "f32" else R.FP64_NOMINAL_TFLOPS),
@@ -2363,11 +2363,11 @@ def main():
 
     # roofline of the dominant kernel (assembly), per launch
     if sym:
-        evals = (pairs - n_near) * 49.0  # separated pairs in the FP32 kernel (near pairs: FP64)
+        evals = (pairs - n_near) / 2 * 49.0  # each separated pair once for both orders (near pairs: FP64)
         flop = evals * R.EFIE_FLOP_PER_EVAL
         mufu = evals * R.EFIE_MUFU_PER_EVAL
         per_eval = f"{R.EFIE_FLOP_PER_EVAL} FLOP + {R.EFIE_MUFU_PER_EVAL} MUFU per evaluation x 49 " \
-                   f"evaluations per separated pair x (F^2 - {n_near} near pairs); kernel time = both kernels"
+                   f"evaluations per unordered separated pair x (F^2 - {n_near} near pairs) / 2; kernel time = all kernels"
     else:
         evals = pairs * R.ref_rule_evals_per_pair(gq)
         flop = evals * R.CFIE_FLOP_PER_EVAL
@@ -2391,7 +2391,7 @@ def main():
             "mufu": {"achieved_gops": mufu / kern_avg_s / 1e9, "peak_gops": mufu_peak,
                      "frac": mufu / kern_avg_s / 1e9 / mufu_peak},
             "algorithmic": per_eval,
-            "kernel": ("mom_sym_regular_kernel + mom_sym_near_kernel" if sym else
+            "kernel": ("sym_pairs_kernel + mom_sym_regular_rows_kernel + mom_sym_near_kernel" if sym else
                        f"mom_ref_zmat_edge_kernel<{gq},{gq - 1}> (Z row by Z row)"),
             "kernel_ms": kern_avg_s * 1e3}
 
@@ -2399,7 +2399,7 @@ def main():
             "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_per_step,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32",
             "data": "synthetic", "config": config, "roofline": roof, "clocks": clocks.summary(),
-            "gpu_launches": args.steps * (2 if sym else 1)}
+            "gpu_launches": args.steps * (4 if sym else 1)}
 
     # time to a 1e-4 error in J, plain FP32 path vs the mixed-precision path (reported beside the
     # headline; both formulations on the same 30 720-unknown sphere for the default workload)

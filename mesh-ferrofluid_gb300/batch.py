@@ -7,8 +7,9 @@ of meshes of uneven size (and wavenumber) into one vertex / face array and runs
   ``formulation="efie_sym"`` (the 7-point-rule EFIE, pairs sharing a vertex in FP64) one
   launch of the separated-pair kernel and one of the near-pair kernel
   (``mb_mom_sym_zmat_batched_c64``); with ``formulation="cfie_ref"`` (the reference's EFIE +
-  MFIE operator and collapsed Gauss rule, gaussQR 4) one launch
-  (``mb_mom_ref_zmat_batched_c64``);
+  MFIE operator and collapsed Gauss rule, gaussQR 4) one call whose quadrature is sized by each pair's
+  separation (``mb_mom_ref_zmat_batched_tiers_c64``; other rule sizes
+  ``mb_mom_ref_zmat_batched_c64``);
 * the excitation of ``nc`` plane waves per mesh in one launch (``mb_mom_sym_rhs_batched_c64``)
   into a padded block [max E_i, n_mesh * nc];
 * GMRES on every (mesh, wave) column in lockstep with the block-diagonal product

@@ -681,7 +681,7 @@ __global__ void __launch_bounds__(128, NX <= 4 ? 4 : 3) close_pairs_kernel(const
 // x 3 of a face remain of 9 reductions per ordered pair: a reduction costs a cycle of its SM, which
 // with 9 bounds the whole at 13 ms for 20480 faces.  Into a matrix of its own (not one that is added
 // to) the kernel sums above the diagonal only, half the reductions, and mirror_kernel copies.
-// Measured (GB300), 20480 faces: 22.35 (every ordered pair, row by row) -> 13.66 (both sides) -> 10.05 ms + 1.48 ms for
+// Measured (GB300), 20480 faces: 22.35 (every ordered pair, row by row) -> 13.66 (both sides) -> 10.05 ms + 1.08 ms for
 // the mirror, 0.49 instead of 0.96 for the zeros, 0.5 ms for the pairs left.  (rows, slots, blocks per SM), both
 // sides: 8/16/4 best of 4/8/5 15.4, 8/16/3 14.1, 12/22/3 14.1, 16/28/2 14.8 ms.  Bound: FMA pipe.  Entry errors
 // against 64 bits 0.45 .. 0.65 of the row kernel's beyond 4 edges.
@@ -703,25 +703,36 @@ __device__ __forceinline__ void add_both(float2* __restrict__ z, int64_t m, int6
     if (!UPPER || m == n) atomicAdd(z + n * n_edges + m, e);
 }
 
-// Zeros from the diagonal's 32 x 32 tiles to the right, a row per block.
+constexpr int kMirror = 32;  // tile of mirror_kernel
+
+// Zeros from the diagonal's tiles to the right, a row per block.
 __global__ void __launch_bounds__(256) zero_upper_kernel(float2* __restrict__ z, int64_t n) {
     float2* row = z + (int64_t)blockIdx.x * n;
-    for (int64_t c = (int64_t)blockIdx.x / 32 * 32 + threadIdx.x; c < n; c += 256) row[c] = make_float2(0.f, 0.f);
+    for (int64_t c = (int64_t)blockIdx.x / kMirror * kMirror + threadIdx.x; c < n; c += 256) row[c] = make_float2(0.f, 0.f);
 }
 
-// z[n, m] = z[m, n] for m < n, a 32 x 32 tile above the diagonal per block.  Tile rows y and t - 1 - y together
+// z[n, m] = z[m, n] for m < n, a tile above the diagonal per block.  Tile rows y and t - 1 - y together
 // have t + 1 tiles: the grid is (t + 1) x ceil(t / 2).
+// Bound: HBM.  A thread's four loads are in flight together: 30720 edges (7.5 GB) 1.08 ms, 6.99 TB/s, against 1.47 one
+// after the other; tiles of 64 1.27.
 __global__ void __launch_bounds__(256) mirror_kernel(float2* __restrict__ z, int64_t n, int t) {
-    __shared__ float2 s[32][33];
+    __shared__ float2 s[kMirror][kMirror + 1];
     const int x = blockIdx.x, y = blockIdx.y;
     if (x <= y && 2 * y == t - 1) return;  // the middle row pairs with itself
-    const int64_t i0 = 32 * (int64_t)(x > y ? y : t - 1 - y), j0 = 32 * (int64_t)(x > y ? x - 1 : t - 1 - x);
-    const int c = threadIdx.x & 31;
-    for (int r = threadIdx.x >> 5; r < 32; r += 8)
+    const int64_t i0 = kMirror * (int64_t)(x > y ? y : t - 1 - y), j0 = kMirror * (int64_t)(x > y ? x - 1 : t - 1 - x);
+    constexpr int kRows = 256 / kMirror;
+    const int c = threadIdx.x % kMirror, r0 = threadIdx.x / kMirror;
+#pragma unroll
+    for (int q = 0; q < kMirror / kRows; ++q) {
+        const int r = r0 + kRows * q;
         if (i0 + r < n && j0 + c < n) s[r][c] = z[(i0 + r) * n + j0 + c];
+    }
     __syncthreads();
-    for (int r = threadIdx.x >> 5; r < 32; r += 8)
+#pragma unroll
+    for (int q = 0; q < kMirror / kRows; ++q) {
+        const int r = r0 + kRows * q;
         if (j0 + r < n && i0 + c < n && j0 + r > i0 + c) z[(j0 + r) * n + i0 + c] = s[c][r];
+    }
 }
 
 template <bool UPPER>
@@ -979,7 +990,7 @@ int launch_mom_sym_pairs(const float* verts, const int32_t* faces, const int32_t
     if (gx > 0x7fffffffLL || gy > 65535) return set_error(MB_ERR_SIZE, "mesh too large for one launch");
     // a matrix that is not added to is summed above the diagonal only, half the reductions, and mirrored
     const auto kernel = overwrite ? sym_pairs_kernel<true> : sym_pairs_kernel<false>;
-    const int64_t tiles = (n_edges + 31) / 32;
+    const int64_t tiles = (n_edges + kMirror - 1) / kMirror;
     if (overwrite && (n_edges > 0x7fffffffLL || (tiles + 1) / 2 > 65535))
         return set_error(MB_ERR_SIZE, "matrix too large for one launch");
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kEdgeSumBytes);

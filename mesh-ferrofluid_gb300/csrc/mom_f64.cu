@@ -37,7 +37,7 @@ struct F64Rows {
     double2 r[kF64Points];   // r1 - r2, r2 of a test point
     double w[kF64Points];    // its weight; once per row, times twice the area, in a[4]
     double r0[kF64Points];   // 1 - r1
-    double a[kF64Points][5]; // x - A0, its square, and the weight on this face; once per row
+    double a[kF64Points][6]; // A = x - A0, its square, the weight on this face, and n.A; once per row
     // of each row: A0 (0-2), A1 - A0 (3-5), A2 - A0 (6-8), n1 (9-11), L / (2 area) (12), h^2 (13), 2 area (14),
     // A1 (15-17), A2 (18-20)
     double v[kF64Rows][21];
@@ -77,7 +77,7 @@ __device__ __forceinline__ void f64_sums(const F64Rows& sh, const double* rv, in
                                          const double (&p1)[NS], const double (&p2)[NS], const double (&wj)[NS],
                                          const double (&yn)[NS], double k, const V3<double>& c0,
                                          const V3<double>& c1, const V3<double>& c2, double be1, double be2,
-                                         double xn, bool same, double* re, double* im, double* self) {
+                                         double xn0, bool same, double* re, double* im, double* self) {
     double ar = 0.0, ai = 0.0, sa = 0.0;
     const V3<double> n = {rv[9], rv[10], rv[11]};
     const double turn = k * (kAngles / (2.0 * kPi)), m4k = -4.0 / k;
@@ -87,6 +87,7 @@ __device__ __forceinline__ void f64_sums(const F64Rows& sh, const double* rv, in
         const V3<double> a = {sh.a[i][0], sh.a[i][1], sh.a[i][2]};
         const double aa = sh.a[i][3];
         const double w = sh.a[i][4];
+        const double xn = xn0 + sh.a[i][5];
         V3<double> x;
         double xa, x2;
         if constexpr (CLOSE) {
@@ -205,10 +206,13 @@ __global__ void __launch_bounds__(kF64Threads, NS <= 4 ? 4 : 2) mom_f64_kernel(
                                   fma(r.x, rv[5], r.y * rv[8])};
             sh.a[i][0] = a.x, sh.a[i][1] = a.y, sh.a[i][2] = a.z, sh.a[i][3] = dot(a, a);
             sh.a[i][4] = sh.w[i] * rv[14];
+            sh.a[i][5] = dot3(rv + 9, a);
         }
         __syncthreads();
         const V3<double> b = {B0.x - rv[0], B0.y - rv[1], B0.z - rv[2]};
-        const double be1 = dot3(rv + 3, b), be2 = dot3(rv + 6, b), xn = -dot3(rv + 9, b);  // x.n: A lies in the face
+        const double be1 = dot3(rv + 3, b), be2 = dot3(rv + 6, b);
+        // x.n = n.(A0 - B0) + n.A; the second is rounding for a face's own normal, but the normals are the caller's
+        const double xn = -dot3(rv + 9, b);
         const V3<double> c0 = {rv[0] - B0.x, rv[1] - B0.y, rv[2] - B0.z};  // the test corners from B0
         const V3<double> c1 = {rv[15] - B0.x, rv[16] - B0.y, rv[17] - B0.z};
         const V3<double> c2 = {rv[18] - B0.x, rv[19] - B0.y, rv[20] - B0.z};

@@ -509,7 +509,11 @@ static int gmres_core(const GmresMatrix& A, int64_t n, const double* b, double* 
                       int64_t* cycles_out, double* relres_out, int* status_out, cudaStream_t s) {
     GmresWork g = carve(workspace, n, m);
     GmresCyclePlan plan;
-    gmres_cycle_begin(&plan, A.kind, n, m);
+    plan.ok = false;
+    // The resident cycle reads b, x and its workspace 16 bytes at a time; the launches below take b and the
+    // workspace at their elements' 8 (a buffer of doubles from its second on).
+    if (((reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(workspace)) & 15) == 0)
+        gmres_cycle_begin(&plan, A.kind, n, m);
     if (plan.ok) return gmres_resident(A, n, b, x, m, max_iters, tol, g, plan, iters_out, cycles_out, relres_out, status_out, s);
     std::complex<double>* H = hs.H;
     std::complex<double>* cs = hs.cs;

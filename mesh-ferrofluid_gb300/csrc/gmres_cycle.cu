@@ -32,6 +32,7 @@ namespace {
 
 constexpr int kThreads = 1024, kWarps = 32;
 constexpr int64_t kMaxUnknowns = 12288;
+constexpr int kStaticShared = 1024;  // bytes of shared memory left to the kernel's own variables
 constexpr long long kPollLimit = 1ll << 22;  // about 2 s of polls
 
 struct CycleArgs {
@@ -585,13 +586,15 @@ int gmres_cycle_begin(GmresCyclePlan* p, int kind, int64_t n, int m) {
     cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
     if (!coop || n > kMaxUnknowns ||
-        !cycle_plan(kind, n, m, sms, smem - 1024, &p->rows, &p->pad, &p->grid, &p->bytes, &p->staged))
+        !cycle_plan(kind, n, m, sms, smem - kStaticShared, &p->rows, &p->pad, &p->grid, &p->bytes, &p->staged))
         return MB_OK;
     p->kernel = kind == 0 ? (p->staged ? (const void*)gmres_cycle_kernel<0, true> : (const void*)gmres_cycle_kernel<0, false>)
               : kind == 1 ? (p->staged ? (const void*)gmres_cycle_kernel<1, true> : (const void*)gmres_cycle_kernel<1, false>)
                           : (p->staged ? (const void*)gmres_cycle_kernel<2, true> : (const void*)gmres_cycle_kernel<2, false>);
+    // The limit belongs to the process, not to this solve: another thread's solve may set it between two cycles
+    // of this one, so it is the same for every plan.
     int per_sm = 0;
-    if (cudaFuncSetAttribute(p->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->bytes) != cudaSuccess ||
+    if (cudaFuncSetAttribute(p->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem - kStaticShared) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, p->kernel, kThreads, p->bytes) != cudaSuccess || per_sm < 1) {
         cudaGetLastError();
         return MB_OK;

@@ -481,26 +481,26 @@ static void residual_of(const GmresMatrix& A, int64_t n, const double* x, const 
 }
 
 // Restart cycles as one resident kernel each (gmres_cycle.cu): two launches and one host
-// synchronisation per cycle.
+// synchronisation per cycle.  *done false: the driver refused a cycle's launch; x and *st are those of the cycles
+// before it, from which the caller goes on.
 static int gmres_resident(const GmresMatrix& A, int64_t n, const double* b, double* x, int m, int max_iters, double tol,
-                          const GmresWork& g, const GmresCyclePlan& plan, int64_t* iters_out, int64_t* cycles_out,
-                          double* relres_out, int* status_out, cudaStream_t s) {
+                          const GmresWork& g, const GmresCyclePlan& plan, GmresState* out, bool* done, cudaStream_t s) {
     const GmresCycleRegion q(g.cycle, m);
     cudaMemsetAsync(&q.head->st, 0, sizeof(GmresState), s);
     GmresHead head{};
     const GmresState& st = head.st;
+    *done = false;
     for (long long c = 0; c < (long long)max_iters + 2 && !st.finished; ++c) {
         residual_of(A, n, x, b, g.r, s);
-        int rc = gmres_cycle_launch(plan, A.a, n, b, x, g.r, m, tol, max_iters, g.v32, g.w, g.cycle, s);
-        if (rc) return rc;
+        bool refused = false;
+        int rc = gmres_cycle_launch(plan, A.a, n, b, x, g.r, m, tol, max_iters, g.v32, g.w, g.cycle, &refused, s);
+        if (rc || refused) return rc;
         cudaMemcpyAsync(&head, q.head, sizeof(head), cudaMemcpyDeviceToHost, s);
         if ((rc = sync_check(s, "gmres cycle"))) return rc;
         if (head.sync.error) return set_error(MB_ERR_CUDA, "gmres cycle: a wait between the grid's blocks ran out");
+        *out = st;
     }
-    if (iters_out) *iters_out = st.iters;
-    if (cycles_out) *cycles_out = st.cycles;
-    if (relres_out) *relres_out = st.relres;
-    if (status_out) *status_out = st.converged ? 0 : 1;
+    *done = true;
     return MB_OK;
 }
 
@@ -514,7 +514,19 @@ static int gmres_core(const GmresMatrix& A, int64_t n, const double* b, double* 
     // workspace at their elements' 8 (a buffer of doubles from its second on).
     if (((reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(workspace)) & 15) == 0)
         gmres_cycle_begin(&plan, A.kind, n, m);
-    if (plan.ok) return gmres_resident(A, n, b, x, m, max_iters, tol, g, plan, iters_out, cycles_out, relres_out, status_out, s);
+    GmresState st{};
+    if (plan.ok) {
+        bool done = false;
+        const int rc = gmres_resident(A, n, b, x, m, max_iters, tol, g, plan, &st, &done, s);
+        if (rc) return rc;
+        if (done) {
+            if (iters_out) *iters_out = st.iters;
+            if (cycles_out) *cycles_out = st.cycles;
+            if (relres_out) *relres_out = st.relres;
+            if (status_out) *status_out = st.converged ? 0 : 1;
+            return MB_OK;
+        }
+    }
     std::complex<double>* H = hs.H;
     std::complex<double>* cs = hs.cs;
     std::complex<double>* sn = hs.sn;
@@ -528,7 +540,7 @@ static int gmres_core(const GmresMatrix& A, int64_t n, const double* b, double* 
     double bnorm;
     if ((rc = norm_of(b, n, g.nrm, &bnorm, s))) return rc;
     if (bnorm == 0.0) bnorm = 1.0;
-    int64_t iters = 0, cycles = 0;
+    int64_t iters = st.iters, cycles = st.cycles;
     double relres = 0.0;
     int status = 1;
     while (true) {

@@ -604,7 +604,9 @@ int gmres_cycle_begin(GmresCyclePlan* p, int kind, int64_t n, int m) {
 }
 
 int gmres_cycle_launch(const GmresCyclePlan& p, const void* a, int64_t n, const double* b, double* x, const double* r,
-                       int m, double tol, long long max_iters, float* v32, double* v64, void* region, cudaStream_t s) {
+                       int m, double tol, long long max_iters, float* v32, double* v64, void* region, bool* refused,
+                       cudaStream_t s) {
+    *refused = false;
     const GmresCycleRegion q(region, m);
     // the counters and sums of a cycle start from zero
     cudaMemsetAsync(&q.head->sync, 0, GmresCycleRegion::zero_bytes(m), s);
@@ -613,11 +615,11 @@ int gmres_cycle_launch(const GmresCyclePlan& p, const void* a, int64_t n, const 
                 p.rows, p.pad, tol, max_iters};
     void* args[] = {&g};
     const cudaError_t e = cudaLaunchCooperativeKernel(p.kernel, dim3((unsigned)p.grid), dim3(kThreads), args, p.bytes, s);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        return set_error(MB_ERR_CUDA, "gmres cycle: %s", cudaGetErrorString(e));
-    }
-    return MB_OK;
+    if (e == cudaSuccess) return MB_OK;
+    cudaGetLastError();
+    // a context with fewer SMs than the device says, or one that takes no such launch
+    *refused = e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported;
+    return *refused ? MB_OK : set_error(MB_ERR_CUDA, "gmres cycle: %s", cudaGetErrorString(e));
 }
 
 }  // namespace mb

@@ -56,8 +56,10 @@ struct GmresCyclePlan {
 // Plans the resident cycle for a matrix kind (0 complex64, 1 float32, 2 float64), n unknowns and restart m;
 // plan->ok false where the launch-per-operation form has to run.
 int gmres_cycle_begin(GmresCyclePlan* plan, int kind, int64_t n, int m);
-// One cycle from the residual r (complex128): x updated, GmresState advanced.
+// One cycle from the residual r (complex128): x updated, GmresState advanced.  *refused: the driver does not
+// grant the launch here and nothing ran.
 int gmres_cycle_launch(const GmresCyclePlan& plan, const void* a, int64_t n, const double* b, double* x, const double* r,
-                       int m, double tol, long long max_iters, float* v32, double* v64, void* region, cudaStream_t s);
+                       int m, double tol, long long max_iters, float* v32, double* v64, void* region, bool* refused,
+                       cudaStream_t s);
 
 }  // namespace mb

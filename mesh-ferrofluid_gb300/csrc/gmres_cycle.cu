@@ -336,7 +336,9 @@ __device__ void givens_column(const CycleArgs& g, int j, const double2* h1, cons
     }
     if (threadIdx.x == 0) {
         const double2 a = chain[j];
-        const double rr = sqrt(fma(a.x, a.x, fma(a.y, a.y, hn * hn))), ir = rr == 0.0 ? 0.0 : 1.0 / rr;
+        // a matrix of entries about 1e+-150: the squares leave the range, the values do not
+        const double r2 = fma(a.x, a.x, fma(a.y, a.y, hn * hn));
+        const double rr = r2 > 1e-280 && r2 < 1e280 ? sqrt(r2) : hypot(hypot(a.x, a.y), hn), ir = rr == 0.0 ? 0.0 : 1.0 / rr;
         const double2 c = rr == 0.0 ? make_double2(1.0, 0.0) : make_double2(a.x * ir, a.y * ir);
         const double s = hn * ir;
         cs[j] = c;

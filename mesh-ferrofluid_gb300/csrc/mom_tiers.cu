@@ -290,12 +290,14 @@ __global__ void __launch_bounds__(128, 2) far_pairs_kernel(const TierArgs args, 
     __syncthreads();
     if (q >= m.nf) return;
     const float4* rq = rec + (kRec / 4) * q;
-    const float4 q0 = __ldg(rq), q1 = __ldg(rq + 1), q2 = __ldg(rq + 2), q3 = __ldg(rq + 3), q4 = __ldg(rq + 4),
+    const float k = (float)m.k, k2 = k * k;
+    const float4 q0 = __ldg(rq);
+    if (!(k2 * q0.w <= 0.09f)) return;  // tier 1 needs (k rho)^2 <= (2e-6 / 2.7e-4)^(1/2) = 0.086
+    const float4 q1 = __ldg(rq + 1), q2 = __ldg(rq + 2), q3 = __ldg(rq + 3), q4 = __ldg(rq + 4),
                  q5 = __ldg(rq + 5), q6 = __ldg(rq + 6);
     const float B[3][3] = {{q2.x, q2.y, q2.z}, {q3.x, q3.y, q3.z}, {q4.x, q4.y, q4.z}};
     const float BB[3] = {q6.x, q6.y, q6.z}, hq[3] = {q4.w, q5.w, q6.w};
     const int col[3] = {__float_as_int(q1.w), __float_as_int(q2.w), __float_as_int(q3.w)};
-    const float k = (float)m.k, k2 = k * k;
     const double kt = m.k * kInv2Pi;
     const float kth = (float)kt, ktl = (float)(kt - (double)kth), four_k = 4.f / k;
     constexpr float SA = -0.16666371f, SB = 0.00828212f;                     // sin
@@ -591,7 +593,7 @@ __device__ __forceinline__ void shared_test_entries(const float* __restrict__ rp
 constexpr int kTilePairs = 1024;
 
 template <int NX, int NY, bool CLOSE>
-__global__ void __launch_bounds__(128, NX <= 4 ? 4 : 3) close_pairs_kernel(const TierArgs args, int tp, int tq) {
+__global__ void __launch_bounds__(128, NX <= 4 ? 4 : CLOSE ? 2 : 3) close_pairs_kernel(const TierArgs args, int tp, int tq) {
     __shared__ float4 s_t[NX * NX], s_s[NY * NY], s_src[(NY * NY + 1) / 2 * 2];
     __shared__ float s_b[19][4];
     __shared__ float4 s_p[256], s_q[256];
@@ -618,7 +620,8 @@ __global__ void __launch_bounds__(128, NX <= 4 ? 4 : 3) close_pairs_kernel(const
     // tq is a power of two up to 128: a thread keeps one source face and steps through the test faces
     const float limit = CLOSE || NX > 3 ? far_limit(__int_as_float(s_rho), k2) : __int_as_float(0x7f800000);
     const int b = threadIdx.x & (tq - 1);
-    if (b < nq) {
+    // (tier 3 ends at k rho = 0.8: a larger face has nothing for the launch of tiers 2 and 3)
+    if (b < nq && (CLOSE || k2 * s_q[b].w <= 0.65f)) {
         const float4 q = s_q[b];
         for (int a = threadIdx.x / tq; a < np; a += 128 / tq) {
             const float4 p = s_p[a];
@@ -640,15 +643,36 @@ __global__ void __launch_bounds__(128, NX <= 4 ? 4 : 3) close_pairs_kernel(const
     __syncthreads();
     const float* rec = args.rec + kRec * m.f0;
     if constexpr (CLOSE) {
-        for (int i = threadIdx.x; i < 9 * n0; i += 128) {
-            const int c = s_list[0][i / 9], e = i % 9;
-            const int64_t p = p0 + c / tq, q = q0 + (c & (tq - 1));
-            float re, im;
-            mom_entry_fast<NX, NY>(args.verts, args.faces, args.areas, args.normals, s_t, s_s, k, m.f0 + p, e / 3,
-                                   m.f0 + q, e % 3, &re, &im);
-            const int64_t row = __float_as_int(rec[kRec * p + kEdge + 4 * (e / 3)]);
-            const int64_t col = __float_as_int(rec[kRec * q + kEdge + 4 * (e % 3)]);
-            atomicAdd(reinterpret_cast<float2*>(m.z) + row * m.pitch + col, make_float2(re, im));
+        // e1 slowest: neighbouring threads have the same test corner and the corners of one source face
+        const int per = 3 * n0;
+        if constexpr (NX == 3) {
+            // short entries: where the list gives every thread enough, all three by one thread, whose source points
+            // serve them all (5120 faces, k 10: 10.65 -> 10.44 ms; gaussQR 4 and 5: no gain)
+            const int span = n0 >= 512 ? 3 : 1;
+            for (int i = threadIdx.x; i < (span == 3 ? per : 3 * per); i += 128) {
+                const int first = (i >= per) + (i >= 2 * per), r = i - first * per, c = s_list[0][r / 3], e2 = r % 3;
+                const int64_t p = p0 + c / tq, q = q0 + (c & (tq - 1));
+                const int64_t col = __float_as_int(rec[kRec * q + kEdge + 4 * e2]);
+#pragma unroll 1
+                for (int e1 = first; e1 < first + span; ++e1) {
+                    float re, im;
+                    mom_entry_fast<NX, NY>(args.verts, args.faces, args.areas, args.normals, s_t, s_s, k, m.f0 + p, e1,
+                                           m.f0 + q, e2, &re, &im);
+                    const int64_t row = __float_as_int(rec[kRec * p + kEdge + 4 * e1]);
+                    atomicAdd(reinterpret_cast<float2*>(m.z) + row * m.pitch + col, make_float2(re, im));
+                }
+            }
+        } else {
+            for (int i = threadIdx.x; i < 3 * per; i += 128) {
+                const int e1 = (i >= per) + (i >= 2 * per), r = i - e1 * per, c = s_list[0][r / 3], e2 = r % 3;
+                const int64_t p = p0 + c / tq, q = q0 + (c & (tq - 1));
+                float re, im;
+                mom_entry_fast<NX, NY>(args.verts, args.faces, args.areas, args.normals, s_t, s_s, k, m.f0 + p, e1,
+                                       m.f0 + q, e2, &re, &im);
+                const int64_t row = __float_as_int(rec[kRec * p + kEdge + 4 * e1]);
+                const int64_t col = __float_as_int(rec[kRec * q + kEdge + 4 * e2]);
+                atomicAdd(reinterpret_cast<float2*>(m.z) + row * m.pitch + col, make_float2(re, im));
+            }
         }
     } else {
         if (threadIdx.x < (NY * NY + 1) / 2 * 2) {  // barycentric form of the source rule: (r3 - r4, r4, weight)
@@ -914,15 +938,19 @@ __global__ void __launch_bounds__(128, 4)
 
 }  // namespace
 
-// Tile sizes: 32 test faces per block of tier 1 once that leaves 8 blocks per SM (its per-thread
-// source set-up is amortised over them), 8 below; the close pairs' tiles hold 1024 pairs on
-// large meshes, fewer on small ones: 8 times the chip's 608 resident blocks, so that the last
-// wave is a small part (1280 faces in tier 4: 2.83 ms with 2.6 waves of 1024-pair tiles, 2.56 ms as edge rows).
-void mom_tier_tiles(int64_t nf, int* rows, int* tp, int* tq) {
-    *rows = nf >= 5000 ? 32 : 8;
-    const double per_block = (double)nf * (double)nf / 4864.0;
-    *tp = per_block >= 1024 ? 16 : per_block >= 256 ? 8 : per_block >= 64 ? 4 : 7;
-    *tq = per_block >= 64 ? 4 * *tp : 2;  // the smallest, 14 pairs: 126 entries, one per thread
+// Tile sizes for that many (test face, source face) pairs in a launch, over all its meshes.  Tier 1's test faces per
+// block (its per-thread source set-up is amortised over them) matter little: 4 to 32 of them within 2 % of the call at 1280
+// faces (the fewer the better), 8 / 16 / 32 3.40 / 3.35 / 3.36 ms at 5120, 35.0 / 34.4 / 34.3 at 20480.  The close pairs' tiles hold
+// 1024 pairs on large meshes, fewer on small ones, so that the last wave is a small part of the time; 14 x 16 pairs are 2016
+// entries, 15.75 rounds of 128 threads.  Measured, us, gaussQR 4, tp x tq 16x64 / 8x64 / 14x16 / 4x32 / 4x16 / 7x2:
+// 3 meshes of 80 faces 314 / 172 / - / 82 / 57 / 59; one of 320, k 1, 370 / 268 / 192 / 176 / 151 / 200; 64 of 80 838 /
+// 698 / - / 586 / 571 / 690; one of 1280, k 30, 2115 / 2090 / 2008 / 2025 / 2089 / 2351; 50 of 320 3788 / 3695 / - / 3981 /
+// 4415 / 8230; one of 5120, k 10, gaussQR 3, 10.36 / 10.43 ms, 8x32 11.02.
+void mom_tier_tiles(int64_t pairs, int* rows, int* tp, int* tq) {
+    *rows = pairs >= 5000 * 5000 ? 32 : 8;
+    const double per_block = (double)pairs / 4864.0;  // were there 8 times the 608 resident blocks
+    *tp = per_block >= 4096 ? 16 : per_block >= 1024 ? 8 : per_block >= 200 ? 14 : per_block >= 3 ? 4 : 7;
+    *tq = per_block >= 1024 ? 64 : per_block >= 200 ? 16 : per_block >= 40 ? 32 : per_block >= 3 ? 16 : 2;
 }
 
 int64_t mom_tier_blocks(int64_t nf, int64_t tp, int64_t tq) { return ((nf + tp - 1) / tp) * ((nf + tq - 1) / tq); }
@@ -961,7 +989,7 @@ int launch_mom_tiers(const float* verts, const int32_t* faces, int64_t nf, const
     if (nf <= 0) return MB_OK;
     if (int rc = tier_records(verts, faces, normals, fei, nf, gpx, gwx, nx, gpy, gwy, ny, rec, s)) return rc;
     int rows, tp, tq;
-    mom_tier_tiles(nf, &rows, &tp, &tq);
+    mom_tier_tiles(nf * nf, &rows, &tp, &tq);
     const TierArgs a{verts, faces, areas, normals, rec, gpx, gwx, gpy, gwy, nullptr, nullptr, nullptr, 0, nf, n_edges, k, z};
     return MB_TIERS(a, mom_tier_blocks(nf, rows, 128), mom_tier_blocks(nf, tp, tq), rows, tp, tq, nullptr, nullptr, s);
 }

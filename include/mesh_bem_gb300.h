@@ -447,6 +447,8 @@ int mb_mom_ref_zmat_batched_persistent_c64(const float* verts, const int32_t* fa
                                            const int64_t* block_offsets, int64_t total_blocks, const double* ks,
                                            int n_mesh, const float* gpx, const float* gwx, int nx, const float* gpy,
                                            const float* gwy, int ny, float* z, void* stream);
+/* Tile sizes for mb_mom_ref_zmat_batched_tiers_c64 over meshes of F_i faces: face_pairs = sum of F_i^2. */
+int mb_mom_tier_tiles(int64_t face_pairs, int32_t* rows, int32_t* tp, int32_t* tq);
 /* The same matrices as mb_mom_zmat_rwg_tiers_c64 builds them; gaussQR 3 to 5.  far_offsets / close_offsets
  * [n_mesh + 1]: first block of each mesh with ceil(F_i / rows) x ceil(F_i / 128) blocks (rows <= 32) and with
  * ceil(F_i / tp) x ceil(F_i / tq) blocks (tp <= 256, tq a power of two <= 128, tp tq <= 1024).  workspace: as above for the

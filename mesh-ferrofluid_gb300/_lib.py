@@ -46,6 +46,7 @@ _SIGS = {
     "mb_face_geometry_f64": [_P, _I64, _P, _I64, _P, _P, _P],
     "mb_index_range_i32": [_P, _I64, _I64, _P, _P, _P],
     "mb_mom_tiers_workspace_bytes": [_I64],
+    "mb_mom_tier_tiles": [_I64, _P, _P, _P],
     "mb_mom_sym_zmat_rwg_pairs_c64": [_P, _I64, _P, _I64, _P, _I64, _D, _I, _P, _I64, _P, _P],
     "mb_mom_zmat_rwg_tiers_c64": [_P, _I64, _P, _I64, _P, _P, _P, _I64, _P, _P, _I, _P, _P, _I, _D, _P, _I64, _P,
                                   _P],

@@ -8,7 +8,7 @@ of meshes of uneven size (and wavenumber) into one vertex / face array and runs
   launch of the separated-pair kernel and one of the near-pair kernel
   (``mb_mom_sym_zmat_batched_c64``); with ``formulation="cfie_ref"`` (the reference's EFIE +
   MFIE operator and collapsed Gauss rule, gaussQR 4) one call whose quadrature is sized by each pair's
-  separation (``mb_mom_ref_zmat_batched_tiers_c64``; other rule sizes
+  separation (``mb_mom_ref_zmat_batched_tiers_c64``; other rule sizes and batches of small meshes
   ``mb_mom_ref_zmat_batched_c64``);
 * the excitation of ``nc`` plane waves per mesh in one launch (``mb_mom_sym_rhs_batched_c64``)
   into a padded block [max E_i, n_mesh * nc];
@@ -90,12 +90,18 @@ class MeshBatch:
             nfs = desc[:, 1]
             per = 3 * nfs * ((3 * nfs + 127) // 128)
             self.ref_boff = torch.tensor(np.concatenate([[0], np.cumsum(per)]).astype(np.int64), device=dev)
-            if gaussQR in (3, 4, 5):
-                rows, tp, tq = self._tier_tiles = (32, 16, 64)
+            pairs, self._tier_blocks = int((nfs * nfs).sum()), None
+            # Below 256 faces every pair of a closed mesh takes the reference's points, and the tiered call's three
+            # more launches cost 12 us: 20 x 8 faces 63 us against 79, 64 x 80 615 / 631 (gaussQR 4).  gaussQR 3, with
+            # little to save on a close pair, from half a million face pairs on: 3 x 320 192 / 207, 12 x 320 617 / 586.
+            if gaussQR in (3, 4, 5) and nfs.max() >= 256 and (gaussQR > 3 or pairs >= 500_000):
+                tile = [ctypes.c_int32() for _ in range(3)]
+                _lib.call("mb_mom_tier_tiles", pairs, *(ctypes.byref(t) for t in tile))
+                rows, tp, tq = self._tier_tiles = tuple(t.value for t in tile)
                 tiles = [((nfs + a - 1) // a) * ((nfs + b - 1) // b) for a, b in ((rows, 128), (tp, tq))]
-                off = np.stack([np.concatenate([[0], np.cumsum(t)]) for t in tiles]).astype(np.int64)
-                self._tier_blocks = (int(off[0, -1]), int(off[1, -1]))
-                self._tier_off = torch.tensor(off, device=dev)
+                off = [np.concatenate([[0], np.cumsum(t)]).astype(np.int64) for t in tiles]
+                self._tier_blocks = tuple(int(o[-1]) for o in off)
+                self._tier_off = tuple(torch.tensor(o, device=dev) for o in off)
         self.ks = torch.tensor(np.asarray(wavenumbers, np.float64), device=dev)
         if not bool(torch.all(self.ks > 0)):
             raise ValueError("wavenumbers must be > 0")
@@ -149,7 +155,7 @@ class MeshBatch:
             out.zero_()
         if self.formulation == "cfie_ref":
             cfg = getattr(self, "asm_config", None)
-            if self.gq in (3, 4, 5) and cfg in (None, ("grid", None)):
+            if self._tier_blocks is not None and cfg in (None, ("grid", None)):
                 ws = torch.empty(int(_lib.load().mb_mom_tiers_workspace_bytes(self.total_faces)), dtype=torch.uint8,
                                  device=self.device)
                 _lib.call("mb_mom_ref_zmat_batched_tiers_c64", _lib.ptr(self.verts), _lib.ptr(self.faces),
@@ -200,8 +206,8 @@ class MeshBatch:
         """Pick the assembly's tile and block schedule by timing each candidate.  EFIE: the one-
         pair-per-thread kernel, or the rows layout with 8, 16 or 32 test faces per block and the
         meshes' blocks in packing order or largest mesh first.  Reference CFIE: a grid
-        over the meshes' tiles ("grid", None; each face pair's quadrature sized by its separation
-        for gaussQR 3-5, one block per (mesh, row, 128-column tile) for 2) or a resident grid taking
+        over the meshes' tiles ("grid", None; each face pair's quadrature sized by its separation,
+        or, for gaussQR 2 and small meshes, one block per (mesh, row, 128-column tile)) or a resident grid taking
         the (mesh, row, 128-column) tiles from a work counter ("persistent", None).  Returns the chosen configuration."""
         if self.desc is None:
             self._set_nc(1)

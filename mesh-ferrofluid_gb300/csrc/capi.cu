@@ -94,6 +94,7 @@ int launch_face_geometry(const T* verts, int64_t nv, const int32_t* faces, int64
 int index_range(const int32_t* idx, int64_t count, int64_t limit, int32_t* work, int32_t* outside, cudaStream_t s);
 int launch_edge_rows(const int32_t* fei, int64_t nf, int64_t n_edges, int32_t* er, cudaStream_t s);
 bool mom_tier_rule(int nx, int ny);
+void mom_tier_tiles(int64_t pairs, int* rows, int* tp, int* tq);
 int launch_mom_sym_pairs(const float* verts, const int32_t* faces, const int32_t* fei, int64_t nf, int64_t n_edges, double k,
                          bool overwrite, float* rec, float* z, cudaStream_t s);
 int launch_mom_tiers(const float* verts, const int32_t* faces, int64_t nf, const float* areas, const float* normals,
@@ -315,6 +316,12 @@ int mb_index_range_i32(const int32_t* indices, int64_t count, int64_t limit, int
 }
 
 int64_t mb_mom_tiers_workspace_bytes(int64_t n_faces) { return n_faces > 0 ? 128 * n_faces : 0; }
+
+int mb_mom_tier_tiles(int64_t face_pairs, int32_t* rows, int32_t* tp, int32_t* tq) {
+    MB_REQUIRE(face_pairs >= 0 && rows && tp && tq, "null pointer argument or negative count");
+    mom_tier_tiles(face_pairs, rows, tp, tq);
+    return MB_OK;
+}
 
 int mb_mom_sym_zmat_rwg_pairs_c64(const float* verts, int64_t n_verts, const int32_t* faces, int64_t n_faces,
                                   const int32_t* face_edge_indices, int64_t n_edges, double wavenumber, int overwrite,

@@ -95,6 +95,79 @@ __device__ __forceinline__ void sym_far_pair(const T (*s_rule)[4], const T (*s_y
     }
 }
 
+// Two separated pairs (fy, fxa) and (fy, fxb) at once in packed f32x2 arithmetic (lane .x
+// the first source face, .y the second): the same sums as sym_far_pair with half the FP32
+// instructions.  X0..X2 hold both faces' shifted corners per coordinate; acc as in
+// sym_far_pair, packed.
+template <int LAYER, int NPHI>
+__device__ __forceinline__ void sym_far_pair2(const float4 (*s_r4)[2], const float4 (*s_y4)[2], const float3& ny,
+                                              const float2 X0[3], const float2 X1[3], const float2 X2[3],
+                                              float2 acc[9]) {
+    // s_r4[j] = {(r0, r0, r1, r1), (r2, r2, w, w)}, s_y4[j] = {(y.x, y.x, y.y, y.y),
+    // (y.z, y.z, wA, wA)}: every value already duplicated, so one 16-byte shared load yields two
+    // packed operands and no register moves are needed to broadcast them
+    float2 e1[3], e2[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        e1[c] = sub2(X1[c], X0[c]);
+        e2[c] = sub2(X2[c], X1[c]);
+    }
+    const float2 nx0 = fma2(e1[1], e2[2], mul2(bc(-1.f), mul2(e1[2], e2[1])));
+    const float2 nx1 = fma2(e1[2], e2[0], mul2(bc(-1.f), mul2(e1[0], e2[2])));
+    const float2 nx2 = fma2(e1[0], e2[1], mul2(bc(-1.f), mul2(e1[1], e2[0])));
+    const float2 n2 = fma2(nx0, nx0, fma2(nx1, nx1, mul2(nx2, nx2)));
+    const float2 ax = make_float2(0.5f * sqrtf(n2.x), 0.5f * sqrtf(n2.y));
+#pragma unroll 1
+    for (int i = 0; i < 7; ++i) {
+        // re-read the tables every outer point instead of holding all 28 of them in registers
+        asm volatile("" ::: "memory");
+        const float4 ra = s_r4[i][0], rb = s_r4[i][1];
+        const float2 r0 = make_float2(ra.x, ra.y), r1 = make_float2(ra.z, ra.w), r2 = make_float2(rb.x, rb.y);
+        float2 x[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) x[c] = fma2(r0, X0[c], fma2(r1, X1[c], mul2(r2, X2[c])));
+        float2 s0 = bc(0.f), s1 = bc(0.f), s2 = bc(0.f);
+#pragma unroll
+        for (int j = 0; j < 7; ++j) {
+            const float4 ya = s_y4[j][0], yb = s_y4[j][1];
+            const float2 dx = sub2(x[0], make_float2(ya.x, ya.y));
+            const float2 dy = sub2(x[1], make_float2(ya.z, ya.w));
+            const float2 dz = sub2(x[2], make_float2(yb.x, yb.y));
+            const float2 d2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
+            const float2 ri = make_float2(rsqrtf(d2.x), rsqrtf(d2.y));
+            float2 g = mul2(ri, make_float2(yb.z, yb.w));
+            if constexpr (LAYER == 2) g = mul2(g, mul2(ri, ri));
+            if constexpr (NPHI == 3) {
+                const float4 qa = s_r4[j][0], qb = s_r4[j][1];
+                s0 = fma2(g, make_float2(qa.x, qa.y), s0);
+                s1 = fma2(g, make_float2(qa.z, qa.w), s1);
+                s2 = fma2(g, make_float2(qb.x, qb.y), s2);
+            } else {
+                s0 = add2(s0, g);
+            }
+        }
+        if constexpr (LAYER == 2) {
+            const float2 dn = fma2(x[0], bc(ny.x), fma2(x[1], bc(ny.y), mul2(x[2], bc(ny.z))));
+            s0 = mul2(s0, dn);
+            s1 = mul2(s1, dn);
+            s2 = mul2(s2, dn);
+        }
+        const float2 wx = mul2(make_float2(rb.z, rb.w), ax);
+        if constexpr (NPHI == 3) {
+            const float2 sa[3] = {s0, s1, s2};
+            const float2 rr[3] = {r0, r1, r2};
+#pragma unroll
+            for (int b = 0; b < 3; ++b) {
+                const float2 wb = mul2(wx, rr[b]);
+#pragma unroll
+                for (int a = 0; a < 3; ++a) acc[3 * a + b] = fma2(sa[a], wb, acc[3 * a + b]);
+            }
+        } else {
+            acc[0] = fma2(s0, wx, acc[0]);
+        }
+    }
+}
+
 // Block set-up shared by the panel and packed kernels: the 7-point rule, fy's shifted rule
 // points with weights, and fy's unit normal.
 template <typename T>
@@ -173,19 +246,21 @@ __device__ __forceinline__ void tri_curls(const V3<T>& p0, const V3<T>& p1, cons
 
 // Packed operators [V, V] without the [F, F, 3, 3] panels: OP 1 single layer, 2 double layer
 // (P1 x P1), 3 hypersingular (Maue: curl phi_a(fy) . curl phi_b(fx) times the P0 single
-// layer).  FP64: one block per test face fy sweeps every source face fx, accumulates the three
+// layer).  One block per test face fy sweeps every source face fx, accumulates the three
 // packed rows faces[fy, a] in shared memory (3 V values) and adds them to `packed` at the
-// end.  Pairs sharing a vertex are skipped here and added by lap_sym_near_kernel.
-template <int OP>
-__global__ void __launch_bounds__(kSymThreads, 1)
-    lap_sym_tight_kernel(const double* __restrict__ verts, const int32_t* __restrict__ faces, int64_t nf, int64_t nv,
-                         int64_t row_begin, double* __restrict__ packed) {
-    using T = double;
+// end.  Pairs sharing a vertex are skipped here and added by lap_sym_near_kernel.  FP64, and FP32 meshes of a few
+// hundred faces (launch_sym_pairs).
+template <typename T, int OP>
+__global__ void __launch_bounds__(kSymThreads, sizeof(T) == 4 ? (OP == 3 ? 6 : 4) : 1)
+    lap_sym_tight_kernel(const T* __restrict__ verts, const int32_t* __restrict__ faces, int64_t nf, int64_t nv,
+                         int64_t row_begin, T* __restrict__ packed) {
     constexpr int LAYER = OP == 2 ? 2 : 1;
     constexpr int NPHI = OP == 3 ? 1 : 3;
     __shared__ T s_rule[7][4];
     __shared__ T s_y[7][4];
     __shared__ T s_n[3];
+    __shared__ float4 s_r4[7][2];  // the same tables with every value duplicated (float path)
+    __shared__ float4 s_y4[7][2];
     extern __shared__ __align__(16) unsigned char tight_smem[];
     T* rows = reinterpret_cast<T*>(tight_smem);
     const int64_t fy = row_begin + blockIdx.x;
@@ -197,6 +272,17 @@ __global__ void __launch_bounds__(kSymThreads, 1)
     V3<T> cy[3];
     if constexpr (OP == 3) tri_curls(v3<T>(0, 0, 0), Y1, Y2, cy);
     __syncthreads();
+    if (threadIdx.x < 7) {
+        const int j = threadIdx.x;
+        const float r0 = (float)s_rule[j][0], r1 = (float)s_rule[j][1], r2 = (float)s_rule[j][2];
+        const float rw = (float)s_rule[j][3];
+        s_r4[j][0] = make_float4(r0, r0, r1, r1);
+        s_r4[j][1] = make_float4(r2, r2, rw, rw);
+        const float y0 = (float)s_y[j][0], y1 = (float)s_y[j][1], y2 = (float)s_y[j][2], yw = (float)s_y[j][3];
+        s_y4[j][0] = make_float4(y0, y0, y1, y1);
+        s_y4[j][1] = make_float4(y2, y2, yw, yw);
+    }
+    __syncthreads();
     const V3<T> ny = v3<T>(s_n[0], s_n[1], s_n[2]);
     // each thread sweeps its own strip of consecutive source faces: neighbouring faces share
     // vertices, and lanes of a warp working on neighbours would collide in the shared-memory
@@ -204,30 +290,71 @@ __global__ void __launch_bounds__(kSymThreads, 1)
     const int64_t strip = (nf + blockDim.x - 1) / blockDim.x;
     const int64_t strip0 = (int64_t)threadIdx.x * strip;
     const int64_t strip1 = strip0 + strip < nf ? strip0 + strip : nf;
+    if constexpr (sizeof(T) == 4 && OP != 3) {
+        // two source faces per thread and iteration (fxa, fxa + 1), packed arithmetic
+        // (the P0 sums of OP 3 are light enough that occupancy matters more)
+        const float3 nyf = make_float3(ny.x, ny.y, ny.z);
 #pragma unroll 1
-    for (int64_t fx = strip0; fx < strip1; ++fx) {
-        if (share_vertex(faces, fy, fx)) continue;
-        const int32_t vx[3] = {__ldg(faces + 3 * fx), __ldg(faces + 3 * fx + 1), __ldg(faces + 3 * fx + 2)};
-        const V3<T> X0 = load3(verts, vx[0]) - o;
-        const V3<T> X1 = load3(verts, vx[1]) - o;
-        const V3<T> X2 = load3(verts, vx[2]) - o;
-        T acc[9];
+        for (int64_t k = 0; k < strip; k += 2) {
+            const int64_t fxa = strip0 + k;
+            if (fxa >= strip1) break;
+            const int64_t fxb_raw = fxa + 1;
+            const bool has_b = fxb_raw < strip1;
+            const int64_t fxb = has_b ? fxb_raw : fxa;
+            const bool use_a = !share_vertex(faces, fy, fxa);
+            const bool use_b = has_b && !share_vertex(faces, fy, fxb);
+            if (!use_a && !use_b) continue;
+            const int32_t va[3] = {__ldg(faces + 3 * fxa), __ldg(faces + 3 * fxa + 1), __ldg(faces + 3 * fxa + 2)};
+            const int32_t vb[3] = {__ldg(faces + 3 * fxb), __ldg(faces + 3 * fxb + 1), __ldg(faces + 3 * fxb + 2)};
+            float2 X[3][3];  // corner, coordinate
 #pragma unroll
-        for (int c = 0; c < 9; ++c) acc[c] = 0;
-        sym_far_pair<T, LAYER, NPHI>(s_rule, s_y, ny, X0, X1, X2, acc);
-        if constexpr (OP == 3) {
-            V3<T> cx[3];
-            tri_curls(X0, X1, X2, cx);
-            const T w = acc[0] * T(kInv4Pi);
+            for (int v = 0; v < 3; ++v) {
+                const V3<T> pa = load3(verts, va[v]) - o;
+                const V3<T> pb = load3(verts, vb[v]) - o;
+                X[v][0] = make_float2(pa.x, pb.x);
+                X[v][1] = make_float2(pa.y, pb.y);
+                X[v][2] = make_float2(pa.z, pb.z);
+            }
+            float2 acc[9];
 #pragma unroll
-            for (int a = 0; a < 3; ++a)
+            for (int c = 0; c < 9; ++c) acc[c] = bc(0.f);
+            sym_far_pair2<LAYER, NPHI>(s_r4, s_y4, nyf, X[0], X[1], X[2], acc);
+            {
 #pragma unroll
-                for (int b = 0; b < 3; ++b) atomicAdd(rows + a * nv + vx[b], dot(cy[a], cx[b]) * w);
-        } else {
+                for (int a = 0; a < 3; ++a)
 #pragma unroll
-            for (int a = 0; a < 3; ++a)
+                    for (int b = 0; b < 3; ++b) {
+                        if (use_a) atomicAdd(rows + a * nv + va[b], acc[3 * a + b].x * T(kInv4Pi));
+                        if (use_b) atomicAdd(rows + a * nv + vb[b], acc[3 * a + b].y * T(kInv4Pi));
+                    }
+            }
+        }
+    } else {
+#pragma unroll 1
+        for (int64_t fx = strip0; fx < strip1; ++fx) {
+            if (share_vertex(faces, fy, fx)) continue;
+            const int32_t vx[3] = {__ldg(faces + 3 * fx), __ldg(faces + 3 * fx + 1), __ldg(faces + 3 * fx + 2)};
+            const V3<T> X0 = load3(verts, vx[0]) - o;
+            const V3<T> X1 = load3(verts, vx[1]) - o;
+            const V3<T> X2 = load3(verts, vx[2]) - o;
+            T acc[9];
 #pragma unroll
-                for (int b = 0; b < 3; ++b) atomicAdd(rows + a * nv + vx[b], acc[3 * a + b] * T(kInv4Pi));
+            for (int c = 0; c < 9; ++c) acc[c] = 0;
+            sym_far_pair<T, LAYER, NPHI>(s_rule, s_y, ny, X0, X1, X2, acc);
+            if constexpr (OP == 3) {
+                V3<T> cx[3];
+                tri_curls(X0, X1, X2, cx);
+                const T w = acc[0] * T(kInv4Pi);
+#pragma unroll
+                for (int a = 0; a < 3; ++a)
+#pragma unroll
+                    for (int b = 0; b < 3; ++b) atomicAdd(rows + a * nv + vx[b], dot(cy[a], cx[b]) * w);
+            } else {
+#pragma unroll
+                for (int a = 0; a < 3; ++a)
+#pragma unroll
+                    for (int b = 0; b < 3; ++b) atomicAdd(rows + a * nv + vx[b], acc[3 * a + b] * T(kInv4Pi));
+            }
         }
     }
     __syncthreads();
@@ -238,7 +365,7 @@ __global__ void __launch_bounds__(kSymThreads, 1)
     }
 }
 
-// FP32: a thread keeps one source face fx and meets the block's test faces.  The 7-point rule is its
+// FP32 (which meshes: launch_sym_pairs): a thread keeps one source face fx and meets the block's test faces.  The 7-point rule is its
 // centroid and two orbits s A_a of the corners A_a relative to the centroid (s = 1 - 3 q), so with
 // D the difference of the centroids
 //     R^2 = |D|^2 + 2 s D.A_a - 2 s' D.B_b + s^2 |A_a|^2 + s'^2 |B_b|^2 - 2 s s' A_a.B_b
@@ -763,24 +890,41 @@ int launch_laplace_sym(const T* verts, const int32_t* faces, int64_t nf, int lay
 // [row_begin, row_end), added to packed [nv, nv].
 constexpr int64_t kTightSmemMax = 160 * 1024;
 
-static int launch_sym_pairs(const double* verts, const int32_t* faces, int64_t nf, int64_t nv, int op, int64_t row_begin,
-                            int64_t row_end, double* packed, cudaStream_t s) {
-    const int64_t smem = 3 * nv * (int64_t)sizeof(double);
+template <typename T>
+static int launch_sym_rows(const T* verts, const int32_t* faces, int64_t nf, int64_t nv, int op, int64_t row_begin,
+                           int64_t row_end, T* packed, cudaStream_t s) {
     if (row_end - row_begin > 0x7fffffffLL) return set_error(MB_ERR_SIZE, "mesh too large for one launch");
-    const unsigned blocks = (unsigned)(row_end - row_begin);
     auto go = [&](auto kernel) -> int {
-        if (smem > 48 * 1024) {
-            const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return set_error(MB_ERR_CUDA, cudaGetErrorString(e));
-        }
-        kernel<<<blocks, kSymThreads, (size_t)smem, s>>>(verts, faces, nf, nv, row_begin, packed);
+        // the same limit for every mesh: it is the process's, and another thread may be between these two calls
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTightSmemMax);
+        if (e != cudaSuccess) return set_error(MB_ERR_CUDA, "%s", cudaGetErrorString(e));
+        kernel<<<(unsigned)(row_end - row_begin), kSymThreads, (size_t)(3 * nv) * sizeof(T), s>>>(verts, faces, nf, nv,
+                                                                                               row_begin, packed);
         return MB_OK;
     };
-    return op == 1 ? go(lap_sym_tight_kernel<1>) : op == 2 ? go(lap_sym_tight_kernel<2>) : go(lap_sym_tight_kernel<3>);
+    return op == 1 ? go(lap_sym_tight_kernel<T, 1>) : op == 2 ? go(lap_sym_tight_kernel<T, 2>) : go(lap_sym_tight_kernel<T, 3>);
+}
+
+static int launch_sym_pairs(const double* verts, const int32_t* faces, int64_t nf, int64_t nv, int op, int64_t row_begin,
+                            int64_t row_end, double* packed, cudaStream_t s) {
+    return launch_sym_rows(verts, faces, nf, nv, op, row_begin, row_end, packed, s);
+}
+
+// Whether a block per test face is the faster form for FP32: small meshes, where lap_sym_pairs_kernel's blocks are
+// few and its set-up and its close pairs, one after the other, are most of their time.  Measured (GB300, us, rows form /
+// pairs form, operators 1, 2, 3, without the pairs sharing a vertex where the rows are a window):
+//   416 faces 25 / 35, 27 / 36, 25 / 34; 680 39 / 46, 41 / 49, 31 / 44; 1300 90 / 94, 98 / 102, 68 / 90;
+//   1740 139 / 122, 150 / 131, 107 / 116; 2112 192 / 154, 207 / 166, 141 / 148; 2960 383 / 254, 397 / 267, 264 / 241;
+//   300 rows of 680 faces 18 / 28, 19 / 30, 17 / 27, of 2112 39 / 42, 41 / 45, 37 / 41, of 2960 52 / 52, 54 / 54, 49 / 50;
+//   100 rows of 874 17 / 19, 19 / 20, 17 / 19; 30 rows of 680 14 / 10, 15 / 10, 16 / 10, of 126 8 / 8, 8 / 10, 8 / 8.
+static bool rows_form(int64_t nf, int64_t rows, int op) {
+    if (nf < 150) return true;
+    return rows >= 64 && nf < 2600 && rows * nf < (op == 3 ? 6000000 : 2200000);
 }
 
 static int launch_sym_pairs(const float* verts, const int32_t* faces, int64_t nf, int64_t nv, int op, int64_t row_begin,
                             int64_t row_end, float* packed, cudaStream_t s) {
+    if (rows_form(nf, row_end - row_begin, op)) return launch_sym_rows(verts, faces, nf, nv, op, row_begin, row_end, packed, s);
     const int64_t gx = (nf + kPairThreads - 1) / kPairThreads, rows = row_end - row_begin;
     const int per = pair_rows(rows, gx);
     const int64_t gy = (rows + per - 1) / per;

@@ -122,6 +122,11 @@ int mb_face_geometry_f64(const double* verts, int64_t n_verts, const int32_t* fa
  * device memory. */
 int mb_index_range_i32(const int32_t* indices, int64_t count, int64_t limit, int32_t* work, int32_t* outside,
                        void* stream);
+/* The same for the vertex ids of n_faces faces, and how they are listed, for the calls that choose a kernel by it:
+ * face_order (host, two int32) = the mean number of different ids of ten consecutive faces, and of
+ * groups of eight ids among 32 consecutive faces (csrc/face_order.cuh).  work: 12 bytes of device memory. */
+int mb_index_range_order_i32(const int32_t* faces, int64_t n_faces, int64_t limit, int32_t* work, int32_t* outside,
+                             int32_t* face_order, void* stream);
 /* No counterpart in the reference (its scatter_add_ runs after the whole face-edge matrix
  * exists).  edge_rows [2 n_edges + 1] int32: for Z row m (edge m) the face-edge rows 3f + e
  * of its faces (smaller first; -1 for a missing second face); edge_rows[2 n_edges] = 1 when
@@ -646,6 +651,10 @@ int mb_pack_tight_f32(const float* m_real, const float* m_imag, const int32_t* f
                       int64_t n_verts, int order, float* packed, void* stream);
 int mb_pack_tight_f64(const double* m_real, const double* m_imag, const int32_t* faces,
                       int64_t n_faces, int64_t n_verts, int order, double* packed, void* stream);
+/* mb_pack_tight_f32 of real P1 panels, faster where face_order (host, from mb_index_range_order_i32, or NULL) says
+ * that neighbouring faces follow one another. */
+int mb_pack_tight_ordered_f32(const float* m_real, const int32_t* faces, int64_t n_faces, int64_t n_verts,
+                              const int32_t* face_order, float* packed, void* stream);
 
 /* Hypersingular operator, P1 Galerkin, for the Neumann and mixed branches of
  * MeshBEMSolver3d.solve (src/mesh_BEM/mesh_BEM_solver_3d.py:268-281, 306-341), which the

@@ -45,6 +45,7 @@ _SIGS = {
     "mb_face_geometry_f32": [_P, _I64, _P, _I64, _P, _P, _P],
     "mb_face_geometry_f64": [_P, _I64, _P, _I64, _P, _P, _P],
     "mb_index_range_i32": [_P, _I64, _I64, _P, _P, _P],
+    "mb_index_range_order_i32": [_P, _I64, _I64, _P, _P, _P, _P],
     "mb_mom_tiers_workspace_bytes": [_I64],
     "mb_mom_tier_tiles": [_I64, _P, _P, _P],
     "mb_mom_sym_zmat_rwg_pairs_c64": [_P, _I64, _P, _I64, _P, _I64, _D, _I, _P, _I64, _P, _P],
@@ -65,6 +66,7 @@ _SIGS = {
     "mb_laplace_panels_f64": [_P, _I64, _P, _I64, _P, _P, _P, _P, _P, _I, _I, _I, _D, _I64, _I64,
                               _P, _P, _P],
     "mb_pack_tight_f32": [_P, _P, _P, _I64, _I64, _I, _P, _P],
+    "mb_pack_tight_ordered_f32": [_P, _P, _I64, _I64, _P, _P, _P],
     "mb_pack_tight_f64": [_P, _P, _P, _I64, _I64, _I, _P, _P],
     "mb_panel_relation": [_P, _I64, _P, _P],
     "mb_mom_sym_zmat_rwg_c64": [_P, _I64, _P, _I64, _P, _I64, _D, _I64, _I64, _P, _P],

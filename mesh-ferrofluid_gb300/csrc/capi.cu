@@ -50,8 +50,9 @@ int launch_mom_interp(const T*, const int32_t*, const int32_t*, const T*, const 
 template <typename T>
 int launch_laplace_panels(const T*, const int32_t*, int64_t, const T*, const T*, const T*, const int*,
                           const uint8_t*, int, int, int, double, int64_t, int64_t, T*, T*, cudaStream_t);
+struct FaceOrder;
 template <typename T>
-int launch_pack_tight(const T*, const T*, const int32_t*, int64_t, int64_t, int, T*, cudaStream_t);
+int launch_pack_tight(const T*, const T*, const int32_t*, int64_t, int64_t, int, const FaceOrder*, T*, cudaStream_t);
 template <typename T>
 int launch_hypersingular(const T*, const int32_t*, int64_t, const T*, T*, cudaStream_t);
 int64_t near_pairs_workspace_bytes(int64_t nf, int64_t nv);
@@ -91,7 +92,8 @@ int gnn_adam(float* w, float* m1, float* m2, const float* g, int64_t count, floa
 template <typename T>
 int launch_face_geometry(const T* verts, int64_t nv, const int32_t* faces, int64_t nf, T* areas, T* normals,
                          cudaStream_t s);
-int index_range(const int32_t* idx, int64_t count, int64_t limit, int32_t* work, int32_t* outside, cudaStream_t s);
+int index_range(const int32_t* idx, int64_t count, int64_t limit, int32_t* work, int32_t* outside, FaceOrder* order,
+                cudaStream_t s);
 int launch_edge_rows(const int32_t* fei, int64_t nf, int64_t n_edges, int32_t* er, cudaStream_t s);
 bool mom_tier_rule(int nx, int ny);
 void mom_tier_tiles(int64_t pairs, int* rows, int* tp, int* tq);
@@ -312,7 +314,7 @@ MB_FACE_GEOMETRY(f64, double)
 int mb_index_range_i32(const int32_t* indices, int64_t count, int64_t limit, int32_t* work, int32_t* outside,
                        void* stream) {
     MB_REQUIRE(count >= 0 && outside && (count == 0 || (indices && work)), "null pointer argument or negative count");
-    return index_range(indices, count, limit, work, outside, as_stream(stream));
+    return index_range(indices, count, limit, work, outside, nullptr, as_stream(stream));
 }
 
 int64_t mb_mom_tiers_workspace_bytes(int64_t n_faces) { return n_faces > 0 ? 128 * n_faces : 0; }
@@ -527,12 +529,29 @@ MB_LAP(f64, double)
         if (n_faces == 0) return MB_OK;                                                               \
         MB_REQUIRE(m_real && faces && packed, "null pointer argument");                               \
         MB_REQUIRE(order == 0 || order == 1, "order must be 0 or 1");                                 \
-        return launch_pack_tight<T>(m_real, m_imag, faces, n_faces, n_verts, order, packed,           \
+        return launch_pack_tight<T>(m_real, m_imag, faces, n_faces, n_verts, order, nullptr, packed,  \
                                     as_stream(stream));                                               \
     }
 MB_PACK(f32, float)
 MB_PACK(f64, double)
 #undef MB_PACK
+
+int mb_index_range_order_i32(const int32_t* faces, int64_t n_faces, int64_t limit, int32_t* work, int32_t* outside,
+                             int32_t* face_order, void* stream) {
+    MB_REQUIRE(n_faces >= 0 && outside && face_order && (n_faces == 0 || (faces && work)),
+               "null pointer argument or negative count");
+    return index_range(faces, 3 * n_faces, limit, work, outside, reinterpret_cast<FaceOrder*>(face_order),
+                       as_stream(stream));
+}
+
+int mb_pack_tight_ordered_f32(const float* m_real, const int32_t* faces, int64_t n_faces, int64_t n_verts,
+                              const int32_t* face_order, float* packed, void* stream) {
+    MB_REQUIRE(n_faces >= 0 && n_verts >= 0, "bad sizes");
+    if (n_faces == 0) return MB_OK;
+    MB_REQUIRE(m_real && faces && packed, "null pointer argument");
+    return launch_pack_tight<float>(m_real, nullptr, faces, n_faces, n_verts, 1,
+                                    reinterpret_cast<const FaceOrder*>(face_order), packed, as_stream(stream));
+}
 
 #define MB_HYP(SFX, T)                                                                                \
     int mb_laplace_hypersingular_##SFX(const T* verts, int64_t n_verts, const int32_t* faces,           \

@@ -18,6 +18,7 @@
 #include <stdint.h>
 
 #include "common.cuh"
+#include "face_order.cuh"
 #include "packed.cuh"
 #include "vertex_slots.cuh"
 
@@ -925,8 +926,11 @@ int launch_pack_rows(const T* m, const T* verts, const int32_t* faces, int64_t n
 // vertex_slots.cuh.  A warp's 32 panels of a row (1152 consecutive bytes) come by 4-byte asynchronous
 // copies (any alignment: a row starts at 36 F fy bytes), kPackStages - 1 rows ahead, into the
 // warp's own buffer, whose 9-float stride meets no bank twice.
-// Bound: HBM, each panel read once.  Measured (GB300, 5120 faces, 944 MB of panels): 680 us with the rows in
-// shared memory (the compare-and-swap loop of shared additions).
+// Bound: HBM, each panel read once, or, where the faces and vertices are not listed neighbour by neighbour, the reductions
+// (9 instead of 3 per pair, one 32-byte sector each). Measured (GB300, us, pack_rows_kernel / this): subdivided
+// sphere 5120 faces 614 / 285, 20480 27.1 / 4.3 ms; strips along the vertex ids 2960 124 / 98, 4048 409 / 166, 7080 1141 / 479;
+// strips across them 2112 55 / 122, 3444 189 / 270, 4704 492 / 510, 8064 4880 / 1455; any order 1280 35 / 78, 5120
+// 587 / 1188; below 2500 faces at most 15 us apart in this kernel's favour. So: from 2500 faces on, by the order.
 constexpr int kPackStages = 3;
 constexpr int kPackSmem = kPairSumBytes + kPackStages * kPairThreads * 9 * (int)sizeof(float);
 
@@ -981,28 +985,29 @@ __global__ void __launch_bounds__(kPairThreads)
     if (q < nf) flush_sums(s_slots, col, nv, s_sum, packed);
 }
 
-// a float P1 packing; 0: not one
-static int pack_pairs(const double*, const double*, const int32_t*, int64_t, int64_t, int, double*, cudaStream_t) {
-    return 0;
-}
-static int pack_pairs(const float* m_r, const float* m_i, const int32_t* faces, int64_t nf, int64_t nv, int order,
-                      float* packed, cudaStream_t stream) {
+static bool pack_pairs(const double*, const int32_t*, int64_t, int64_t, double*, cudaStream_t) { return false; }
+static bool pack_pairs(const float* m, const int32_t* faces, int64_t nf, int64_t nv, float* packed, cudaStream_t stream) {
     const int64_t gx = (nf + kPairThreads - 1) / kPairThreads;
     const int per = pair_rows(nf, gx);
     const int64_t gy = (nf + per - 1) / per;
-    if (m_i != nullptr || order != 1 || gy > 65535) return 0;
-    pack_pairs_kernel<<<dim3((unsigned)gx, (unsigned)gy), kPairThreads, kPackSmem, stream>>>(m_r, faces, nf, nv, per,
+    if (gy > 65535) return false;
+    pack_pairs_kernel<<<dim3((unsigned)gx, (unsigned)gy), kPairThreads, kPackSmem, stream>>>(m, faces, nf, nv, per,
                                                                                              packed);
-    return 1;
+    return true;
 }
 
+// faces_order (host, may be null): the mesh's FaceOrder.  P1 real panels go by rows; FP32 ones by pairs of faces from 2500
+// faces on where the order is known and suits, and where the rows do not fit shared memory.
 template <typename T>
 int launch_pack_tight(const T* m_r, const T* m_i, const int32_t* faces, int64_t nf, int64_t nv,
-                      int order, T* packed, cudaStream_t stream) {
+                      int order, const FaceOrder* faces_order, T* packed, cudaStream_t stream) {
     if (nf <= 0) return MB_OK;
-    if (pack_pairs(m_r, m_i, faces, nf, nv, order, packed, stream)) return check_launch("pack_pairs");
-    if (m_i == nullptr && order == 1 && 3 * nv * (int64_t)sizeof(T) <= kPackRowSmemMax)
-        return launch_pack_rows<T, false>(m_r, nullptr, faces, nf, nv, packed, stream);
+    if (m_i == nullptr && order == 1) {
+        const bool rows = 3 * nv * (int64_t)sizeof(T) <= kPackRowSmemMax;
+        const bool by_order = nf >= 2500 && faces_order && faces_order->ids <= 20 && faces_order->sectors <= 32;
+        if ((by_order || !rows) && pack_pairs(m_r, faces, nf, nv, packed, stream)) return check_launch("pack_pairs");
+        if (rows) return launch_pack_rows<T, false>(m_r, nullptr, faces, nf, nv, packed, stream);
+    }
     const int threads = 256;
     const int64_t blocks = (nf * nf + threads - 1) / threads;
     if (blocks > 0x7fffffffLL) return set_error(MB_ERR_SIZE, "mesh too large for one launch");
@@ -1011,9 +1016,9 @@ int launch_pack_tight(const T* m_r, const T* m_i, const int32_t* faces, int64_t 
     return check_launch("pack_tight");
 }
 template int launch_pack_tight<float>(const float*, const float*, const int32_t*, int64_t, int64_t, int,
-                                      float*, cudaStream_t);
+                                      const FaceOrder*, float*, cudaStream_t);
 template int launch_pack_tight<double>(const double*, const double*, const int32_t*, int64_t, int64_t,
-                                       int, double*, cudaStream_t);
+                                       int, const FaceOrder*, double*, cudaStream_t);
 
 // Hypersingular operator of the Laplace problem, P1 Galerkin, by Maue's integration by parts
 // (J.-C. Nedelec 1982; O. Steinbach, Numerical Approximation Methods for Elliptic Boundary

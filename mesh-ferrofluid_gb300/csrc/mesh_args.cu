@@ -6,6 +6,7 @@
 // one index array four launches and two waits; here one launch each and one wait.  A CFIE assembly with
 // one excitation on 80 faces: 564 -> 171 us.
 #include "common.cuh"
+#include "face_order.cuh"
 
 namespace mb {
 
@@ -44,6 +45,12 @@ __global__ void __launch_bounds__(256) index_range_kernel(const int32_t* __restr
     if (bad) *outside = 1;  // all writers store the same value
 }
 
+__global__ void __launch_bounds__(32 * kOrderSamples) face_order_kernel(const int32_t* __restrict__ ids, int64_t nf,
+                                                                       FaceOrder* __restrict__ out) {
+    const FaceOrder o = face_order(ids, nf);
+    if (threadIdx.x == 0) *out = o;
+}
+
 }  // namespace
 
 template <typename T>
@@ -57,20 +64,29 @@ template int launch_face_geometry<float>(const float*, int64_t, const int32_t*, 
 template int launch_face_geometry<double>(const double*, int64_t, const int32_t*, int64_t, double*, double*,
                                           cudaStream_t);
 
-// *outside: 1 if an index is not in [0, limit), else 0 (waits for the stream).  work: 4 bytes on the device.
-int index_range(const int32_t* idx, int64_t count, int64_t limit, int32_t* work, int32_t* outside, cudaStream_t s) {
+// *outside: 1 if an index is not in [0, limit), else 0 (waits for the stream).  work: 4 bytes on the device.  With order
+// (count = 3 per face; work: 12 bytes) the order of the faces, too, by the same wait.
+int index_range(const int32_t* idx, int64_t count, int64_t limit, int32_t* work, int32_t* outside, FaceOrder* order,
+                cudaStream_t s) {
     *outside = 0;
+    if (order) *order = FaceOrder{0, 0};
     if (count <= 0) return MB_OK;
+    int32_t got[3] = {0, 0, 0};
     cudaError_t e = cudaMemsetAsync(work, 0, sizeof(int32_t), s);
     if (e == cudaSuccess) {
         // four indices a thread; at most two blocks an SM
         const int64_t blocks = (count + 1023) / 1024;
         index_range_kernel<<<(unsigned)(blocks < 304 ? blocks : 304), 256, 0, s>>>(idx, count, limit, work);
+        if (order)
+            face_order_kernel<<<1, 32 * kOrderSamples, 0, s>>>(idx, count / 3, reinterpret_cast<FaceOrder*>(work + 1));
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(outside, work, sizeof(int32_t), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(got, work, sizeof(int32_t) * (order ? 3 : 1), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return set_error(MB_ERR_CUDA, "index range: %s", cudaGetErrorString(e));
+    *outside = got[0];
+    if (order) *order = FaceOrder{got[1], got[2]};
     return MB_OK;
 }
 

@@ -349,17 +349,22 @@ def shape_function(dim: int, order_type: int, r1: torch.Tensor, r2: torch.Tensor
     raise RuntimeError("We only accept 2D/3D for calculating shape function")
 
 
-def indices_outside(idx: torch.Tensor, limit: int) -> bool:
-    """Whether an index lies outside [0, limit): one kernel and one sync for contiguous int32 CUDA tensors."""
+def indices_outside(idx: torch.Tensor, limit: int, face_order=None) -> bool:
+    """Whether an index lies outside [0, limit): one kernel and one sync for contiguous int32 CUDA tensors.
+    ``face_order`` (two C int32; idx a contiguous int32 CUDA [F, 3]) receives how the faces are listed, by the same sync."""
     if idx.numel() == 0:
         return False
     if not (idx.is_cuda and idx.dtype == torch.int32 and idx.is_contiguous()):
         lo, hi = torch.aminmax(idx)
         return int(lo) < 0 or int(hi) >= limit
-    work = torch.empty(1, dtype=torch.int32, device=idx.device)
+    work = torch.empty(3, dtype=torch.int32, device=idx.device)
     bad = ctypes.c_int32(0)
-    _lib.call("mb_index_range_i32", _lib.ptr(idx), idx.numel(), int(limit), _lib.ptr(work), ctypes.byref(bad),
-              _lib.stream_of(idx))
+    if face_order is None:
+        _lib.call("mb_index_range_i32", _lib.ptr(idx), idx.numel(), int(limit), _lib.ptr(work), ctypes.byref(bad),
+                  _lib.stream_of(idx))
+    else:
+        _lib.call("mb_index_range_order_i32", _lib.ptr(idx), idx.shape[0], int(limit), _lib.ptr(work),
+                  ctypes.byref(bad), ctypes.byref(face_order), _lib.stream_of(idx))
     return bool(bad.value)
 
 
@@ -369,7 +374,9 @@ def pack_matrix_tight(order_type: int, unpacked_matrix: torch.Tensor, verts: tor
     n_verts = verts.shape[-2]
     faces = _lib.check_tensor(faces.contiguous(), "faces", dtype=torch.int32, ndim=2)
     nf = faces.shape[0]
-    if nf and indices_outside(faces, n_verts):
+    # the choice of kernel for a large mesh needs the order of its faces (smaller ones go by rows in any order)
+    order = (ctypes.c_int32 * 2)() if nf >= 2500 else None
+    if nf and indices_outside(faces, n_verts, order):
         raise ValueError(f"faces reference vertex ids outside [0, {n_verts})")
     m = unpacked_matrix.contiguous()
     if m.shape[:2] != (nf, nf) or m.shape[2] != m.shape[3] or m.shape[2] not in (1, 3):
@@ -385,6 +392,10 @@ def pack_matrix_tight(order_type: int, unpacked_matrix: torch.Tensor, verts: tor
         base = m.dtype
         mr, mi = m, None
         out = torch.zeros((n_verts, n_verts), dtype=base, device=m.device)
+    if order is not None and base == torch.float32 and mi is None and int(order_type) == int(OrderType.LINEAR):
+        _lib.call("mb_pack_tight_ordered_f32", _lib.ptr(mr), _lib.ptr(faces), nf, n_verts, ctypes.byref(order),
+                  _lib.ptr(out), _lib.stream_of(m))
+        return out
     _lib.call(f"mb_pack_tight_{_lib.sfx(base)}", _lib.ptr(mr), _lib.ptr(mi), _lib.ptr(faces), nf,
               n_verts, int(order_type), _lib.ptr(out), _lib.stream_of(m))
     return torch.view_as_complex(out) if mi is not None else out

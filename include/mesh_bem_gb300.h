@@ -707,6 +707,11 @@ int mb_laplace_sym_tight_f32(const float* verts, int64_t n_verts, const int32_t*
 int mb_laplace_sym_tight_f64(const double* verts, int64_t n_verts, const int32_t* faces, int64_t n_faces,
                              int op, const int32_t* near_pairs, int64_t n_near, int64_t row_begin,
                              int64_t row_end, double* packed, void* stream);
+/* mb_laplace_sym_tight_f32, faster on large meshes whose neighbouring faces follow one another (looked at on the
+ * device: csrc/face_order.cuh).  work: 8 bytes of device memory. */
+int mb_laplace_sym_tight_ordered_f32(const float* verts, int64_t n_verts, const int32_t* faces, int64_t n_faces,
+                                     int op, const int32_t* near_pairs, int64_t n_near, int64_t row_begin,
+                                     int64_t row_end, int32_t* work, float* packed, void* stream);
 
 /* Single-layer collocation system at face centroids (the Laplace form of the large sphere
  * solve; no counterpart in the reference): out[i - row_begin, j] = int_{T_j} 1/(4 pi

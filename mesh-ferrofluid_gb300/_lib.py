@@ -82,6 +82,7 @@ _SIGS = {
     "mb_laplace_sym_f32": [_P, _I64, _P, _I64, _I, _I, _P, _I64, _I64, _I64, _P, _P],
     "mb_laplace_sym_f64": [_P, _I64, _P, _I64, _I, _I, _P, _I64, _I64, _I64, _P, _P],
     "mb_laplace_sym_tight_f32": [_P, _I64, _P, _I64, _I, _P, _I64, _I64, _I64, _P, _P],
+    "mb_laplace_sym_tight_ordered_f32": [_P, _I64, _P, _I64, _I, _P, _I64, _I64, _I64, _P, _P, _P],
     "mb_laplace_sym_tight_f64": [_P, _I64, _P, _I64, _I, _P, _I64, _I64, _I64, _P, _P],
     "mb_laplace_colloc_sl_f32": [_P, _I64, _P, _I64, _P, _I64, _I64, _I64, _P, _P],
     "mb_laplace_colloc_sl_f64": [_P, _I64, _P, _I64, _P, _I64, _I64, _I64, _P, _P],

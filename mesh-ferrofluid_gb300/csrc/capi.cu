@@ -66,7 +66,7 @@ int launch_laplace_sym(const T*, const int32_t*, int64_t, int, int, const int32_
                        cudaStream_t);
 template <typename T>
 int launch_laplace_sym_tight(const T*, const int32_t*, int64_t, int64_t, int, const int32_t*, int64_t, int64_t,
-                             int64_t, T*, cudaStream_t);
+                             int64_t, FaceOrder*, T*, cudaStream_t);
 template <typename T>
 int launch_laplace_colloc_sl(const T*, const int32_t*, int64_t, const int32_t*, int64_t, int64_t, int64_t, T*,
                              cudaStream_t);
@@ -638,11 +638,22 @@ MB_LSYM(f64, double)
         MB_REQUIRE(verts && faces && packed && (near_pairs || n_near == 0), "null pointer argument"); \
         MB_REQUIRE(0 <= row_begin && row_begin <= row_end && row_end <= n_faces, "bad row range");    \
         return launch_laplace_sym_tight<T>(verts, faces, n_faces, n_verts, op, near_pairs, n_near,    \
-                                           row_begin, row_end, packed, as_stream(stream));            \
+                                           row_begin, row_end, nullptr, packed, as_stream(stream));   \
     }
 MB_LSYMT(f32, float)
 MB_LSYMT(f64, double)
 #undef MB_LSYMT
+
+int mb_laplace_sym_tight_ordered_f32(const float* verts, int64_t n_verts, const int32_t* faces, int64_t n_faces, int op,
+                                     const int32_t* near_pairs, int64_t n_near, int64_t row_begin, int64_t row_end,
+                                     int32_t* work, float* packed, void* stream) {
+    MB_REQUIRE(n_faces >= 0 && n_verts >= 0 && n_near >= 0, "bad sizes");
+    if (n_faces == 0) return MB_OK;
+    MB_REQUIRE(verts && faces && packed && work && (near_pairs || n_near == 0), "null pointer argument");
+    MB_REQUIRE(0 <= row_begin && row_begin <= row_end && row_end <= n_faces, "bad row range");
+    return launch_laplace_sym_tight<float>(verts, faces, n_faces, n_verts, op, near_pairs, n_near, row_begin, row_end,
+                                           reinterpret_cast<FaceOrder*>(work), packed, as_stream(stream));
+}
 
 #define MB_SYM(SFX, T)                                                                                \
     int mb_mom_sym_zmat_rwg_##SFX(const T* verts, int64_t n_verts, const int32_t* faces, int64_t n_faces,   \

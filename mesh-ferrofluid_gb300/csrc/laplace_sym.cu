@@ -25,6 +25,7 @@
 
 #include "closed_form.cuh"
 #include "common.cuh"
+#include "face_order.cuh"
 #include "packed.cuh"
 #include "vertex_slots.cuh"
 
@@ -244,6 +245,17 @@ __device__ __forceinline__ void tri_curls(const V3<T>& p0, const V3<T>& p1, cons
     c[2] = inv2a * (p0 - p1);
 }
 
+// Ten consecutive faces with more vertices than this (face_order.cuh) are not listed neighbour by neighbour.  5120
+// faces, us, operators 1, 2, 3, a block per face / groups of faces: 14 vertices 1026 / 494, 1064 / 573, 801 / 429; 17: 1030 / 650,
+// 1068 / 675, 806 / 626; 23: 1036 / 893, 1076 / 902, 818 / 877; 30: 1036 / 1171, 1074 / 1173, 815 / 1158.
+constexpr int kOrderIds = 20;
+
+__global__ void __launch_bounds__(32 * kOrderSamples) lap_face_order_kernel(const int32_t* __restrict__ faces, int64_t nf,
+                                                                           FaceOrder* __restrict__ out) {
+    const FaceOrder o = face_order(faces, nf);
+    if (threadIdx.x == 0) *out = o;
+}
+
 // Packed operators [V, V] without the [F, F, 3, 3] panels: OP 1 single layer, 2 double layer
 // (P1 x P1), 3 hypersingular (Maue: curl phi_a(fy) . curl phi_b(fx) times the P0 single
 // layer).  One block per test face fy sweeps every source face fx, accumulates the three
@@ -253,7 +265,9 @@ __device__ __forceinline__ void tri_curls(const V3<T>& p0, const V3<T>& p1, cons
 template <typename T, int OP>
 __global__ void __launch_bounds__(kSymThreads, sizeof(T) == 4 ? (OP == 3 ? 6 : 4) : 1)
     lap_sym_tight_kernel(const T* __restrict__ verts, const int32_t* __restrict__ faces, int64_t nf, int64_t nv,
-                         int64_t row_begin, T* __restrict__ packed) {
+                         int64_t row_begin, const FaceOrder* __restrict__ order, T* __restrict__ packed) {
+    if constexpr (sizeof(T) == 4)
+        if (order && order->ids <= kOrderIds) return;  // lap_sym_pairs_kernel's
     constexpr int LAYER = OP == 2 ? 2 : 1;
     constexpr int NPHI = OP == 3 ? 1 : 3;
     __shared__ T s_rule[7][4];
@@ -444,7 +458,9 @@ __device__ void close_pair_entries(const float* __restrict__ verts, const int32_
 template <int OP>
 __global__ void __launch_bounds__(kPairThreads, 5)
     lap_sym_pairs_kernel(const float* __restrict__ verts, const int32_t* __restrict__ faces, int64_t nf, int64_t nv,
-                         int64_t row_begin, int64_t row_end, int rows_per_block, float* __restrict__ packed) {
+                         int64_t row_begin, int64_t row_end, int rows_per_block, const FaceOrder* __restrict__ order,
+                         float* __restrict__ packed) {
+    if (order && order->ids > kOrderIds) return;  // lap_sym_tight_kernel's
     constexpr float s1 = (float)(1.0 - 3.0 * 0.10128650732345634), s2 = (float)(1.0 - 3.0 * 0.47014206410511509);
     constexpr float w0 = 0.225f, w1 = 0.12593918054482715f, w2 = 0.13239415278850619f;
     constexpr float a1 = (1.f - s1) / 3.f, a2 = (1.f - s2) / 3.f;
@@ -887,27 +903,28 @@ int launch_laplace_sym(const T* verts, const int32_t* faces, int64_t nf, int lay
     return check_launch("laplace_sym");
 }
 // Packed operators (op 1 single layer, 2 double layer, 3 hypersingular) for test rows
-// [row_begin, row_end), added to packed [nv, nv].
+// [row_begin, row_end), added to packed [nv, nv].  order: 8 bytes of device memory for the FP32 kernels' choice, or null
+// (many rows of a large mesh then go by a block per face).
 constexpr int64_t kTightSmemMax = 160 * 1024;
 
 template <typename T>
 static int launch_sym_rows(const T* verts, const int32_t* faces, int64_t nf, int64_t nv, int op, int64_t row_begin,
-                           int64_t row_end, T* packed, cudaStream_t s) {
+                           int64_t row_end, const FaceOrder* order, T* packed, cudaStream_t s) {
     if (row_end - row_begin > 0x7fffffffLL) return set_error(MB_ERR_SIZE, "mesh too large for one launch");
     auto go = [&](auto kernel) -> int {
         // the same limit for every mesh: it is the process's, and another thread may be between these two calls
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTightSmemMax);
         if (e != cudaSuccess) return set_error(MB_ERR_CUDA, "%s", cudaGetErrorString(e));
         kernel<<<(unsigned)(row_end - row_begin), kSymThreads, (size_t)(3 * nv) * sizeof(T), s>>>(verts, faces, nf, nv,
-                                                                                               row_begin, packed);
+                                                                                               row_begin, order, packed);
         return MB_OK;
     };
     return op == 1 ? go(lap_sym_tight_kernel<T, 1>) : op == 2 ? go(lap_sym_tight_kernel<T, 2>) : go(lap_sym_tight_kernel<T, 3>);
 }
 
 static int launch_sym_pairs(const double* verts, const int32_t* faces, int64_t nf, int64_t nv, int op, int64_t row_begin,
-                            int64_t row_end, double* packed, cudaStream_t s) {
-    return launch_sym_rows(verts, faces, nf, nv, op, row_begin, row_end, packed, s);
+                            int64_t row_end, FaceOrder*, double* packed, cudaStream_t s) {
+    return launch_sym_rows(verts, faces, nf, nv, op, row_begin, row_end, nullptr, packed, s);
 }
 
 // Whether a block per test face is the faster form for FP32: small meshes, where lap_sym_pairs_kernel's blocks are
@@ -915,23 +932,32 @@ static int launch_sym_pairs(const double* verts, const int32_t* faces, int64_t n
 // pairs form, operators 1, 2, 3, without the pairs sharing a vertex where the rows are a window):
 //   416 faces 25 / 35, 27 / 36, 25 / 34; 680 39 / 46, 41 / 49, 31 / 44; 1300 90 / 94, 98 / 102, 68 / 90;
 //   1740 139 / 122, 150 / 131, 107 / 116; 2112 192 / 154, 207 / 166, 141 / 148; 2960 383 / 254, 397 / 267, 264 / 241;
-//   300 rows of 680 faces 18 / 28, 19 / 30, 17 / 27, of 2112 39 / 42, 41 / 45, 37 / 41, of 2960 52 / 52, 54 / 54, 49 / 50;
-//   100 rows of 874 17 / 19, 19 / 20, 17 / 19; 30 rows of 680 14 / 10, 15 / 10, 16 / 10, of 126 8 / 8, 8 / 10, 8 / 8.
+//   300 rows of 680 faces 18 / 28, 19 / 30, 17 / 27, of 2112 39 / 42, 41 / 45, 37 / 41, of 2960 52 / 52, 54 / 54, 49 / 50, of
+//   4048 80 / 56, 82 / 59, 68 / 53; 100 rows of 874 17 / 19, 19 / 20, 17 / 19; 30 rows of 680 14 / 10, 15 / 10, 16 / 10, of
+//   126 8 / 8, 8 / 10, 8 / 8.
+// Where the pairs form may run, looking at the faces' order and the other form's empty launch cost it 8 to 15 us more.
 static bool rows_form(int64_t nf, int64_t rows, int op) {
     if (nf < 150) return true;
-    return rows >= 64 && nf < 2600 && rows * nf < (op == 3 ? 6000000 : 2200000);
+    if (rows < 64 || nf >= 3600) return false;
+    return rows < 512 || (nf < 2600 && rows * nf < (op == 3 ? 6000000 : 2200000));
 }
 
 static int launch_sym_pairs(const float* verts, const int32_t* faces, int64_t nf, int64_t nv, int op, int64_t row_begin,
-                            int64_t row_end, float* packed, cudaStream_t s) {
-    if (rows_form(nf, row_end - row_begin, op)) return launch_sym_rows(verts, faces, nf, nv, op, row_begin, row_end, packed, s);
+                            int64_t row_end, FaceOrder* order, float* packed, cudaStream_t s) {
     const int64_t gx = (nf + kPairThreads - 1) / kPairThreads, rows = row_end - row_begin;
+    // few rows: groups of faces in any order (each row form's block would sweep the mesh for one row)
+    if (nf >= 150 && rows < 64) order = nullptr;
+    else if (rows_form(nf, rows, op) || !order) return launch_sym_rows(verts, faces, nf, nv, op, row_begin, row_end, nullptr, packed, s);
     const int per = pair_rows(rows, gx);
     const int64_t gy = (rows + per - 1) / per;
     if (gx > 0x7fffffffLL || gy > 65535) return set_error(MB_ERR_SIZE, "mesh too large for one launch");
+    if (order) {
+        lap_face_order_kernel<<<1, 32 * kOrderSamples, 0, s>>>(faces, nf, order);
+        if (int rc = launch_sym_rows(verts, faces, nf, nv, op, row_begin, row_end, order, packed, s)) return rc;
+    }
     auto go = [&](auto kernel) -> int {
         kernel<<<dim3((unsigned)gx, (unsigned)gy), kPairThreads, kPairSumBytes, s>>>(verts, faces, nf, nv, row_begin,
-                                                                                     row_end, per, packed);
+                                                                                     row_end, per, order, packed);
         return MB_OK;
     };
     return op == 1 ? go(lap_sym_pairs_kernel<1>) : op == 2 ? go(lap_sym_pairs_kernel<2>) : go(lap_sym_pairs_kernel<3>);
@@ -939,12 +965,12 @@ static int launch_sym_pairs(const float* verts, const int32_t* faces, int64_t nf
 
 template <typename T>
 int launch_laplace_sym_tight(const T* verts, const int32_t* faces, int64_t nf, int64_t nv, int op,
-                             const int32_t* pairs, int64_t n_pairs, int64_t row_begin, int64_t row_end, T* packed,
-                             cudaStream_t s) {
+                             const int32_t* pairs, int64_t n_pairs, int64_t row_begin, int64_t row_end,
+                             FaceOrder* order, T* packed, cudaStream_t s) {
     if (nf <= 0 || row_end <= row_begin) return MB_OK;
     if (op < 1 || op > 3) return set_error(MB_ERR_ARG, "op must be 1 (single), 2 (double) or 3 (hypersingular)");
     if (3 * nv * (int64_t)sizeof(T) > kTightSmemMax) return set_error(MB_ERR_SIZE, "too many vertices for the packed assembly");
-    if (int rc = launch_sym_pairs(verts, faces, nf, nv, op, row_begin, row_end, packed, s)) return rc;
+    if (int rc = launch_sym_pairs(verts, faces, nf, nv, op, row_begin, row_end, order, packed, s)) return rc;
     if (n_pairs > 0) {
         const int64_t near_blocks = (n_pairs * kNearLanes + 127) / 128;
         if (near_blocks > 0x7fffffffLL) return set_error(MB_ERR_SIZE, "near-pair list too long for one launch");
@@ -955,9 +981,9 @@ int launch_laplace_sym_tight(const T* verts, const int32_t* faces, int64_t nf, i
     return check_launch("laplace_sym_tight");
 }
 template int launch_laplace_sym_tight<float>(const float*, const int32_t*, int64_t, int64_t, int, const int32_t*,
-                                             int64_t, int64_t, int64_t, float*, cudaStream_t);
-template int launch_laplace_sym_tight<double>(const double*, const int32_t*, int64_t, int64_t, int,
-                                              const int32_t*, int64_t, int64_t, int64_t, double*, cudaStream_t);
+                                             int64_t, int64_t, int64_t, FaceOrder*, float*, cudaStream_t);
+template int launch_laplace_sym_tight<double>(const double*, const int32_t*, int64_t, int64_t, int, const int32_t*,
+                                              int64_t, int64_t, int64_t, FaceOrder*, double*, cudaStream_t);
 
 template int launch_laplace_sym<float>(const float*, const int32_t*, int64_t, int, int, const int32_t*, int64_t,
                                        int64_t, int64_t, float*, cudaStream_t);

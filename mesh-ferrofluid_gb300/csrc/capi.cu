@@ -317,7 +317,7 @@ int mb_index_range_i32(const int32_t* indices, int64_t count, int64_t limit, int
     return index_range(indices, count, limit, work, outside, nullptr, as_stream(stream));
 }
 
-int64_t mb_mom_tiers_workspace_bytes(int64_t n_faces) { return n_faces > 0 ? 128 * n_faces : 0; }
+int64_t mb_mom_tiers_workspace_bytes(int64_t n_faces) { return n_faces > 0 ? 128 * n_faces + 16 : 0; }
 
 int mb_mom_tier_tiles(int64_t face_pairs, int32_t* rows, int32_t* tp, int32_t* tq) {
     MB_REQUIRE(face_pairs >= 0 && rows && tp && tq, "null pointer argument or negative count");

@@ -317,7 +317,7 @@ __device__ __forceinline__ void sym_regular_pair<float>(const float* __restrict_
 // Single-mesh float separated pairs: a block owns kSymRows test faces (their vertices, RWG
 // constants and edge ids staged in shared memory) and 128 source faces; each thread sets up
 // its source face once and evaluates it against every test face of the block.
-// REST: only the pairs that sym_pairs_kernel leaves (rec: the face records).
+// REST: only the pairs that sym_pairs_kernel leaves (rec: the face records; all of them where *form is 0).
 constexpr int kSymRows = 32;
 
 // The test faces p0 .. p0 + nr - 1 (bits) that sym_pairs_kernel leaves with source face q.  Most threads need one
@@ -363,7 +363,8 @@ __global__ void __launch_bounds__(128) mom_sym_regular_rows_kernel(const float* 
                                                                    int64_t n_edges, float k, int64_t nf,
                                                                    int64_t p_begin, int64_t p_end,
                                                                    float* __restrict__ z,
-                                                                   const float* __restrict__ rec) {
+                                                                   const float* __restrict__ rec,
+                                                                   const int* __restrict__ form) {
     __shared__ float4 s_c[REST ? kSymRows : 1];
     __shared__ float s_b[7][4];
     __shared__ float s_A[kSymRows][9], s_cm[kSymRows][3], s_ap[kSymRows];
@@ -371,7 +372,7 @@ __global__ void __launch_bounds__(128) mom_sym_regular_rows_kernel(const float* 
     const int64_t p0 = p_begin + (int64_t)blockIdx.y * kSymRows;
     const int64_t q = (int64_t)blockIdx.x * 128 + threadIdx.x;
     uint32_t mine = 0xffffffffu;  // test faces left to this kernel
-    if constexpr (REST) mine = rest_faces(rec, p0, (int)min((int64_t)kSymRows, p_end - p0), q, nf, k, s_c);
+    if (REST && *form) mine = rest_faces(rec, p0, (int)min((int64_t)kSymRows, p_end - p0), q, nf, k, s_c);
     if (REST && !__syncthreads_or(mine != 0)) return;
     if (threadIdx.x < 28) s_b[threadIdx.x / 4][threadIdx.x % 4] = (float)c_d7[threadIdx.x / 4][threadIdx.x % 4];
     if (threadIdx.x < kSymRows && p0 + threadIdx.x < p_end) {
@@ -938,7 +939,7 @@ int launch_mom_sym_regular(const T* verts, const int32_t* faces, const int32_t* 
         const int64_t py = (p_end - p_begin + kSymRows - 1) / kSymRows;
         if (q_blocks > 0x7fffffffLL || py > 65535) return set_error(MB_ERR_SIZE, "mesh too large for one launch");
         mom_sym_regular_rows_kernel<false><<<dim3((unsigned)q_blocks, (unsigned)py), 128, 0, s>>>(
-            verts, faces, fei, n_edges, (float)k, nf, p_begin, p_end, z, nullptr);
+            verts, faces, fei, n_edges, (float)k, nf, p_begin, p_end, z, nullptr, nullptr);
         return check_launch("mom_sym_regular");
     }
     const int64_t blocks = (p_end - p_begin) * q_blocks;
@@ -950,11 +951,11 @@ int launch_mom_sym_regular(const T* verts, const int32_t* faces, const int32_t* 
 
 // The separated pairs that sym_pairs_kernel leaves, all test faces.
 int launch_mom_sym_rest(const float* verts, const int32_t* faces, const int32_t* fei, int64_t n_edges, double k, int64_t nf,
-                        const float* rec, float* z, cudaStream_t s) {
+                        const float* rec, const int* form, float* z, cudaStream_t s) {
     const int64_t q_blocks = (nf + 127) / 128, py = (nf + kSymRows - 1) / kSymRows;
     if (q_blocks > 0x7fffffffLL || py > 65535) return set_error(MB_ERR_SIZE, "mesh too large for one launch");
     mom_sym_regular_rows_kernel<true><<<dim3((unsigned)q_blocks, (unsigned)py), 128, 0, s>>>(verts, faces, fei, n_edges,
-                                                                                             (float)k, nf, 0, nf, z, rec);
+                                                                                             (float)k, nf, 0, nf, z, rec, form);
     return check_launch("mom_sym_rest");
 }
 

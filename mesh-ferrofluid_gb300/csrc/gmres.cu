@@ -1377,7 +1377,7 @@ struct PgMatrix {
     const float* scale;  // kind 2: its scale (device)
 };
 
-// Steps per captured group.  A cycle usually ends well before its m steps (kind 2 stops once it has gained
+// Steps per captured group, at most.  A cycle usually ends well before its m steps (kind 2 stops once it has gained
 // inner_rtol), and the launches of a step after that, each returning at once, cost a microsecond
 // each: with whole cycles of 50 captured, 1.8 of 13.6 ms at 7680 unknowns, and 1.5 ms of capturing,
 // instantiating and launching 400 nodes.  The host reads the state after every group.
@@ -1401,8 +1401,8 @@ static void pg_head_t(const PgMatrix& A, int64_t n, const double2* b, const doub
 }
 
 template <typename B>
-static void pg_steps_t(const PgMatrix& A, int64_t n, const int32_t* cols, const float2* vals, int m, const PgWork& W,
-                       unsigned* cnt, cudaStream_t s) {
+static void pg_steps_t(const PgMatrix& A, int64_t n, const int32_t* cols, const float2* vals, int m, int count,
+                       const PgWork& W, unsigned* cnt, cudaStream_t s) {
     const unsigned vb = (unsigned)((n + 255) / 256), rb = (unsigned)((n + 7) / 8);
     const int sblk = (int)std::min<int64_t>((n + 127) / 128, kPgMaxBlocks);
     // dot-product chunks: at least 256 elements (8 a lane), at most kPgMaxBlocks chunks
@@ -1414,7 +1414,7 @@ static void pg_steps_t(const PgMatrix& A, int64_t n, const int32_t* cols, const 
     B* V = static_cast<B*>(W.V);
     B* w = static_cast<B*>(W.w);
     B* z = reinterpret_cast<B*>(W.z);
-    for (int j = 0; j < kPgGroup; ++j) {
+    for (int j = 0; j < count; ++j) {
         pg_precond_kernel<B><<<rb, 256, 0, s>>>(cols, vals, n, V, z, W.st);
         if constexpr (sizeof(B) == 8) {
             if (A.kind == 2)
@@ -1487,15 +1487,17 @@ int pgmres(int kind, const void* z, const void* z_half, const float* half_scale,
         if (graph) cudaGraphDestroy(graph);
         if (cap) cudaStreamDestroy(cap);
     };
-    auto steps = [&](cudaStream_t t) {
-        if (kind == 1) pg_steps_t<double2>(A, n, m_cols, vals, m, W, cnt, t);
-        else pg_steps_t<float2>(A, n, m_cols, vals, m, W, cnt, t);
+    // a cycle in equal groups of at most kPgGroup, so that few captured steps lie beyond its last (20: 7 + 7 + 7)
+    const int groups = (m + kPgGroup - 1) / kPgGroup, group = (m + groups - 1) / groups;
+    auto steps = [&](int count, cudaStream_t t) {
+        if (kind == 1) pg_steps_t<double2>(A, n, m_cols, vals, m, count, W, cnt, t);
+        else pg_steps_t<float2>(A, n, m_cols, vals, m, count, W, cnt, t);
     };
     if (use_graph) {
         if (cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking) != cudaSuccess ||
             cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
             return cleanup(), set_error(MB_ERR_CUDA, "pgmres: stream capture failed");
-        steps(cap);
+        steps(group, cap);
         cudaError_t ce = cudaStreamEndCapture(cap, &graph);
         if (ce != cudaSuccess || cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess)
             return cleanup(), set_error(MB_ERR_CUDA, "pgmres: graph capture / instantiate failed");
@@ -1509,12 +1511,12 @@ int pgmres(int kind, const void* z, const void* z_half, const float* half_scale,
     for (long long c = 0; c < max_cycles; ++c) {
         if (kind == 1) pg_head_t<double2>(A, n, b2, x2, W, cnt, s);
         else pg_head_t<float2>(A, n, b2, x2, W, cnt, s);
-        for (int j = 0; j < m; j += kPgGroup) {
+        for (int j = 0; j < m; j += group) {
             if (use_graph) {
                 if (cudaGraphLaunch(exec, s) != cudaSuccess)
                     return cleanup(), set_error(MB_ERR_CUDA, "pgmres: graph launch failed");
             } else {
-                steps(s);
+                steps(std::min(group, m - j), s);
             }
             if ((rc = read_state())) return cleanup(), rc;
             if (!hs.active) break;

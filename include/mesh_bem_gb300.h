@@ -127,6 +127,9 @@ int mb_index_range_i32(const int32_t* indices, int64_t count, int64_t limit, int
  * groups of eight ids among 32 consecutive faces (csrc/face_order.cuh).  work: 12 bytes of device memory. */
 int mb_index_range_order_i32(const int32_t* faces, int64_t n_faces, int64_t limit, int32_t* work, int32_t* outside,
                              int32_t* face_order, void* stream);
+/* The FP64 functions that the library's kernels use in place of CUDA's (csrc/f64_steps.cuh), over arrays [n] of device
+ * memory, for their test: function 0 x^(-1/2), 1 x^(1/2), 2 x / y, 3 sin(2 pi x y / 256), 4 cos(2 pi x y / 256). */
+int mb_f64_steps(int function, const double* x, const double* y, int64_t n, double* out, void* stream);
 /* No counterpart in the reference (its scatter_add_ runs after the whole face-edge matrix
  * exists).  edge_rows [2 n_edges + 1] int32: for Z row m (edge m) the face-edge rows 3f + e
  * of its faces (smaller first; -1 for a missing second face); edge_rows[2 n_edges] = 1 when

@@ -44,6 +44,7 @@ _SIGS = {
                                   _I64, _I64, _P, _P],
     "mb_face_geometry_f32": [_P, _I64, _P, _I64, _P, _P, _P],
     "mb_face_geometry_f64": [_P, _I64, _P, _I64, _P, _P, _P],
+    "mb_f64_steps": [_I, _P, _P, _I64, _P, _P],
     "mb_index_range_i32": [_P, _I64, _I64, _P, _P, _P],
     "mb_index_range_order_i32": [_P, _I64, _I64, _P, _P, _P, _P],
     "mb_mom_tiers_workspace_bytes": [_I64],

@@ -51,6 +51,7 @@ template <typename T>
 int launch_laplace_panels(const T*, const int32_t*, int64_t, const T*, const T*, const T*, const int*,
                           const uint8_t*, int, int, int, double, int64_t, int64_t, T*, T*, cudaStream_t);
 struct FaceOrder;
+int launch_f64_steps(int which, const double* x, const double* y, int64_t n, double* out, cudaStream_t s);
 template <typename T>
 int launch_pack_tight(const T*, const T*, const int32_t*, int64_t, int64_t, int, const FaceOrder*, T*, cudaStream_t);
 template <typename T>
@@ -315,6 +316,11 @@ int mb_index_range_i32(const int32_t* indices, int64_t count, int64_t limit, int
                        void* stream) {
     MB_REQUIRE(count >= 0 && outside && (count == 0 || (indices && work)), "null pointer argument or negative count");
     return index_range(indices, count, limit, work, outside, nullptr, as_stream(stream));
+}
+
+int mb_f64_steps(int function, const double* x, const double* y, int64_t n, double* out, void* stream) {
+    MB_REQUIRE(function >= 0 && function <= 4 && n >= 0 && (n == 0 || (x && out && (y || function < 2))), "bad arguments");
+    return launch_f64_steps(function, x, y, n, out, as_stream(stream));
 }
 
 int64_t mb_mom_tiers_workspace_bytes(int64_t n_faces) { return n_faces > 0 ? 128 * n_faces + 16 : 0; }

@@ -15,6 +15,7 @@
 //   int_T (rho_y - rho)/R^3 dS = - sum_i u_i ln((R+_i + l+_i)/(R-_i + l-_i)).
 #pragma once
 #include "common.cuh"
+#include "f64_steps.cuh"
 
 namespace mb {
 
@@ -75,27 +76,11 @@ __device__ __forceinline__ void potential_integrals(const V3<R>& x, const V3<R> 
 // they take few instructions: the edges' directions once per triangle; a corner's distance once (it is R+ of one
 // edge and R- of the next); sum (beta+ - beta-) as the solid angle, which is one arc tangent of
 //   2 area |d| / (r0 r1 r2 + (r0.r1) r2 + (r1.r2) r0 + (r2.r0) r1),  r_i.r_j = (r_i^2 + r_j^2 - L_ij^2) / 2
-// instead of six; roots and quotients from the hardware's approximations (about 2^-20) by one third-order step.
+// instead of six; roots and quotients by f64_steps.cuh.
 struct FaceEdges {
     V3<double> n, l[3], u[3];
     double len[3], area2;  // edge lengths, twice the area
 };
-
-__device__ __forceinline__ double rsqrt_step(double x) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double t = fma(-(x * y), y, 1.0);
-    return fma(t * y, fma(t, 0.375, 0.5), y);
-}
-__device__ __forceinline__ double sqrt_step(double x) { return x > 0.0 ? x * rsqrt_step(x) : sqrt(x); }
-__device__ __forceinline__ double quotient_step(double a, double b) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-    const double e = fma(-b, y, 1.0);
-    y = fma(y, fma(e, e, e), y);
-    const double q = a * y;
-    return fma(fma(-b, q, a), y, q);
-}
 
 __device__ __forceinline__ FaceEdges face_edges(const V3<double> P[3]) {
     FaceEdges f;

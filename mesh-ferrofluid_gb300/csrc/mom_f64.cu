@@ -13,22 +13,19 @@
 //   * |x - y|^2 = |A|^2 - 2 (B0 - A0).A + |y - A0|^2 - 2 Y.A: the last product is there already.  Between close
 //     pairs that sum would cancel, so a warp that holds one takes the coordinates' differences, and y.u from
 //     (x - y).u, which is as small as |x - y|;
-//   * the reciprocal root from the hardware's approximation (about 2^-20) by one third-order step
-//     y (1 + t/2 + 3 t^2/8), t = 1 - r^2 y^2;
-//   * sin and cos from a table of 256 angles, filled by each block, and the Taylor series about the nearest
-//     (|d| <= pi/256: d^7/7! = 8e-18 is dropped);
+//   * the reciprocal root, sine and cosine by f64_steps.cuh, its table of angles filled by each block;
 //   * the test face's values once per block and row (shared memory), the source face's length factor once per
 //     thread for all its rows.
 #include <algorithm>
 
 #include "common.cuh"
+#include "f64_steps.cuh"
 
 namespace mb {
 
 namespace {
 
 constexpr int kF64Threads = 128;
-constexpr int kAngles = 256;
 constexpr int kF64Points = 256;  // test points: rules up to 16 x 16
 constexpr int kF64Rows = 8;      // rows of a block
 
@@ -43,28 +40,6 @@ struct F64Rows {
     double v[kF64Rows][21];
     double3 s[16];           // source points: r3 - r4, r4, weight / (4 pi)
 };
-
-__device__ __forceinline__ double rsqrt_f64(double x) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double t = fma(-(x * y), y, 1.0);
-    return fma(t * y, fma(t, 0.375, 0.5), y);
-}
-
-// sin and cos of 2 pi turn x / 256
-__device__ __forceinline__ void sincos_f64(const double2* table, double x, double turn, double* s, double* c) {
-    constexpr double kStep = 2.0 * kPi / kAngles;
-    constexpr double kMagic = 6755399441055744.0;  // 1.5 * 2^52: adding it rounds
-    const double z = fma(x, turn, kMagic);
-    const double f = fma(x, turn, kMagic - z);
-    const double2 t = table[__double2loint(z) & (kAngles - 1)];
-    constexpr double k2 = kStep * kStep;
-    const double q = f * f;
-    const double sd = f * fma(q, fma(q, kStep * k2 * k2 / 120.0, -kStep * k2 / 6.0), kStep);
-    const double cm = q * fma(q, fma(q, -k2 * k2 * k2 / 720.0, k2 * k2 / 24.0), -0.5 * k2);  // cos - 1
-    *s = fma(t.y, sd, fma(t.x, cm, t.x));
-    *c = fma(-t.x, sd, fma(t.y, cm, t.y));
-}
 
 __device__ __forceinline__ double dot3(const double* a, const V3<double>& b) {
     return a[0] * b.x + a[1] * b.y + a[2] * b.z;
@@ -116,10 +91,10 @@ __device__ __forceinline__ void f64_sums(const F64Rows& sh, const double* rv, in
                 r2 = fma(-2.0, ya, x2 + p0[j]);
                 uy = fma(-ya, xn, yn[j] * xa);
             }
-            const double ri = rsqrt_f64(r2);
+            const double ri = rsqrt_step(r2);
             const double R = r2 * ri;
             double sn, cs;
-            sincos_f64(sh.angle, R, turn, &sn, &cs);
+            sincos_step(sh.angle, R, turn, &sn, &cs);
             const double g = wj[j] * ri;
             const double gr = g * cs, gs = g * sn;
             const double c = fma(k, ya, m4k);
@@ -149,11 +124,7 @@ __global__ void __launch_bounds__(kF64Threads, NS <= 4 ? 4 : 2) mom_f64_kernel(
     constexpr int NY = NS == 1 ? 1 : (NS == 4 ? 2 : (NS == 9 ? 3 : 4));
     __shared__ F64Rows sh;
     const int t = threadIdx.x, nt = nx * nx;
-    for (int i = t; i < kAngles; i += kF64Threads) {
-        double s, c;
-        sincospi(i * (2.0 / kAngles), &s, &c);
-        sh.angle[i] = make_double2(s, c);
-    }
+    fill_angles(sh.angle);
     for (int i = t; i < nt; i += kF64Threads) {
         const double r1 = gpx[i / nx];
         sh.r[i] = make_double2(r1 - gpx[i % nx] * r1, gpx[i % nx] * r1);

@@ -912,10 +912,13 @@ static int launch_sym_rows(const T* verts, const int32_t* faces, int64_t nf, int
                            int64_t row_end, const FaceOrder* order, T* packed, cudaStream_t s) {
     if (row_end - row_begin > 0x7fffffffLL) return set_error(MB_ERR_SIZE, "mesh too large for one launch");
     auto go = [&](auto kernel) -> int {
-        // the same limit for every mesh: it is the process's, and another thread may be between these two calls
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTightSmemMax);
-        if (e != cudaSuccess) return set_error(MB_ERR_CUDA, "%s", cudaGetErrorString(e));
-        kernel<<<(unsigned)(row_end - row_begin), kSymThreads, (size_t)(3 * nv) * sizeof(T), s>>>(verts, faces, nf, nv,
+        const size_t smem = (size_t)(3 * nv) * sizeof(T);
+        if (smem > 48 * 1024) {
+            // the same limit for every mesh: it is the process's, and another thread may be between these two calls
+            const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTightSmemMax);
+            if (e != cudaSuccess) return set_error(MB_ERR_CUDA, "%s", cudaGetErrorString(e));
+        }
+        kernel<<<(unsigned)(row_end - row_begin), kSymThreads, smem, s>>>(verts, faces, nf, nv,
                                                                                                row_begin, order, packed);
         return MB_OK;
     };
@@ -935,11 +938,11 @@ static int launch_sym_pairs(const double* verts, const int32_t* faces, int64_t n
 //   300 rows of 680 faces 18 / 28, 19 / 30, 17 / 27, of 2112 39 / 42, 41 / 45, 37 / 41, of 2960 52 / 52, 54 / 54, 49 / 50, of
 //   4048 80 / 56, 82 / 59, 68 / 53; 100 rows of 874 17 / 19, 19 / 20, 17 / 19; 30 rows of 680 14 / 10, 15 / 10, 16 / 10, of
 //   126 8 / 8, 8 / 10, 8 / 8.
-// Where the pairs form may run, looking at the faces' order and the other form's empty launch cost it 8 to 15 us more.
+// Where many rows may go by pairs, the look at the faces' order and the other form's empty launch cost 10 to 18 us more,
+// which a mesh in any order pays for nothing: 2.5 % of a call at these lines (5120 faces 1041 -> 1060 us), 5 % at 2600.
 static bool rows_form(int64_t nf, int64_t rows, int op) {
     if (nf < 150) return true;
-    if (rows < 64 || nf >= 3600) return false;
-    return rows < 512 || (nf < 2600 && rows * nf < (op == 3 ? 6000000 : 2200000));
+    return rows >= 64 && nf < (op == 3 ? 4800 : 3600);
 }
 
 static int launch_sym_pairs(const float* verts, const int32_t* faces, int64_t nf, int64_t nv, int op, int64_t row_begin,

@@ -193,12 +193,13 @@ def laplace_sym_tight(verts: torch.Tensor, faces: torch.Tensor, op: int, near: t
             part[r1:].zero_()
         out += pack_matrix_tight(int(OrderType.LINEAR), part, verts, faces)
         return out
-    args = (_lib.ptr(verts), nv, _lib.ptr(faces), nf, int(op), _lib.ptr(near), near.shape[0], r0, r1)
-    if verts.dtype == torch.float32 and nf >= 1024:  # large meshes: the kernel is chosen by the order of the faces
+    if nf >= 3600 and verts.dtype == torch.float32:  # large meshes: the kernel is chosen by the order of the faces
         work = torch.empty(2, dtype=torch.int32, device=verts.device)
-        _lib.call("mb_laplace_sym_tight_ordered_f32", *args, _lib.ptr(work), _lib.ptr(out), _lib.stream_of(verts))
-    else:
-        _lib.call(f"mb_laplace_sym_tight_{_lib.sfx(verts.dtype)}", *args, _lib.ptr(out), _lib.stream_of(verts))
+        _lib.call("mb_laplace_sym_tight_ordered_f32", _lib.ptr(verts), nv, _lib.ptr(faces), nf, int(op), _lib.ptr(near),
+                  near.shape[0], r0, r1, _lib.ptr(work), _lib.ptr(out), _lib.stream_of(verts))
+        return out
+    _lib.call(f"mb_laplace_sym_tight_{_lib.sfx(verts.dtype)}", _lib.ptr(verts), nv, _lib.ptr(faces), nf, int(op),
+              _lib.ptr(near), near.shape[0], r0, r1, _lib.ptr(out), _lib.stream_of(verts))
     return out
 
 

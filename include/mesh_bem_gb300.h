@@ -147,8 +147,9 @@ int mb_mom_zmat_rwg_edges_c64(const float* verts, int64_t n_verts, const int32_t
                               float* z, void* stream);
 /* The same matrix with each face pair's quadrature sized by its separation (csrc/mom_tiers.cu: the
  * reference's points on close pairs, rules of the same exactness with fewer points on the
- * others, entries equal within FP32 rounding); accumulated into z.  float32 meshes, gaussQR 3
- * to 5; any number of faces per edge.  workspace: mb_mom_tiers_workspace_bytes(n_faces), 16-byte aligned. */
+ * others, entries equal within FP32 rounding); accumulated into z by atomic additions, so that an
+ * entry's last bit may differ from call to call (mb_mom_zmat_rwg_edges_c64 and _gather_c64 repeat
+ * bit for bit).  float32 meshes, gaussQR 3 to 5; any number of faces per edge.  workspace: mb_mom_tiers_workspace_bytes(n_faces), 16-byte aligned. */
 int64_t mb_mom_tiers_workspace_bytes(int64_t n_faces);
 int mb_mom_zmat_rwg_tiers_c64(const float* verts, int64_t n_verts, const int32_t* faces, int64_t n_faces,
                               const float* face_areas, const float* face_normals, const int32_t* face_edge_indices,

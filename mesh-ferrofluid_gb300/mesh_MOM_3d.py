@@ -200,8 +200,11 @@ def assemble_Z_rwg(verts, faces, face_areas, face_normals, face_edge_indices, n_
     ~3 % slower at 20480 faces: neighbouring threads read scattered source faces).
     ``order="tiers"`` (float32, gaussQR 3-5, no ``rows``): each face pair's quadrature sized by
     its separation -- the reference's points on close pairs, one set of fewer points of the same
-    exactness for all nine entries of the others; equal to the other orders within FP32 rounding.
-    ``order="auto"`` (default) takes "tiers" when it applies, else the edge order when it applies
+    exactness for all nine entries of the others; equal to the other orders within FP32 rounding.  An
+    entry's up to four terms are atomic additions whose order may differ from call to call, and with it
+    its last bit; ``"edges"`` (two terms) and ``"gather"`` repeat bit for bit.
+    ``order="auto"`` (default) takes "tiers" when it applies and
+    ``torch.use_deterministic_algorithms`` is off, else the edge order when it applies
     (float32, a fast rule, no ``rows``, every edge on at most two faces) and the face order otherwise.
     ``edge_rows_map``: ``edge_rows(face_edge_indices, F, E)`` computed once by the caller.
     ``out_host`` (complex64 [E, E] CPU tensor, pinned for overlap): Z goes to host memory,
@@ -233,7 +236,8 @@ def assemble_Z_rwg(verts, faces, face_areas, face_normals, face_edge_indices, n_
         return out_host
     if order == "auto":
         order = "faces"
-        if dt == torch.float32 and rows is None and (nx, ny) in _TIER_RULES:
+        if dt == torch.float32 and rows is None and (nx, ny) in _TIER_RULES \
+                and not torch.are_deterministic_algorithms_enabled():
             order = "tiers"
         elif dt == torch.float32 and rows is None and (nx, ny) in _EDGE_RULES:
             try:

@@ -23,7 +23,7 @@ struct FaceOrder {
     int ids;      // different ids of ten consecutive faces' 30, mean of the samples: 12 to 14 vertices along a strip, 14 on a
                   // subdivided sphere, 30 in any order; 21 to 23 edges, 30 in any order
     int sectors;  // of 32 consecutive faces, groups of eight ids (32 bytes of a float row) among the first corners, plus
-                  // the second, plus the third: 12 along a strip of neighbouring ids, 22 on a subdivided sphere, 53 on strips
+                  // the second, plus the third: 12 along a strip of neighbouring ids, 19 to 37 on a subdivided sphere, 53 on strips
                   // across the ids, 90 in any order
 };
 

@@ -930,7 +930,9 @@ int launch_pack_rows(const T* m, const T* verts, const int32_t* faces, int64_t n
 // (9 instead of 3 per pair, one 32-byte sector each). Measured (GB300, us, pack_rows_kernel / this): subdivided
 // sphere 5120 faces 614 / 285, 20480 27.1 / 4.3 ms; strips along the vertex ids 2960 124 / 98, 4048 409 / 166, 7080 1141 / 479;
 // strips across them 2112 55 / 122, 3444 189 / 270, 4704 492 / 510, 8064 4880 / 1455; any order 1280 35 / 78, 5120
-// 587 / 1188; below 2500 faces at most 15 us apart in this kernel's favour. So: from 2500 faces on, by the order.
+// 587 / 1188; below 2500 faces at most 15 us apart in this kernel's favour. So: from 2500 faces on, by the order: the groups
+// of eight ids (face_order.cuh) are 12 along the ids, 19 to 37 on spheres subdivided in two ways of numbering, 42 with their
+// faces in runs of eight in any order (602 / 414), and 51 to 53 across the ids.
 constexpr int kPackStages = 3;
 constexpr int kPackSmem = kPairSumBytes + kPackStages * kPairThreads * 9 * (int)sizeof(float);
 
@@ -1004,7 +1006,7 @@ int launch_pack_tight(const T* m_r, const T* m_i, const int32_t* faces, int64_t 
     if (nf <= 0) return MB_OK;
     if (m_i == nullptr && order == 1) {
         const bool rows = 3 * nv * (int64_t)sizeof(T) <= kPackRowSmemMax;
-        const bool by_order = nf >= 2500 && faces_order && faces_order->ids <= 20 && faces_order->sectors <= 32;
+        const bool by_order = nf >= 2500 && faces_order && faces_order->ids <= 20 && faces_order->sectors <= 45;
         if ((by_order || !rows) && pack_pairs(m_r, faces, nf, nv, packed, stream)) return check_launch("pack_pairs");
         if (rows) return launch_pack_rows<T, false>(m_r, nullptr, faces, nf, nv, packed, stream);
     }

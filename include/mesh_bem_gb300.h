@@ -360,7 +360,9 @@ size_t mb_gmres_workspace_bytes(int64_t n, int restart);
  * products, FP64 Arnoldi (CGS2) and Givens rotations, and an FP64 residual b - Z x at the
  * start of every restart cycle (iterative refinement).  b, x: interleaved complex128 [n];
  * x holds the initial guess on entry and the solution on return.  restart in [1, 128].
- * Runs on `stream` and returns after synchronising it (the host drives the Arnoldi loop).
+ * Runs on `stream` and returns after synchronising it.  Up to 12288 unknowns a restart cycle is one cooperative
+ * kernel; above, where the driver refuses that launch, and for b, x or a workspace that is not on a 16-byte
+ * boundary, the host drives the Arnoldi loop.
  * workspace: >= mb_gmres_workspace_bytes(n, restart) bytes of device memory owned by the
  * caller.  info (host pointer, may be NULL) receives the outcome. */
 int mb_gmres_c64(const float* z, int64_t n, const double* b, double* x, int restart, int max_iters,

@@ -13,6 +13,8 @@ constexpr double kPi = 3.14159265358979323846;
 constexpr double kInv4Pi = 0.0795774715459476678844;  // 1 / (4 pi)
 constexpr double kInv2Pi = 0.159154943091895335769;   // 1 / (2 pi)
 
+constexpr int kSms = 152;  // SMs of a GB300, for the sizes of grids
+
 // Records a message for mb_last_error(); returns `code`.
 int set_error(int code, const char* fmt, ...);
 // Checks cudaGetLastError() after a launch; returns MB_OK or MB_ERR_CUDA.

@@ -9,7 +9,8 @@
 //     residual of every restart cycle);
 //   * Arnoldi by classical Gram-Schmidt with one re-orthogonalisation pass (CGS2) on a
 //     complex128 basis, dot products accumulated in FP64 (block partials + FP64 atomics);
-//   * Givens rotations and the small least-squares solve on the host (m <= 128 numbers).
+//   * Givens rotations and the small least-squares solve on the host (m <= 128 numbers);
+//   * up to 12288 unknowns a restart cycle as one resident kernel instead (gmres_cycle.cu).
 // Each restart cycle starts from the FP64 residual, so the inner FP32 matvec limits only
 // the per-cycle reduction, not the final accuracy (GMRES with iterative refinement).
 // Every loop is bounded by max_iters; nothing waits on the device except cudaStreamSynchronize.

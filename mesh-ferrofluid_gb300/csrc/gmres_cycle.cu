@@ -5,9 +5,9 @@
 // product is 0.01 ms, the Gram-Schmidt kernels running as 8 blocks over serial loops.  Here the
 // grid stays resident for the cycle.  Each worker block owns a range of rows: it computes its
 // part of the product and keeps its rows of the whole complex128 basis in shared memory, so
-// Gram-Schmidt reads no global memory beyond the sums.  Per step the blocks meet four times:
-// the two passes' sums V^H w (FP64 atomics, as in gmres.cu), the new basis vector, and the
-// first sums again.  One more block applies the Givens rotations of a step while the workers are
+// Gram-Schmidt reads no global memory beyond the sums.  Per step the blocks meet three times:
+// for the two passes' sums V^H w (FP64 atomics, as in gmres.cu) and for the new basis vector, and once
+// more where its norm has to be summed again.  One more block applies the Givens rotations of a step while the workers are
 // in the next step's product; when it finds the estimate below the target the workers drop
 // that step and add V y to x.  Precisions are those of gmres.cu: products in FP32 (or FP64 for a
 // float64 matrix) with FP64 lane sums, everything else FP64.

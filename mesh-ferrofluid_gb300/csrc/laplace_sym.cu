@@ -389,8 +389,8 @@ __global__ void __launch_bounds__(kSymThreads, sizeof(T) == 4 ? (OP == 3 ? 6 : 4
 // Lanes of a packed register are the two orbits of fx.  The sums are over k(R) - k(R_c): the
 // constant's integrals are known, and the rounding is that of the differences.  Entries are added by
 // vertex_slots.cuh.  Bound: SFU (49 reciprocal roots per pair, 0.28 ms at 5120 faces) and issue
-// slots.  Measured (GB300, 5120 faces): single / double / hypersingular 982 / 1020 / 757 ->
-// 485 / 541 / 421 us.
+// slots.  Measured (GB300, 5120 faces of a subdivided sphere, the pairs sharing a vertex included): single / double /
+// hypersingular 1028 / 1065 / 805 -> 512 / 586 / 442 us.
 // Pairs whose centroids are closer than twice the sum of the corner distances, where the
 // expansion of R^2 would cancel, are listed and evaluated from coordinate differences.
 constexpr int kRowRec = 28;  // floats per staged test face

@@ -4,7 +4,7 @@
 // Bound: launches and waits, not bytes.  As tensor operations the areas and normals of a mesh of a few hundred
 // faces take 18 launches (two gathers of three vertices, two cross products, norms, divisions) and the range of
 // one index array four launches and two waits; here one launch each and one wait.  A CFIE assembly with
-// one excitation on 80 faces: 564 -> 171 us.
+// one excitation on 80 faces: 610 -> 171 us.
 #include "common.cuh"
 #include "face_order.cuh"
 
@@ -76,7 +76,7 @@ int index_range(const int32_t* idx, int64_t count, int64_t limit, int32_t* work,
     if (e == cudaSuccess) {
         // four indices a thread; at most two blocks an SM
         const int64_t blocks = (count + 1023) / 1024;
-        index_range_kernel<<<(unsigned)(blocks < 304 ? blocks : 304), 256, 0, s>>>(idx, count, limit, work);
+        index_range_kernel<<<(unsigned)(blocks < 2 * kSms ? blocks : 2 * kSms), 256, 0, s>>>(idx, count, limit, work);
         if (order)
             face_order_kernel<<<1, 32 * kOrderSamples, 0, s>>>(idx, count / 3, reinterpret_cast<FaceOrder*>(work + 1));
         e = cudaGetLastError();

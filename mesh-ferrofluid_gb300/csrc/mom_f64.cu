@@ -249,8 +249,8 @@ void launch_f64(const double* verts, const int32_t* faces, const double* areas, 
                 double* zr, double* zi, cudaStream_t stream) {
     const int64_t col_blocks = (3 * nf + kF64Threads - 1) / kF64Threads, rows = row_end - row_begin;
     // The table costs a block about a twentieth of a row of 36 evaluations, so a block takes several rows, as long
-    // as there are eight blocks for each of the 152 SMs' places (4 of 128 threads) to even out the close pairs.
-    const int64_t rpb = std::min<int64_t>(kF64Rows, std::max<int64_t>(1, rows * col_blocks / (152 * 4 * 8)));
+    // as there are eight blocks for each of the SMs' places (4 of 128 threads) to even out the close pairs.
+    const int64_t rpb = std::min<int64_t>(kF64Rows, std::max<int64_t>(1, rows * col_blocks / (kSms * 4 * 8)));
     const unsigned blocks = (unsigned)((rows + rpb - 1) / rpb * col_blocks);
     if (fei)
         mom_f64_kernel<NS, true><<<blocks, kF64Threads, 0, stream>>>(verts, faces, areas, normals, fei, n_edges, gpx,

@@ -5,9 +5,9 @@
 // collapsed Gauss-Legendre rule whose points are laid out from the vertex opposite the
 // local edge (x = (1-r1) v_e + (r1-r2) v_{e+1} + r2 v_{e+2}, r2 = p_j r1, weight w_i w_j 2A,
 // Jacobian r1; :410-421).  The rule is not invariant under vertex rotation, so the nine
-// entries of a triangle pair use nine different point sets: the work per entry is
-// irreducible at Nt x Ns kernel evaluations, exactly as in the reference.  What this file
-// removes is everything around it:
+// entries of a triangle pair use nine different point sets: Nt x Ns kernel evaluations per
+// entry, exactly as in the reference (mom_tiers.cu evaluates fewer on separated pairs).  What this
+// file removes is everything around them:
 //   * one sincos per point pair shared by G and grad G (the reference evaluates both
 //     separately, :461-465), a MUFU rsqrt instead of sqrt + divide;
 //   * the per-test-point moment form: with the origin moved to the source vertex B0,

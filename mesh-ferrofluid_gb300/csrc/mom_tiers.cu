@@ -26,8 +26,9 @@
 // Gauss-Legendre, a normal that is not perpendicular to its face and coordinates that are
 // not finite put every pair concerned into tier 4.
 //
-// Measured on GB300 (2070 MHz), whole call: 20480 faces, k 10, unit sphere 499.3 -> 35.1 ms (far pairs 26.2, close
-// pairs 4.0 + 3.6); 5120 faces, k 6, ellipsoid 32.1 -> 4.8 ms; 1280 faces at k 10, all in tier 4, 2.54 -> 2.63 ms.
+// Measured on GB300 (2070 MHz), whole call: 20480 faces, k 10, unit sphere 500.0 -> 34.8 ms (far pairs 26.2, close
+// pairs 4.0 + 3.6); 5120 faces, k 6, ellipsoid 32.2 -> 4.6 ms; all pairs in tier 4: 1280 faces, k 10, gaussQR 4 2.13 -> 2.10
+// ms, gaussQR 5 5.12 -> 5.15, 5120 faces, k 30, 31.3 -> 31.3 and 78.8 -> 79.1.
 // Error of the entries against 64 bits by distance, of the 1296 points' FP32 error: 1.0 .. 1.1 below 4 h, 0.5 .. 0.95
 // beyond (kh 0.15 .. 0.9).  The four adds of an entry are atomic, so its last bit depends on their order.
 //
@@ -50,6 +51,11 @@ namespace {
 // ---------------------------------------------------------------------------------------
 // face records: 32 floats per face
 // ---------------------------------------------------------------------------------------
+// sin x = x (1 + SA x^2 + SB x^4) and cos x = 1 + CA x^2 + CB x^4 + CC x^6, least squares on |x| <= 0.43 (off by
+// 5e-8 of x and 3e-10)
+constexpr float SA = -0.16666371f, SB = 0.00828212f;
+constexpr float CA = -0.49999997f, CB = 0.04166572f, CC = -0.00138007f;
+
 // degree-4 rule: corners (1 - 2 q, q, q) of two orbits lie at s A_a from the centroid
 constexpr float kS1 = (float)(1.0 - 3.0 * 0.445948490915965), kW1 = 0.223381589678011f;
 constexpr float kS2 = (float)(1.0 - 3.0 * 0.091576213509771), kW2 = 0.109951743655322f;
@@ -301,8 +307,6 @@ __global__ void __launch_bounds__(128, 2) far_pairs_kernel(const TierArgs args, 
     const int col[3] = {__float_as_int(q1.w), __float_as_int(q2.w), __float_as_int(q3.w)};
     const double kt = m.k * kInv2Pi;
     const float kth = (float)kt, ktl = (float)(kt - (double)kth), four_k = 4.f / k;
-    constexpr float SA = -0.16666371f, SB = 0.00828212f;                     // sin
-    constexpr float CA = -0.49999997f, CB = 0.04166572f, CC = -0.00138007f;  // cos
     const float wqx = kW1, wqy = kW2, wsx = kW1 * kS1, wsy = kW2 * kS2;
 #pragma unroll 1
     for (int i = 0; i < np; ++i) {
@@ -354,8 +358,8 @@ __global__ void __launch_bounds__(128, 2) far_pairs_kernel(const TierArgs args, 
                     rinv.y = rsqrtf(r2.y);
                     const float2 R = mul2(r2, rinv), d0 = sub2(R, bc(R0));
                     const float2 th = mul2(fma2(d0, d0, ns), bc(kp));  // -k (R - R_c)
-                    // |th| <= 0.43 by the rule of tier 1: polynomials (least squares on that range, off
-                    // by 5e-8 of th and 3e-10); the SFU's error, 4e-7 and alike over a pair, would not average out
+                    // |th| <= 0.43 by the rule of tier 1: polynomials; the SFU's error, 4e-7 and alike over a pair,
+                    // would not average out
                     const float2 t = mul2(th, th);
                     const float2 sn = mul2(th, fma2(t, fma2(t, bc(SB), bc(SA)), bc(1.f)));
                     const float2 cs = fma2(t, fma2(t, fma2(t, bc(CC), bc(CB)), bc(CA)), bc(1.f));
@@ -781,8 +785,6 @@ __global__ void __launch_bounds__(128, 4)
     if (!*form) return;
     constexpr float s1 = (float)(1.0 - 3.0 * 0.10128650732345634), s2 = (float)(1.0 - 3.0 * 0.47014206410511509);
     constexpr float w0 = 0.225f, w1 = 0.12593918054482715f, w2 = 0.13239415278850619f;
-    constexpr float SA = -0.16666371f, SB = 0.00828212f;                     // sin, as in far_pairs_kernel
-    constexpr float CA = -0.49999997f, CB = 0.04166572f, CC = -0.00138007f;  // cos
     __shared__ float4 s_rec[kEdgeRows * (kRec / 4)];
     __shared__ EdgeSlots s_e;
     extern __shared__ float2 s_sum[];  // [kEdgeSlots][3][128]
@@ -962,7 +964,7 @@ __global__ void __launch_bounds__(128, 4)
 // 4415 / 8230; one of 5120, k 10, gaussQR 3, 10.36 / 10.43 ms, 8x32 11.02.
 void mom_tier_tiles(int64_t pairs, int* rows, int* tp, int* tq) {
     *rows = pairs >= 5000 * 5000 ? 32 : 8;
-    const double per_block = (double)pairs / 4864.0;  // were there 8 times the 608 resident blocks
+    const double per_block = (double)pairs / (kSms * 4 * 8);  // were there 8 times the resident blocks (4 an SM)
     *tp = per_block >= 4096 ? 16 : per_block >= 1024 ? 8 : per_block >= 200 ? 14 : per_block >= 3 ? 4 : 7;
     *tq = per_block >= 1024 ? 64 : per_block >= 200 ? 16 : per_block >= 40 ? 32 : per_block >= 3 ? 16 : 2;
 }

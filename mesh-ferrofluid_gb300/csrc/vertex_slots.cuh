@@ -12,6 +12,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "common.cuh"
+
 namespace mb {
 
 // Measured for the packed Laplace operators at 5120 faces (three operators, us): 16 faces and 20 vertices 1448
@@ -25,7 +27,6 @@ constexpr int kPairSumBytes = 3 * kPairVerts * kPairThreads * (int)sizeof(float)
 // of the blocks, each worth its faces and about 0.6 more for its start; fewer than five blocks an SM leave it waiting
 // (676 faces: 8 a block 35 us, 5 27.5, 2 28.7).  Among those within 1 % the most faces: fewer reductions.
 inline int pair_rows(int64_t rows, int64_t gx) {
-    constexpr int64_t kSms = 152;
     int best = 1;
     double cost = 0.0;
     for (int per = 1; per <= kPairRows; ++per) {

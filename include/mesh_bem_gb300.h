@@ -157,8 +157,8 @@ int mb_mom_zmat_rwg_tiers_c64(const float* verts, int64_t n_verts, const int32_t
                               const float* gw_y, int n_y, double wavenumber, void* workspace,
                               int64_t workspace_bytes, float* z, void* stream);
 /* The separated pairs of the 7-point-rule EFIE (as mb_mom_sym_zmat_rwg_c64 over all faces): accumulated into z, or,
- * with overwrite, the whole of z [n_edges, n_edges] written (what it held does not matter), then, on large
- * meshes whose neighbouring faces follow one another, with each unordered pair evaluated once.  workspace: mb_mom_tiers_workspace_bytes(n_faces), 16-byte aligned. */
+ * with overwrite, the whole of z [n_edges, n_edges] written (what it held does not matter); on large meshes whose
+ * neighbouring faces follow one another with each unordered pair evaluated once.  workspace: mb_mom_tiers_workspace_bytes(n_faces), 16-byte aligned. */
 int mb_mom_sym_zmat_rwg_pairs_c64(const float* verts, int64_t n_verts, const int32_t* faces, int64_t n_faces,
                                   const int32_t* face_edge_indices, int64_t n_edges, double wavenumber, int overwrite,
                                   void* workspace, int64_t workspace_bytes, float* z, void* stream);

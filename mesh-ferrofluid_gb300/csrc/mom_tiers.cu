@@ -708,18 +708,21 @@ __global__ void __launch_bounds__(128, NX <= 4 ? 4 : CLOSE ? 2 : 3) close_pairs_
 // its entries belong at (m, n) and (n, m).  The terms of kEdgeRows test faces are summed per thread in
 // shared memory by distinct test edge (8 faces of the sphere have 16 to 18 of 24), so that about 2 edges
 // x 3 of a face remain of 9 reductions per ordered pair: a reduction costs a cycle of its SM, which
-// with 9 bounds the whole at 13 ms for 20480 faces.  The kernel sums above the diagonal only, half the
-// reductions, and mirror_kernel copies; so it serves a matrix of its own, not one that is added to.
+// with 9 bounds the whole at 13 ms for 20480 faces.  Into a matrix of its own (not one that is added
+// to) the kernel sums above the diagonal only, half the reductions, and mirror_kernel copies.
 // Measured (GB300), 20480 faces: 22.35 (every ordered pair, row by row) -> 10.05 ms + 1.08 ms for
-// the mirror, 0.49 instead of 0.96 for the zeros, 0.5 ms for the pairs left.  (rows, slots, blocks per SM), summing on both
-// sides: 8/16/4 13.66, best of 4/8/5 15.4, 8/16/3 14.1, 12/22/3 14.1, 16/28/2 14.8 ms.  Bound: FMA pipe.  Entry errors
+// the mirror, 0.49 instead of 0.96 for the zeros, 0.5 ms for the pairs left; on both sides 13.66.  (rows, slots, blocks per
+// SM), both sides: 8/16/4 best of 4/8/5 15.4, 8/16/3 14.1, 12/22/3 14.1, 16/28/2 14.8 ms.  Bound: FMA pipe.  Entry errors
 // against 64 bits 0.45 .. 0.65 of the row kernel's beyond 4 edges.
 // Pairs with |D| >= 2 (rho_p + rho_q) and k (rho_p + rho_q) <= 0.6 (the phases' polynomials); the
 // others are left to mom_sym_regular_rows_kernel, which applies the same test.  It takes all of them (sym_form_kernel):
 //   * below 2400 faces, whose grid leaves the chip half empty: rows / pairs 121 / 166 us at 1280, 294 / 299 .. 310 at
 //     2112, 538 / 428 .. 457 at 2960;
 //   * where consecutive faces do not share edges, every term then a reduction: faces in any order 1.51 / 1.57 ms at 5120, 23.5 /
-//     33.3 at 20480; in runs of two 23.5 / 23.1, of four 23.4 / 14.6;
+//     33.3 at 20480; in runs of two 23.5 / 23.1, of four 23.4 / 14.6; on both sides, where a transposed term's reductions
+//     go down a column, also where neighbouring faces' edges are not numbered alike (groups of eight ids, face_order.cuh):
+//     subdivided sphere (33) 23.3 / 11.9, in runs of eight (48) 23.3 / 19.2, of four (57) 23.4 / 25.3, strips across the ids
+//     of 12798 faces (61) 8.8 / 11.8;
 //   * where most faces are too large for the phases: k 10, 5120 faces, 1.50 / 1.75 ms.
 // ---------------------------------------------------------------------------------------
 constexpr int kEdgeRows = 8, kEdgeSlots = 16;
@@ -730,20 +733,22 @@ struct EdgeSlots {
     uint8_t slot[4 * kEdgeRows];
 };
 
-// e at the one of (m, n) and (n, m) above the diagonal, for mirror_kernel to copy
-__device__ __forceinline__ void add_upper(float2* __restrict__ z, int64_t m, int64_t n, int64_t n_edges, float2 e) {
-    atomicAdd(z + min(m, n) * n_edges + max(m, n), e);
-    if (m == n) atomicAdd(z + m * n_edges + m, e);
+// e at (m, n) and (n, m); UPPER: at the one of them above the diagonal, for mirror_kernel to copy
+template <bool UPPER>
+__device__ __forceinline__ void add_both(float2* __restrict__ z, int64_t m, int64_t n, int64_t n_edges, float2 e) {
+    atomicAdd(z + (UPPER ? min(m, n) : m) * n_edges + (UPPER ? max(m, n) : n), e);
+    if (!UPPER || m == n) atomicAdd(z + n * n_edges + m, e);
 }
 
 // *form = 1 where sym_pairs_kernel pays (see above), from samples of the edge ids (face_order.cuh) and of the records.
 constexpr int kFormThreads = 512;
 __global__ void __launch_bounds__(kFormThreads) sym_form_kernel(const float* __restrict__ rec, const int32_t* __restrict__ fei,
-                                                                int64_t nf, float k, int* __restrict__ form) {
+                                                                int64_t nf, float k, int max_sectors,
+                                                                int* __restrict__ form) {
     const FaceOrder o = face_order(fei, nf);  // 30 edges of ten faces in any order, 21 to 24 neighbour by neighbour
     const float rho2 = __ldg(rec + kRec * (nf * threadIdx.x / kFormThreads) + kRho2);
     const int small = __syncthreads_count(2.f * k * sqrtf(rho2) <= 0.6f);
-    if (threadIdx.x == 0) *form = o.ids <= 25 && 2 * small >= kFormThreads;
+    if (threadIdx.x == 0) *form = o.ids <= 25 && o.sectors <= max_sectors && 2 * small >= kFormThreads;
 }
 
 constexpr int kMirror = 32;  // tile of mirror_kernel
@@ -779,6 +784,7 @@ __global__ void __launch_bounds__(256) mirror_kernel(float2* __restrict__ z, int
     }
 }
 
+template <bool UPPER>
 __global__ void __launch_bounds__(128, 4)
     sym_pairs_kernel(const float* __restrict__ rec, int64_t nf, int64_t n_edges, double kd, const int* __restrict__ form,
                      float* __restrict__ z) {
@@ -937,7 +943,7 @@ __global__ void __launch_bounds__(128, 4)
                     float2* d = mine + (3 * slot + b) * 128;
                     *d = add2(*d, e);
                 } else {
-                    add_upper(z2, s_e.id[3 * i + a], col[b], n_edges, e);
+                    add_both<UPPER>(z2, s_e.id[3 * i + a], col[b], n_edges, e);
                 }
             }
         }
@@ -947,7 +953,7 @@ __global__ void __launch_bounds__(128, 4)
 #pragma unroll
         for (int b = 0; b < 3; ++b) {
             const float2 e = mine[(3 * u + b) * 128];
-            if (e.x != 0.f || e.y != 0.f) add_upper(z2, m, col[b], n_edges, e);
+            if (e.x != 0.f || e.y != 0.f) add_both<UPPER>(z2, m, col[b], n_edges, e);
         }
     }
 }
@@ -1032,7 +1038,7 @@ int launch_mom_sym_regular(const T* verts, const int32_t* faces, const int32_t* 
 int launch_mom_sym_pairs(const float* verts, const int32_t* faces, const int32_t* fei, int64_t nf, int64_t n_edges, double k,
                          bool overwrite, float* rec, float* z, cudaStream_t s) {
     if (nf <= 0) return MB_OK;
-    if (!overwrite || nf < 2400) {
+    if (nf < 2400) {
         if (overwrite) {
             const cudaError_t e = cudaMemsetAsync(z, 0, sizeof(float2) * (size_t)n_edges * n_edges, s);
             if (e != cudaSuccess) return set_error(MB_ERR_CUDA, "%s", cudaGetErrorString(e));
@@ -1041,18 +1047,22 @@ int launch_mom_sym_pairs(const float* verts, const int32_t* faces, const int32_t
     }
     const int64_t gx = (nf + kEdgeRows - 1) / kEdgeRows, gy = (nf + 127) / 128;
     if (gx > 0x7fffffffLL || gy > 65535) return set_error(MB_ERR_SIZE, "mesh too large for one launch");
+    // a matrix that is not added to is summed above the diagonal only, half the reductions, and mirrored
+    const auto kernel = overwrite ? sym_pairs_kernel<true> : sym_pairs_kernel<false>;
+    const bool mirror = overwrite && n_edges > 0;
     const int64_t tiles = (n_edges + kMirror - 1) / kMirror;
-    if (n_edges > 0x7fffffffLL || (tiles + 1) / 2 > 65535) return set_error(MB_ERR_SIZE, "matrix too large for one launch");
+    if (mirror && (n_edges > 0x7fffffffLL || (tiles + 1) / 2 > 65535))
+        return set_error(MB_ERR_SIZE, "matrix too large for one launch");
     if (int rc = tier_records(verts, faces, nullptr, fei, nf, nullptr, nullptr, 0, nullptr, nullptr, 0, rec, s)) return rc;
     int* form = reinterpret_cast<int*>(rec + kRec * nf);
-    sym_form_kernel<<<1, kFormThreads, 0, s>>>(rec, fei, nf, (float)k, form);
-    const cudaError_t e = cudaFuncSetAttribute(sym_pairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kEdgeSumBytes);
+    sym_form_kernel<<<1, kFormThreads, 0, s>>>(rec, fei, nf, (float)k, overwrite ? 96 : 53, form);
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kEdgeSumBytes);
     if (e != cudaSuccess) return set_error(MB_ERR_CUDA, "%s", cudaGetErrorString(e));
     float2* z2 = reinterpret_cast<float2*>(z);
-    if (n_edges > 0) zero_upper_kernel<<<(unsigned)n_edges, 256, 0, s>>>(z2, n_edges);
+    if (mirror) zero_upper_kernel<<<(unsigned)n_edges, 256, 0, s>>>(z2, n_edges);
     // test groups fastest: blocks in flight share the rows of one source tile for the transposed terms
-    sym_pairs_kernel<<<dim3((unsigned)gx, (unsigned)gy), 128, kEdgeSumBytes, s>>>(rec, nf, n_edges, k, form, z);
-    if (n_edges > 0)
+    kernel<<<dim3((unsigned)gx, (unsigned)gy), 128, kEdgeSumBytes, s>>>(rec, nf, n_edges, k, form, z);
+    if (mirror)
         mirror_kernel<<<dim3((unsigned)(tiles + 1), (unsigned)((tiles + 1) / 2)), 256, 0, s>>>(z2, n_edges, (int)tiles, form);
     if (int rc = check_launch("mom sym pairs")) return rc;
     return launch_mom_sym_rest(verts, faces, fei, n_edges, k, nf, rec, form, z, s);

@@ -376,7 +376,7 @@ def assemble_Z_rwg_sym(verts, faces, face_edge_indices, n_edges, wavenumber, out
                        faces_range=None, check_indices=True, out_host=None, chunks=16):
     """EFIE RWG matrix [E, E] with the 7-point rule on both triangles.
 
-    Separated pairs run in the mesh dtype (float32 without ``out`` and ``faces_range``, on large meshes whose
+    Separated pairs run in the mesh dtype (float32 without ``faces_range``, on large meshes whose
     neighbouring faces follow one another: each unordered pair evaluated once for both of its places);
     pairs sharing a vertex (``pairs``, default ``near_pairs(faces)``, sorted by test face) have the 1/R
     part integrated in closed form in FP64.  ``faces_range`` restricts the separated pairs to test faces [begin, end) (the near
@@ -411,10 +411,11 @@ def assemble_Z_rwg_sym(verts, faces, face_edge_indices, n_edges, wavenumber, out
                   _lib.ptr(face_edge_indices), n_edges, float(wavenumber), _lib.ptr(pairs), pairs.shape[0],
                   _lib.ptr(out), out_host.data_ptr(), int(chunks), st)
         return out_host
-    if fresh:
+    if dt == torch.float32 and faces_range is None:
         ws = torch.empty(max(1, int(_lib.load().mb_mom_tiers_workspace_bytes(nf))), dtype=torch.uint8, device=dev)
         _lib.call("mb_mom_sym_zmat_rwg_pairs_c64", _lib.ptr(verts), verts.shape[0], _lib.ptr(faces), nf,
-                  _lib.ptr(face_edge_indices), n_edges, float(wavenumber), 1, _lib.ptr(ws), ws.numel(), _lib.ptr(out), st)
+                  _lib.ptr(face_edge_indices), n_edges, float(wavenumber), int(fresh), _lib.ptr(ws), ws.numel(),
+                  _lib.ptr(out), st)
     else:
         f0, f1 = (0, nf) if faces_range is None else faces_range
         _lib.call(f"mb_mom_sym_zmat_rwg_{_lib.csfx(dt)}", _lib.ptr(verts), verts.shape[0], _lib.ptr(faces), nf,

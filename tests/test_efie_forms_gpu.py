@@ -1,7 +1,7 @@
 """The EFIE matrix on both sides of the lines between its two ways with separated pairs (each unordered pair once,
-summed above the diagonal and mirrored; row by row): mesh sizes, faces in any order, wavenumbers at which no, some and all
-pairs are too large for the first.  Reference: the row-by-row matrix, which out= always takes.  Tolerance: that of
-test_efie_pairs_gpu.py."""
+summed above the diagonal and mirrored, or on both sides of a given matrix; row by row): mesh sizes, faces in any order,
+wavenumbers at which no, some and all pairs are too large for the first.  Reference: the row-by-row matrix
+(faces_range), with the near pairs added.  Tolerance: that of test_efie_pairs_gpu.py."""
 import numpy as np
 import pytest
 import torch
@@ -26,7 +26,10 @@ def test_matrix_of_its_own(pkg, nf, kind, k):
     edges, fei, _ = pkg.utils.get_edge_unique(V, F)
     ne, M = edges.shape[0], pkg.mesh_MOM_3d
     pairs = M.near_pairs(F)
-    ref = M.assemble_Z_rwg_sym(V, F, fei, ne, k, pairs=pairs, out=torch.zeros((ne, ne), dtype=torch.complex64, device="cuda"))
+    ref = M.assemble_Z_rwg_sym(V, F, fei, ne, k, faces_range=(0, nf))
+    L = pkg._lib
+    L.call("mb_mom_sym_near_c64", L.ptr(V), V.shape[0], L.ptr(F), nf, L.ptr(fei), ne, L.ptr(pairs), pairs.shape[0], k,
+           L.ptr(ref), L.stream_of(V))
     stale = torch.full((ne, ne), float("nan"), dtype=torch.complex64, device="cuda")  # what the new matrix is laid over
     del stale
     got = M.assemble_Z_rwg_sym(V, F, fei, ne, k, pairs=pairs)

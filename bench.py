@@ -2399,7 +2399,7 @@ def main():
             "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_per_step,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32",
             "data": "synthetic", "config": config, "roofline": roof, "clocks": clocks.summary(),
-            "gpu_launches": args.steps * (4 if sym else 1)}
+            "gpu_launches": args.steps * (5 if sym else 1)}
 
     # time to a 1e-4 error in J, plain FP32 path vs the mixed-precision path (reported beside the
     # headline; both formulations on the same 30 720-unknown sphere for the default workload)
